@@ -1,0 +1,135 @@
+"""The attention kernels that share a query's keys out (csrc/attention_rows.cu in float32, csrc/attention_decode_tile.cu for decode steps in
+bfloat16) against the same attention in 64 bits, with every option: bias by bucketed distance, slopes, sink, window, kept first tokens, chunked
+mask, values inside the key rows.  Rows that no query sees hold NaN."""
+import ctypes
+import math
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+PAGE = 64
+
+
+def _lib():
+    from velomind_b200.kernels.library import library
+    return library()
+
+
+def _p(t):
+    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+
+
+def _i(v):
+    return ctypes.c_int(int(v))
+
+
+def _stream():
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+class Step:
+    """Sequences of `before` cached and `new` tokens, paged in a shuffled order, and the options' tables."""
+
+    def __init__(self, H, Hkv, Dk, Dv, before, new, dtype, in_keys=False, far=40, seed=0):
+        g = torch.Generator().manual_seed(seed)
+        self.H, self.Hkv, self.Dk, self.Dv, self.before, self.new, self.dtype, self.in_keys = H, Hkv, Dk, Dv, before, new, dtype, in_keys
+        lens = [a + n for a, n in zip(before, new)]
+        width = max(-(-n // PAGE) for n in lens) + 1
+        pages = sum(-(-n // PAGE) for n in lens) + 2
+        order = torch.randperm(pages, generator=g).tolist()
+        kp = torch.full((pages, Hkv, PAGE, Dk), float("nan"))
+        vp = torch.full((pages, Hkv, PAGE, Dv), float("nan"))
+        self.table = torch.full((len(lens), width), -1, dtype=torch.int32)
+        self.k, self.v = [], []
+        for s, n in enumerate(lens):
+            k = torch.randn(n, Hkv, Dk, generator=g).to(dtype)
+            v = k[..., :Dv] if in_keys else torch.randn(n, Hkv, Dv, generator=g).to(dtype)
+            self.k.append(k.double()); self.v.append(v.double())
+            for b in range(-(-n // PAGE)):
+                pg = order.pop()
+                self.table[s, b] = pg
+                m = min(PAGE, n - PAGE * b)
+                kp[pg, :, :m] = k[PAGE * b:PAGE * b + m].transpose(0, 1).float()
+                vp[pg, :, :m] = v[PAGE * b:PAGE * b + m].transpose(0, 1).float()
+        self.kp = kp.to(dtype).to(DEV)
+        self.vp = self.kp if in_keys else vp.to(dtype).to(DEV)
+        self.T = sum(new)
+        self.stride = H * Dk + 16
+        self.q = (torch.randn(self.T, self.stride, generator=g) * 1.5).to(dtype)
+        self.positions = torch.cat([torch.arange(a, a + n) for a, n in zip(before, new)]).int()
+        self.seq = torch.cat([torch.full((n,), s) for s, n in enumerate(new)]).int()
+        self.far = far
+        self.rel = torch.randn(7, H, generator=g)
+        self.bucket = (torch.arange(far + 1) % 7).int()
+        self.sink = torch.randn(H, generator=g)
+        self.slopes = torch.rand(H, generator=g) * 0.1
+
+    def want(self, window, keep, chunk, rel, sink, slopes, scale):
+        out = torch.empty(self.T, self.H, self.Dv, dtype=torch.float64)
+        for t in range(self.T):
+            s, i = int(self.seq[t]), int(self.positions[t])
+            j = torch.arange(i + 1)
+            see = torch.ones(i + 1, dtype=torch.bool)
+            if window:
+                see &= i - j < window
+            if chunk:
+                see &= j // chunk == i // chunk
+            see |= j < keep
+            for h in range(self.H):
+                g = h // (self.H // self.Hkv)
+                x = (self.k[s][:i + 1, g] @ self.q[t, h * self.Dk:(h + 1) * self.Dk].double()) * scale
+                if rel:
+                    x = x + self.rel[self.bucket[(i - j).clamp(max=self.far)].long(), h].double()
+                if slopes:
+                    x = x - self.slopes[h].double() * (i - j)
+                x = x[see]
+                top = max(float(x.max()), float(self.sink[h]) if sink else -math.inf)
+                e = torch.exp(x - top)
+                den = e.sum() + (math.exp(float(self.sink[h]) - top) if sink else 0.0)
+                out[t, h] = (e / den) @ self.v[s][:i + 1, g][see]
+        return out
+
+    def run(self, name, window, keep, chunk, rel, sink, slopes, scale, tokens=None):
+        at = slice(0, self.T) if tokens is None else tokens
+        n = len(range(*at.indices(self.T)))
+        out = torch.full((n, self.H, self.Dv), float("nan"), dtype=self.dtype, device=DEV)
+        err = torch.zeros(1, dtype=torch.int32, device=DEV)
+        dev = [t.to(DEV) for t in (self.q[at].contiguous(), self.table, self.positions[at].contiguous(), self.seq[at].contiguous(), self.rel, self.bucket, self.sink, self.slopes)]
+        q, table, pos, seq, r, b, sk, sl = dev
+        head = [_p(q), _i(self.stride), _p(self.kp), _p(self.vp), _p(table), _i(table.shape[1]), _p(pos)]
+        opts = [_p(r if rel else None), _p(b if rel else None), _i(self.far if rel else 0), _p(sk if sink else None), _p(sl if slopes else None),
+                _i(self.Dk if self.in_keys else 0), _p(out)]
+        sizes = [_i(self.H), _i(self.Hkv), _i(self.Dk), _i(self.Dv), ctypes.c_float(scale), _i(window), _i(keep), _i(chunk), _i(self.kp.shape[0])]
+        if name == "rows":
+            rc = _lib().vm_attention_sink_generic(*head, _p(seq), *opts, _i(n), *sizes, _i(0 if self.dtype == torch.float32 else 1), _p(err), _stream())
+        else:
+            rc = _lib().vm_attention_sink_decode_bf16(*head, *opts, _i(n), *sizes, _p(err), _stream())
+        assert rc == 0
+        assert int(err.item()) == 0
+        return out.cpu()
+
+
+# window, kept first tokens, chunk, bias, sink, slopes
+OPTIONS = [(0, 0, 0, False, False, False), (33, 0, 0, True, False, False), (64, 5, 0, True, True, False), (0, 0, 96, False, False, True), (40, 70, 0, False, True, True),
+           (0, 3, 64, False, False, False)]
+
+
+@pytest.mark.parametrize("H,Hkv,Dk,Dv,in_keys", [(3, 3, 64, 64, False), (9, 3, 64, 64, False), (16, 1, 160, 128, True), (10, 1, 20, 6, False), (4, 2, 128, 66, False), (17, 1, 4, 2, False)])
+@pytest.mark.parametrize("options", OPTIONS)
+def test_rows_float32(H, Hkv, Dk, Dv, in_keys, options):
+    """Whole prompts across chunk and page edges, a continued sequence, single tokens; error: 64 or more terms of 2^-24 each."""
+    s = Step(H, Hkv, Dk, Dv, [0, 130, 63, 0, 255], [100, 5, 2, 1, 1], torch.float32, in_keys)
+    scale = Dk ** -0.5
+    got, want = s.run("rows", *options, scale), s.want(*options, scale)
+    assert float((got.double() - want).abs().max()) <= 1e-5
+
+
+def test_rows_do_not_depend_on_the_batch_or_the_cut():
+    """Few tokens (a CTA per token) and many (a CTA for several), in one step and in pieces: the same bits."""
+    s = Step(6, 3, 64, 64, [0, 70, 0, 200], [150, 31, 64, 1], torch.float32)
+    whole = s.run("rows", 50, 3, 0, False, True, False, 0.125)
+    for a, b in ((0, 1), (149, 152), (140, 160), (245, 246)):
+        assert torch.equal(whole[a:b], s.run("rows", 50, 3, 0, False, True, False, 0.125, slice(a, b)))

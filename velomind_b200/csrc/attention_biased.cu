@@ -13,7 +13,7 @@
 // (k [n_pages, Hkv, VM_PAGE_TOKENS, Dk], v [n_pages, Hkv, VM_PAGE_TOKENS, Dv]).  The distance table `bucket_of` has
 // `far + 1` entries; every distance beyond `far` reads the last one.
 //
-// In the plain kernel a warp owns a (token, query head); keys are walked in chunks of 32 that start at absolute multiples
+// The plain kernel is what is left for sizes that attention_rows.cu does not take.  A warp owns a (token, query head); keys are walked in chunks of 32 that start at absolute multiples
 // of 32, one key per lane, and every dot product is summed in index order by one lane: the result for a position does not
 // depend on how the tokens were cut into steps or on what else is in the batch.
 #include "common.cuh"
@@ -229,6 +229,9 @@ VM_API int vm_attention_sink_generic(const void* q, int q_row_stride, const void
     if (n_tokens <= 0) return 0;
     if (H <= 0 || Hkv <= 0 || H % Hkv != 0 || Dk <= 0 || Dk > 2048 || Dv <= 0 || Dv > 1024 || window < 0 || keep_first < 0 || chunk < 0) return VM_ERR_UNSUPPORTED;
     if ((rel != nullptr) != (bucket_of != nullptr) || (rel && far < 0)) return VM_ERR_BAD_ARG;
+    if ((act_dtype == VM_F32 || act_dtype == VM_BF16) && vm_attention_rows_fits(kpages, vpages, H, Hkv, Dk, Dv, v_stride))
+        return vm_attention_rows(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, rel, bucket_of, far, sink, slopes, v_stride,
+                                 out, n_tokens, H, Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, act_dtype, err, stream);
     if (act_dtype == VM_F32)
         return launch_biased<float>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, rel, bucket_of, far, out, n_tokens, H,
                                     Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, sink, slopes, v_stride, err, stream);

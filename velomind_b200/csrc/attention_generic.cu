@@ -1,6 +1,6 @@
 // Attention over the paged cache, any head size / head count / group size, float32 or bf16 storage,
-// float32 arithmetic.  One warp per (token, query head); this is the kernel of the true 32-bit path
-// and the fallback for shapes the tensor-core kernels refuse.
+// float32 arithmetic.  One warp per (token, query head): what is left for head sizes that attention_rows.cu does not take
+// (not a multiple of four, or more than 128), in the true 32-bit path and where the tensor-core kernels refuse a shape.
 //
 // Reference arithmetic: examples/common/llama/llama_graph.cpp:97-103 (scores = q k^T, softmax over the
 // keys a query may see, times v) in the online form of src/cpu/ops/fused_attention.cpp:84-135.  The
@@ -114,6 +114,9 @@ VM_API int vm_attention_generic(const void* q, int q_row_stride, const void* kpa
                                 int act_dtype, int* err, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (H <= 0 || Hkv <= 0 || H % Hkv != 0 || D <= 0 || D > 512) return VM_ERR_UNSUPPORTED;
+    if ((act_dtype == VM_F32 || act_dtype == VM_BF16) && vm_attention_rows_fits(kpages, vpages, H, Hkv, D, D, D))
+        return vm_attention_rows(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, nullptr, nullptr, 0, nullptr, nullptr, D,
+                                 out, n_tokens, H, Hkv, D, D, scale, window, 0, 0, n_pages, act_dtype, err, stream);
     if (act_dtype == VM_F32)
         return launch_generic<float>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, out,
                                      n_tokens, H, Hkv, D, scale, window, n_pages, err, stream);

@@ -224,6 +224,13 @@ int vm_rope_kv_write(void* qkv, const int* positions, const int* seq_of_token, c
                      int n_pages, int act_dtype, int* err, cudaStream_t stream);
 
 // ---- attention
+// ---- attention_rows.cu: the float32 arithmetic of the plain kernels with a query's keys spread over a CTA (arguments as vm_attention_sink_generic;
+// v_stride is given); vm_attention_generic and vm_attention_sink_generic call it where it takes the sizes
+int vm_attention_rows_fits(const void* kpages, const void* vpages, int H, int Hkv, int Dk, int Dv, int v_stride);
+int vm_attention_rows(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
+                      const int* positions, const int* seq_of_token, const float* rel, const int* bucket_of, int far, const float* sink,
+                      const float* slopes, int v_stride, void* out, int n_tokens, int H, int Hkv, int Dk, int Dv, float scale, int window,
+                      int keep_first, int chunk, int n_pages, int act_dtype, int* err, cudaStream_t stream);
 int vm_attention_generic(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
                          int max_blocks, const int* positions, const int* seq_of_token, void* out, int n_tokens, int H, int Hkv,
                          int D, float scale, int window, int n_pages, int act_dtype, int* err, cudaStream_t stream);
