@@ -133,3 +133,37 @@ def test_rows_do_not_depend_on_the_batch_or_the_cut():
     whole = s.run("rows", 50, 3, 0, False, True, False, 0.125)
     for a, b in ((0, 1), (149, 152), (140, 160), (245, 246)):
         assert torch.equal(whole[a:b], s.run("rows", 50, 3, 0, False, True, False, 0.125, slice(a, b)))
+
+
+@pytest.mark.parametrize("H,Hkv,Dk,Dv,in_keys", [(8, 8, 64, 64, False), (16, 4, 64, 64, False), (4, 2, 64, 128, False), (6, 2, 96, 64, False), (4, 4, 128, 64, False), (3, 1, 96, 128, False),
+                                                 (16, 1, 128, 128, True), (20, 1, 160, 128, True), (33, 1, 192, 128, True)])
+@pytest.mark.parametrize("options", OPTIONS)
+def test_decode_tile(H, Hkv, Dk, Dv, in_keys, options):
+    """Lengths around the 32-key turns, the pages and a cluster's first round; the result is rounded to bfloat16 once (half of 2^-8 of it), and
+    sums of 32-bit terms leave 1e-5."""
+    s = Step(H, Hkv, Dk, Dv, [0, 31, 32, 63, 64, 300, 1111], [1] * 7, torch.bfloat16, in_keys, far=700)
+    scale = Dk ** -0.5
+    got, want = s.run("tile", *options, scale), s.want(*options, scale)
+    assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all())
+
+
+def test_decode_tile_with_more_sequences_than_sms():
+    """One CTA per sequence and head group, several turns of every warp."""
+    s = Step(4, 4, 64, 64, [700 - 3 * i for i in range(70)], [1] * 70, torch.bfloat16)
+    got, want = s.run("tile", 0, 0, 0, False, False, False, 0.125), s.want(0, 0, 0, False, False, False, 0.125)
+    assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all())
+
+
+def test_an_infinite_value_stays_infinite():
+    s = Step(4, 1, 64, 64, [40], [1], torch.bfloat16)
+    page, row = int(s.table[0, 0]), 7
+    s.vp[page, 0, row, 3] = float("inf")
+    got = s.run("tile", 0, 0, 0, False, False, False, 0.125)
+    assert bool(torch.isposinf(got[0, :, 3]).all()) and bool(torch.isfinite(got[0, :, 4:]).all()) and bool(torch.isfinite(got[0, :, :3]).all())
+
+
+def test_a_missing_page_is_reported():
+    s = Step(4, 1, 64, 64, [200], [1], torch.bfloat16)
+    s.table[0, 1] = -1
+    with pytest.raises(AssertionError):
+        s.run("tile", 0, 0, 0, False, False, False, 0.125)

@@ -11,7 +11,7 @@
 // added to the float32 scores from a table by distance that the CTA builds in shared memory for its head (rel[bucket(d)],
 // in the softmax's base-2 units), the mask is applied per score, the online softmax is float32.
 //
-// Decode steps.  One CTA per (sequence, query head); its warps take the visible keys in chunks of 32 (a key per lane,
+// Decode steps (of sizes that attention_decode_tile.cu does not take).  One CTA per (sequence, query head); its warps take the visible keys in chunks of 32 (a key per lane,
 // float32 dot products from 16-byte loads), keep a float32 online softmax each, and warp 0 joins the warps' results in warp
 // order: the answer does not depend on the batch.
 #include "mma.cuh"
@@ -470,6 +470,9 @@ VM_API int vm_attention_sink_decode_bf16(const void* q, int q_row_stride, const 
     if (H > 65535) return VM_ERR_UNSUPPORTED;
     const int v_stride = v_row_stride > 0 ? v_row_stride : Dv;
     if (v_stride < Dv || ((Dv % 2) == 0 && (v_stride % 2) != 0)) return VM_ERR_BAD_ARG;
+    if (vm_attention_decode_tile_fits(q, q_row_stride, kpages, vpages, B, H, Hkv, Dk, Dv, v_stride))
+        return vm_attention_decode_tile(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, rel, bucket_of, far, sink, slopes, v_stride, out, B, H,
+                                        Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, err, stream);
     const size_t smem = ((size_t)((Dk + 3) & ~3) + (size_t)DEC_WARPS * (Dv + 2)) * sizeof(float);
     const dim3 grid(B, H);
     cudaError_t e;

@@ -453,6 +453,15 @@ int decode_splits(int B, int Hkv, int G, int table_width) {
 void attention(StepContext& ctx, const void* q, int q_row_stride, const KVView& kv, void* out, int H, int Hkv, int D, float scale, int window) {
     cudaStream_t s = ctx.stream;
     const bool fast = ctx.act_dtype == DType::BF16 && D % 16 == 0 && D <= 128 && q_row_stride % 8 == 0;
+    if (fast && ctx.one_token_each && kv.v_pages == kv.k_pages && vm_attention_decode_tile_fits(q, q_row_stride, kv.k_pages, kv.v_pages, ctx.B, H, Hkv, D, D, D)) {
+        // latents that are keys and values at once, all heads on one kv head (measured, one sequence of 2,048 tokens, 16 heads of 128: 8.2 us against 21 us
+        // for the split kernel below, whose four warps a CTA take a page of 64 keys each)
+        Timed t("attention_decode_bf16", s);
+        check(vm_attention_decode_tile(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, nullptr, nullptr, 0, nullptr, nullptr,
+                                       D, out, ctx.B, H, Hkv, D, D, scale, window, 0, 0, kv.n_pages, ctx.err, s),
+              "attention_decode_bf16", s);
+        return;
+    }
     if (fast && ctx.one_token_each && static_cast<long long>(ctx.B) * H <= DECODE_COUNTERS) {
         const int n_splits = decode_splits(ctx.B, Hkv, H / Hkv, kv.table_width);
         float* partial = static_cast<float*>(ctx.take(static_cast<long long>(ctx.B_cap) * H * MAX_DECODE_SPLITS * (D + 2), DType::F32));   // sized by shape

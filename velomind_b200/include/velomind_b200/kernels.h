@@ -178,6 +178,14 @@ int vm_attention_sink_decode_bf16(const void* q, int q_row_stride, const void* k
                                   int B, int H, int Hkv, int Dk, int Dv, float scale, int window, int keep_first, int chunk, int n_pages, int* err,
                                   cudaStream_t stream);
 
+// ---- attention_decode_tile.cu: decode steps with the query heads of a kv head as one tensor-core tile; vm_attention_sink_decode_bf16 calls it
+// where it takes the sizes (v_stride: elements between value rows, given)
+int vm_attention_decode_tile_fits(const void* q, int q_row_stride, const void* kpages, const void* vpages, int B, int H, int Hkv, int Dk, int Dv, int v_stride);
+int vm_attention_decode_tile(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
+                             const int* positions, const float* rel, const int* bucket_of, int far, const float* sink, const float* slopes,
+                             int v_stride, void* out, int B, int H, int Hkv, int Dk, int Dv, float scale, int window, int keep_first, int chunk,
+                             int n_pages, int* err, cudaStream_t stream);
+
 // ---- attention_biased_fast.cu: the same attention in bfloat16: prompts on mma.sync tiles (keys and values of the sizes that
 // vm_attention_biased_prefill_fits names; n_tiles = sum over the sequences of ceil(new tokens / 64)), decode steps (token s is sequence s's)
 int vm_attention_biased_prefill_fits(int Dk, int Dv);
