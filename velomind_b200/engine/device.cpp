@@ -427,6 +427,7 @@ constexpr int MAX_DECODE_SPLITS = 16;
 constexpr int DECODE_ONE_CTA_BLOCKS = 16;     // block tables up to this wide (1,024 tokens): at most two rounds of pages for ten warps
 constexpr int TC_ATTENTION_MIN_BLOCKS = 20;   // head size 64: the tcgen05 prefill attention when a tile may see this many key blocks
 constexpr int TC_ATTENTION_CTAS_PER_SM = 3;   // CTAs of that kernel an SM holds at once (registers and shared memory)
+constexpr int WS_ATTENTION_MANY_BLOCKS = 16;  // the same for steps of many tiles
 int WS_ATTENTION_MIN_BLOCKS = 32;             // head size 64: the warp-specialised tcgen05 attention when a tile may see this many key blocks
 
 int* decode_counters() {
@@ -440,11 +441,17 @@ int* decode_counters() {
 
 // How many CTAs share the keys of one (sequence, kv head): enough to fill the GPU, a function of the step's SHAPE only
 // (so that a recorded launch stays valid as sequences grow).
-int decode_splits(int B, int Hkv, int G, int table_width) {
+int decode_splits(int B, int Hkv, int G, int D, int table_width) {
     const int groups = B * Hkv * ((G + 15) / 16);           // a CTA serves up to 16 query heads of one kv head
     const int sms = sm_count();
     if (groups <= sms && table_width <= DECODE_ONE_CTA_BLOCKS) return 1;   // short sequences: one CTA of ten warps holds all pages
-    const int want = (sms + groups - 1) / groups;            // about one CTA per SM ...
+    // More than half the SMs have a CTA of their own: ten warps (whose pages fit shared memory up to heads of 64) walk the pages, and nothing is joined across CTAs (measured, 80 groups of 3 heads of
+    // 64: 1,100 tokens 7.2 us against 11.2 us in two splits of four warps, 2,000 tokens 11.6 / 14.8; 128 groups, 2,000 tokens 12.3 / 14.1).
+    if (D <= 64 && groups <= sms && 2 * groups > sms) return 1;
+    // Else about one CTA per SM, in powers of two (24 groups, 2,000 tokens: 8 splits 7.2 us, 7 splits 8.4 us; 64 groups: 4 splits 9.0 us, 3 splits
+    // 10.7 us) ...
+    int want = 1;
+    while (want * groups < sms) want *= 2;
     const int by_width = std::max(1, table_width / 4);       // ... and at least a page per warp of a CTA (the width bounds the pages)
     return std::max(1, std::min(want, std::min(MAX_DECODE_SPLITS, by_width)));
 }
@@ -463,7 +470,7 @@ void attention(StepContext& ctx, const void* q, int q_row_stride, const KVView& 
         return;
     }
     if (fast && ctx.one_token_each && static_cast<long long>(ctx.B) * H <= DECODE_COUNTERS) {
-        const int n_splits = decode_splits(ctx.B, Hkv, H / Hkv, kv.table_width);
+        const int n_splits = decode_splits(ctx.B, Hkv, H / Hkv, D, kv.table_width);
         float* partial = static_cast<float*>(ctx.take(static_cast<long long>(ctx.B_cap) * H * MAX_DECODE_SPLITS * (D + 2), DType::F32));   // sized by shape
         {
             Timed t("attention_decode_bf16", s);
@@ -485,7 +492,10 @@ void attention(StepContext& ctx, const void* q, int q_row_stride, const KVView& 
             tiles128 += (n + 127) / 128;
             tiles64 += (n + 63) / 64;
         }
-        if (D == 64 && most_blocks >= WS_ATTENTION_MIN_BLOCKS && ctx.err != nullptr) {
+        // (many tiles of middling length keep that kernel's CTAs busy too: eight prompts of 576 to 1,024 tokens and 15 heads 44 us against 61 us for the
+        //  mma.sync kernel, four of 1,024 and 32 heads 75 / 90; one of 1,024 and 9 heads 22 / 17, eight of 512 33 / 22)
+        const bool many = most_blocks >= WS_ATTENTION_MANY_BLOCKS && tiles128 * H >= 3ll * sm_count();
+        if (D == 64 && (most_blocks >= WS_ATTENTION_MIN_BLOCKS || many) && ctx.err != nullptr) {
             // the longest prompts: softmax warps, a copy warp and product warps, clusters dealt out to pairs of tile groups
             // (measured, 9 heads: 4,096 tokens 78 us against 88 us for the kernel below, 8,192: 224 / 262; 2,048: 32 / 33;
             //  2,560: 37 / 48, 3,072: 51 / 58, 1,536: 27 / 24, 1,024: 22 / 18: every CTA pays for its set-up and its cluster's exchange once, whatever its share of the keys;
@@ -510,7 +520,9 @@ void attention(StepContext& ctx, const void* q, int q_row_stride, const KVView& 
                   "attention_prefill_tc_bf16", s);
             return;
         }
-        const int groups = most_blocks >= 8 ? 2 : 1;      // measured at 9 heads of 64: 2 groups 39 us, 1 group 43 us, 4 groups 46 us (2,048 tokens)
+        // two groups of warps share a tile's keys where the tiles are long and too few to fill the GPU (measured, 9 heads of 64: one prompt of 2,048 tokens
+        // 40.0 us with two groups, 43.8 us with one, of 1,024 tokens 17.3 / 20.2; of 300 tokens 8.2 / 7.9, sixteen of 40 to 295 16.4 / 12.2, eight of 512 25.1 / 22.2)
+        const int groups = most_blocks >= 16 && tiles64 * H <= 2ll * sm_count() ? 2 : 1;
         Timed t("attention_prefill_bf16", s);
         check(vm_attention_prefill_bf16(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, ctx.cu_tokens, ctx.B,
                                         static_cast<int>(tiles64), out, H, Hkv, D, scale, window, kv.n_pages, ctx.err, groups, s),

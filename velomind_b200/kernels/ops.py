@@ -223,14 +223,18 @@ def decode_counters(device) -> torch.Tensor:
 DECODE_ONE_CTA_BLOCKS = 16     # block tables up to this wide (1,024 tokens): at most two rounds of pages for ten warps
 
 
-def decode_splits(B: int, Hkv: int, G: int, table_width: int, device=None) -> int:
+def decode_splits(B: int, Hkv: int, G: int, table_width: int, device=None, D: int = 64) -> int:
     """How many CTAs share the keys of one (sequence, kv head): enough to fill the GPU, a function of the
     step's SHAPE only (so that a captured launch stays valid as sequences grow)."""
     groups = B * Hkv * (-(-G // 16))          # a CTA serves up to 16 query heads of one kv head
     sms = sm_count(device)
     if groups <= sms and table_width <= DECODE_ONE_CTA_BLOCKS:
         return 1                              # short sequences: one CTA of ten warps holds all pages, nothing is merged across CTAs
-    want = -(-sms // groups)                  # about one CTA per SM ...
+    if D <= 64 and groups <= sms and 2 * groups > sms:
+        return 1                              # a CTA of ten warps on more than half the SMs
+    want = 1                                  # about one CTA per SM, in powers of two ...
+    while want * groups < sms:
+        want *= 2
     table_width = max(1, table_width // 4)    # ... and at least a page per warp of a CTA (the width bounds the pages)
     return max(1, min(want, MAX_DECODE_SPLITS, table_width))
 
