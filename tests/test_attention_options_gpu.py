@@ -92,6 +92,15 @@ class Step:
                 out[t, h] = (e / den) @ self.v[s][:i + 1, g][see]
         return out
 
+    def want_some(self, tokens, heads, *options):
+        """`want` for some tokens and heads."""
+        few = Step.__new__(Step)
+        few.__dict__.update(self.__dict__)
+        few.T, few.positions, few.seq, few.q = len(tokens), self.positions[tokens], self.seq[tokens], self.q[tokens]
+        n = len(range(*heads.indices(self.H)))
+        few.H, few.Hkv = n, max(1, n // (self.H // self.Hkv)) if n < self.H else self.Hkv
+        return few.want(*options)
+
     def run(self, name, window, keep, chunk, rel, sink, slopes, scale, tokens=None):
         at = slice(0, self.T) if tokens is None else tokens
         n = len(range(*at.indices(self.T)))
@@ -103,7 +112,11 @@ class Step:
         opts = [_p(r if rel else None), _p(b if rel else None), _i(self.far if rel else 0), _p(sk if sink else None), _p(sl if slopes else None),
                 _i(self.Dk if self.in_keys else 0), _p(out)]
         sizes = [_i(self.H), _i(self.Hkv), _i(self.Dk), _i(self.Dv), ctypes.c_float(scale), _i(window), _i(keep), _i(chunk), _i(self.kp.shape[0])]
-        if name == "rows":
+        if name == "prompt":
+            new = torch.bincount(self.seq.long(), minlength=len(self.new)).tolist()
+            cu = torch.tensor([0] + list(np.cumsum(new)), dtype=torch.int32, device=DEV)
+            rc = _lib().vm_attention_sink_prefill_bf16(*head, _p(cu), _i(len(new)), _i(sum(-(-m // 64) for m in new)), *opts[:3], _i(7 if rel else 0), *opts[3:], *sizes, _p(err), _stream())
+        elif name == "rows":
             rc = _lib().vm_attention_sink_generic(*head, _p(seq), *opts, _i(n), *sizes, _i(0 if self.dtype == torch.float32 else 1), _p(err), _stream())
         else:
             rc = _lib().vm_attention_sink_decode_bf16(*head, *opts, _i(n), *sizes, _p(err), _stream())
@@ -167,3 +180,18 @@ def test_a_missing_page_is_reported():
     s.table[0, 1] = -1
     with pytest.raises(AssertionError):
         s.run("tile", 0, 0, 0, False, False, False, 0.125)
+
+
+@pytest.mark.parametrize("H,Hkv,Dk,Dv,in_keys", [(4, 2, 64, 64, False), (80, 20, 64, 64, False), (3, 1, 96, 64, True), (2, 1, 160, 128, True), (70, 1, 128, 128, True), (2, 2, 64, 128, False),
+                                                 (4, 4, 32, 16, False)])
+@pytest.mark.parametrize("options", OPTIONS[1:] + [(0, 0, 0, True, False, True)])
+def test_prompt(H, Hkv, Dk, Dv, in_keys, options):
+    """Prompts around the edges of the 64-row tiles and of the masks: blocks that every row of a warp sees whole and blocks that it does not.  Probabilities are rounded to
+    bfloat16 (2^-9 each of values around 1) and so is the result."""
+    s = Step(H, Hkv, Dk, Dv, [0, 130, 63, 0, 0], [130, 5, 70, 1, 129], torch.bfloat16, in_keys, far=300)
+    scale = Dk ** -0.5
+    keep = slice(0, 2) if H > 8 else slice(0, H)                       # (heads compared: the reference is slow)
+    got = s.run("prompt", *options, scale)
+    t = torch.tensor([0, 63, 64, 127, 128, 129, 130, 134, 135, 204, 205, 206, 270, 334])
+    whole = s.want_some(t, keep, *options, scale)
+    assert bool(((got[t][:, keep].double() - whole).abs() <= whole.abs() * 2.0 ** -8 + 6e-3 * float(whole.abs().max())).all())

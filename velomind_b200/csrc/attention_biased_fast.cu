@@ -9,7 +9,11 @@
 // arrive one cache page (64 tokens of one kv head) at a time through cp.async into double-buffered shared memory, keys with
 // DK values a row and values with DV.  Q K^T and P V run on mma.sync m16n8k16 (bf16 in, float32 accumulate); the bias is
 // added to the float32 scores from a table by distance that the CTA builds in shared memory for its head (rel[bucket(d)],
-// in the softmax's base-2 units), the mask is applied per score, the online softmax is float32.
+// in the softmax's base-2 units), the mask is applied per score, the online softmax is float32.  What bounds it is the chain of a block (products,
+// maximum, exponentials, products) at the few warps an SM holds: so the query operands stay in registers, a block has one barrier, and a block
+// that every row of a warp sees whole takes no mask.  Measured against two barriers, operands from shared memory and a mask on every score:
+// 1,400 + 2,000 tokens of 32 heads of 64 with slopes 144 -> 116 us, over a latent of 160 values 267 -> 226; eight prompts of 130 to 509 tokens,
+// 16 heads and a table 31.3 -> 26.5; four of 301 to 850 with a sink 39.6 -> 33.2; eight of 512, chunked, 42.3 -> 36.7.
 //
 // Decode steps (of sizes that attention_decode_tile.cu does not take).  One CTA per (sequence, query head); its warps take the visible keys in chunks of 32 (a key per lane,
 // float32 dot products from 16-byte loads), keep a float32 online softmax each, and warp 0 joins the warps' results in warp
@@ -35,7 +39,7 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
-// VK: a token's value is the first DV values of its key row (one pool, one tile in shared memory: nothing else is fetched for the values)
+// VK: a token's value is the first DV values of its key row (one pool, one tile in shared memory: nothing else is fetched for the values).
 template <int DK, int DV, bool VK>
 __global__ void __launch_bounds__(128)
 attn_biased_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __nv_bfloat16* __restrict__ kpages,
@@ -56,7 +60,7 @@ attn_biased_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride
     const bool biased = rel != nullptr, sloped = slopes != nullptr;
     const bool direct = biased && far + 1 <= DIRECT_TABLE_MAX;
 
-    // ---- which 64 tokens of which sequence (the last tiles of a sequence see the most keys: they are started first)
+    // ---- which BM tokens of which sequence (the last tiles of a sequence see the most keys: they are started first)
     int tile = gridDim.x - 1 - blockIdx.x, seq = 0, t0 = 0, n_rows = 0;
     for (; seq < B; ++seq) {
         const int a = cu_tokens[seq], b = cu_tokens[seq + 1];
@@ -76,8 +80,8 @@ attn_biased_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride
     const int n_steps = kept_blocks + (blk_hi - blk_lo + 1);
     const int* table = block_table + (size_t)seq * max_blocks;
 
-    if (biased) {
-        if (direct) for (int d = tid; d <= far; d += THREADS) sBias[d] = rel[(size_t)bucket_of[d] * H + h] * LOG2E;
+    if (biased) {                                          // (no distance in this tile is above hi)
+        if (direct) for (int d = tid; d <= min(far, hi); d += THREADS) sBias[d] = rel[(size_t)bucket_of[d] * H + h] * LOG2E;
         else for (int r = tid; r < rel_rows; r += THREADS) sBias[r] = rel[(size_t)r * H + h] * LOG2E;
     }
     // ---- Q tile -> shared (rows past the sequence's end are zero)
@@ -89,153 +93,163 @@ attn_biased_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride
     auto load_kv = [&](int step, int buf) {
         const int blk = block_of(step);
         int page = (blk < max_blocks) ? table[blk] : -1;
-        const bool ok = (page >= 0 && page < n_pages);
+        bool ok = (page >= 0 && page < n_pages);
         if (!ok) { if (tid == 0 && err) atomicExch(err, VM_ERRWORD_CACHE_READ); page = 0; }
+        const int live = ok ? hi - blk * BN + 1 : 0;       // rows behind the tile's last token hold nothing yet: zeros
         const __nv_bfloat16* kg = kpages + ((size_t)page * Hkv + hk) * BN * DK;
         const __nv_bfloat16* vg = vpages + ((size_t)page * Hkv + hk) * BN * DV;
         __nv_bfloat16* ks = sK + (size_t)buf * BN * KP;
         __nv_bfloat16* vs = sV + (size_t)buf * BN * VP;
+#pragma unroll
         for (int c = tid; c < BN * KCH; c += THREADS) {
             const int r = c / KCH, ch = c - r * KCH;
-            cp_async16_zfill(ks + r * KP + ch * 8, kg + r * DK + ch * 8, ok);
+            cp_async16_zfill(ks + r * KP + ch * 8, kg + r * DK + ch * 8, r < live);
         }
         if (!VK)
+#pragma unroll
             for (int c = tid; c < BN * VCH; c += THREADS) {
                 const int r = c / VCH, ch = c - r * VCH;
-                cp_async16_zfill(vs + r * VP + ch * 8, vg + r * DV + ch * 8, ok);
+                cp_async16_zfill(vs + r * VP + ch * 8, vg + r * DV + ch * 8, r < live);
             }
     };
     load_kv(0, 0);
     vm_cp_async_commit();
 
-    // ---- per-thread state: rows g and g+8 of the warp's 16 rows
+    // ---- per-thread state: rows g and g + 8 of the warp's 16 rows
     const int g = lane >> 2, t4 = lane & 3;
-    const int row_a = warp * 16 + g, row_b = row_a + 8;
-    const int pos_a = pos0 + row_a, pos_b = pos0 + row_b;
-    const int lo_a = vm_first_seen(pos_a, window, chunk), lo_b = vm_first_seen(pos_b, window, chunk);
-    float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.f, l_b = 0.f;
+    const int row0 = warp * 16 + g;
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
     float o[DV / 8][4];
 #pragma unroll
-    for (int i = 0; i < DV / 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
+    for (int j = 0; j < DV / 8; ++j) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
     unsigned qa[DK / 16][4];
-    bool q_loaded = false;
     const int warp_min_pos = pos0 + warp * 16, warp_max_pos = warp_min_pos + 15;
-    const int warp_lo = vm_first_seen(warp_min_pos, window, chunk);
+    const int warp_lo = vm_first_seen(warp_min_pos, window, chunk), warp_lo_last = vm_first_seen(warp_max_pos, window, chunk);
     const float slope_log2 = sloped ? slopes[h] * LOG2E : 0.f;
 
     for (int step = 0; step < n_steps; ++step) {
         const int buf = step & 1;
         const int blk = block_of(step);
+        vm_cp_async_wait_all();
+        __syncthreads();          // the block is here, and everyone is done with the other buffer
         if (step + 1 < n_steps) load_kv(step + 1, buf ^ 1);
         vm_cp_async_commit();
-        cp_async_wait_n<1>();
-        __syncthreads();
-        if (!q_loaded) {
+        if (step == 0) {
 #pragma unroll
             for (int kk = 0; kk < DK / 16; ++kk)
-                vm_ldmatrix_x4(qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3],
-                               sQ + (warp * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)) * KP + kk * 16 + 8 * (lane >> 4));
-            q_loaded = true;
+                vm_ldmatrix_x4(qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], sQ + (warp * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)) * KP + kk * 16 + 8 * (lane >> 4));
         }
         const int key0 = blk * BN;
         // does any row of this warp see any key of this page?  (its first row reaches lowest)
         const bool in_reach = key0 <= warp_max_pos && (key0 + BN - 1 >= warp_lo || key0 < keep_first);
-        if (in_reach && warp * 16 < n_rows) {
-            const __nv_bfloat16* ks = sK + (size_t)buf * BN * KP;
-            const __nv_bfloat16* vs = VK ? ks : sV + (size_t)buf * BN * VP;
-            float s[BN / 8][4];
+        if (!in_reach || warp * 16 >= n_rows) continue;
+        const __nv_bfloat16* ks = sK + (size_t)buf * BN * KP;
+        const __nv_bfloat16* vs = VK ? ks : sV + (size_t)buf * BN * VP;
+        float s[BN / 8][4];
 #pragma unroll
-            for (int nb = 0; nb < BN / 8; ++nb) { s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f; }
+        for (int nb = 0; nb < BN / 8; ++nb) { s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f; }
 #pragma unroll
-            for (int kk = 0; kk < DK / 16; ++kk) {
+        for (int kk = 0; kk < DK / 16; ++kk)
 #pragma unroll
-                for (int nb = 0; nb < BN / 8; nb += 2) {
-                    unsigned b0, b1, b2, b3;
-                    vm_ldmatrix_x4(b0, b1, b2, b3, ks + (nb * 8 + (lane & 7) + 8 * (lane >> 4)) * KP + kk * 16 + 8 * ((lane >> 3) & 1));
-                    vm_mma_bf16_16816(s[nb], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], b0, b1);
-                    vm_mma_bf16_16816(s[nb + 1], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], b2, b3);
-                }
+            for (int nb = 0; nb < BN / 8; nb += 2) {
+                unsigned b0, b1, b2, b3;
+                vm_ldmatrix_x4(b0, b1, b2, b3, ks + (nb * 8 + (lane & 7) + 8 * (lane >> 4)) * KP + kk * 16 + 8 * ((lane >> 3) & 1));
+                vm_mma_bf16_16816(s[nb], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], b0, b1);
+                vm_mma_bf16_16816(s[nb + 1], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], b2, b3);
             }
-            // ---- scale, bias and mask, in base-2 units: t = s * scale * log2(e) + bias * log2(e)
+        // ---- scale, bias and mask, in base-2 units: t = s * scale * log2(e) + bias * log2(e).  Where every row of the warp sees every key (all
+        // blocks but the masks' edges) there is no mask, and a bias is one look-up at a fixed offset, a slope one product
+        const bool inside = key0 + BN - 1 <= warp_min_pos && (key0 >= warp_lo_last || key0 + BN <= keep_first) &&
+                            (!biased || (direct && warp_max_pos - key0 <= far));
 #pragma unroll
-            for (int nb = 0; nb < BN / 8; ++nb) {
+        for (int j = 0; j < 2; ++j) {
+            const int pos = pos0 + row0 + 8 * j;
+            if (inside) {
+                const float* by_distance = sBias + (pos - key0 - 2 * t4);
+                const float away = -slope_log2 * (float)(pos - key0 - 2 * t4);
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int key = key0 + nb * 8 + 2 * t4 + e;
-                    const bool see_a = key <= pos_a && (key >= lo_a || key < keep_first);
-                    const bool see_b = key <= pos_b && (key >= lo_b || key < keep_first);
-                    float ba = 0.f, bb = 0.f;
-                    if (biased) {
-                        const int da = min(max(pos_a - key, 0), far), db = min(max(pos_b - key, 0), far);
-                        ba = direct ? sBias[da] : sBias[bucket_of[da]];
-                        bb = direct ? sBias[db] : sBias[bucket_of[db]];
+                for (int nb = 0; nb < BN / 8; ++nb)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        float& x = s[nb][2 * j + e];
+                        if (biased) {
+                            x = fmaf(x, scale_log2, by_distance[-(nb * 8 + e)]);
+                            if (sloped) x += fmaf(slope_log2, (float)(nb * 8 + e), away);
+                        } else if (sloped) {
+                            x = fmaf(x, scale_log2, fmaf(slope_log2, (float)(nb * 8 + e), away));
+                        } else {
+                            x *= scale_log2;
+                        }
                     }
-                    if (sloped) {
-                        ba = fmaf(-slope_log2, (float)(pos_a - key), ba);
-                        bb = fmaf(-slope_log2, (float)(pos_b - key), bb);
+            } else {
+                const int lo_r = vm_first_seen(pos, window, chunk);
+#pragma unroll
+                for (int nb = 0; nb < BN / 8; ++nb)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int key = key0 + nb * 8 + 2 * t4 + e;
+                        const bool see = key <= pos && (key >= lo_r || key < keep_first);
+                        float bias = 0.f;
+                        if (biased) {
+                            const int d = min(min(max(pos - key, 0), far), hi);
+                            bias = direct ? sBias[d] : sBias[bucket_of[d]];
+                        }
+                        if (sloped) bias = fmaf(-slope_log2, (float)(pos - key), bias);
+                        float& x = s[nb][2 * j + e];
+                        x = see ? fmaf(x, scale_log2, bias) : -INFINITY;
                     }
-                    s[nb][e] = see_a ? fmaf(s[nb][e], scale_log2, ba) : -INFINITY;
-                    s[nb][2 + e] = see_b ? fmaf(s[nb][2 + e], scale_log2, bb) : -INFINITY;
-                }
-            }
-            float mx_a = -INFINITY, mx_b = -INFINITY;
-#pragma unroll
-            for (int nb = 0; nb < BN / 8; ++nb) {
-                mx_a = fmaxf(mx_a, fmaxf(s[nb][0], s[nb][1]));
-                mx_b = fmaxf(mx_b, fmaxf(s[nb][2], s[nb][3]));
-            }
-            mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 1)); mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 2));
-            mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 1)); mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 2));
-            const float mn_a = fmaxf(m_a, mx_a), mn_b = fmaxf(m_b, mx_b);
-            const float use_a = (mn_a == -INFINITY) ? 0.f : mn_a, use_b = (mn_b == -INFINITY) ? 0.f : mn_b;   // row sees nothing yet
-            const float al_a = fast_exp2(m_a - use_a), al_b = fast_exp2(m_b - use_b);
-            float sum_a = 0.f, sum_b = 0.f;
-            unsigned pa[BN / 16][4];
-#pragma unroll
-            for (int nb = 0; nb < BN / 8; ++nb) {
-                const float p0 = fast_exp2(s[nb][0] - use_a), p1 = fast_exp2(s[nb][1] - use_a);
-                const float p2 = fast_exp2(s[nb][2] - use_b), p3 = fast_exp2(s[nb][3] - use_b);
-                sum_a += p0 + p1; sum_b += p2 + p3;
-                pa[nb >> 1][(nb & 1) * 2 + 0] = vm_pack_bf16(p0, p1);
-                pa[nb >> 1][(nb & 1) * 2 + 1] = vm_pack_bf16(p2, p3);
-            }
-            l_a = l_a * al_a + sum_a; l_b = l_b * al_b + sum_b;          // per-thread partial sums; quads are joined at the end
-            m_a = mn_a; m_b = mn_b;
-#pragma unroll
-            for (int i = 0; i < DV / 8; ++i) { o[i][0] *= al_a; o[i][1] *= al_a; o[i][2] *= al_b; o[i][3] *= al_b; }
-            // ---- O += P V
-#pragma unroll
-            for (int kk = 0; kk < BN / 16; ++kk) {
-#pragma unroll
-                for (int nb = 0; nb < DV / 8; nb += 2) {
-                    unsigned b0, b1, b2, b3;
-                    vm_ldmatrix_x4_trans(b0, b1, b2, b3, vs + (kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)) * VP + nb * 8 + 8 * (lane >> 4));
-                    vm_mma_bf16_16816(o[nb], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b0, b1);
-                    vm_mma_bf16_16816(o[nb + 1], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b2, b3);
-                }
             }
         }
-        __syncthreads();          // everyone is done with `buf` before the next iteration's prefetch overwrites it
-    }
-    vm_cp_async_wait_all();
-
-    l_a += __shfl_xor_sync(0xffffffffu, l_a, 1); l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
-    l_b += __shfl_xor_sync(0xffffffffu, l_b, 1); l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
-    float inv_a = 1.f / l_a, inv_b = 1.f / l_b;
-    if (sink) {                                            // exp(sink) joins the denominator (scores here are in base-2 units)
-        const float sk = sink[h] * LOG2E;
-        const float top_a = fmaxf(m_a, sk), top_b = fmaxf(m_b, sk);
-        const float keep_a = fast_exp2(m_a - top_a), keep_b = fast_exp2(m_b - top_b);
-        inv_a = keep_a / (l_a * keep_a + fast_exp2(sk - top_a));
-        inv_b = keep_b / (l_b * keep_b + fast_exp2(sk - top_b));
+        // ---- online softmax
+        unsigned pa[BN / 16][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            float mx = -INFINITY;
+#pragma unroll
+            for (int nb = 0; nb < BN / 8; ++nb) mx = fmaxf(mx, fmaxf(s[nb][2 * j], s[nb][2 * j + 1]));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1)); mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float top = fmaxf(m[j], mx);
+            const float use = (top == -INFINITY) ? 0.f : top;      // the row sees nothing yet
+            const float al = fast_exp2(m[j] - use);
+            float sum = 0.f;
+#pragma unroll
+            for (int nb = 0; nb < BN / 8; ++nb) {
+                const float p0 = fast_exp2(s[nb][2 * j] - use), p1 = fast_exp2(s[nb][2 * j + 1] - use);
+                sum += p0 + p1;
+                pa[nb >> 1][(nb & 1) * 2 + j] = vm_pack_bf16(p0, p1);
+            }
+            l[j] = l[j] * al + sum;              // per-thread partial sums; quads are joined at the end
+            m[j] = top;
+#pragma unroll
+            for (int nb = 0; nb < DV / 8; ++nb) { o[nb][2 * j] *= al; o[nb][2 * j + 1] *= al; }
+        }
+        // ---- O += P V
+#pragma unroll
+        for (int kk = 0; kk < BN / 16; ++kk) {
+#pragma unroll
+            for (int nb = 0; nb < DV / 8; nb += 2) {
+                unsigned b0, b1, b2, b3;
+                vm_ldmatrix_x4_trans(b0, b1, b2, b3, vs + (kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)) * VP + nb * 8 + 8 * (lane >> 4));
+                vm_mma_bf16_16816(o[nb], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b0, b1);
+                vm_mma_bf16_16816(o[nb + 1], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b2, b3);
+            }
+        }
     }
 #pragma unroll
-    for (int i = 0; i < DV / 8; ++i) {
-        const int d = i * 8 + 2 * t4;
-        if (row_a < n_rows)
-            *reinterpret_cast<unsigned*>(out + ((size_t)(t0 + row_a) * H + h) * DV + d) = vm_pack_bf16(o[i][0] * inv_a, o[i][1] * inv_a);
-        if (row_b < n_rows)
-            *reinterpret_cast<unsigned*>(out + ((size_t)(t0 + row_b) * H + h) * DV + d) = vm_pack_bf16(o[i][2] * inv_b, o[i][3] * inv_b);
+    for (int j = 0; j < 2; ++j) {
+        const int row = row0 + 8 * j;
+        float sum = l[j];
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1); sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        float inv = 1.f / sum;
+        if (sink) {                                    // exp(sink) joins the denominator (scores here are in base-2 units)
+            const float sk = sink[h] * LOG2E, top = fmaxf(m[j], sk), keep = fast_exp2(m[j] - top);
+            inv = keep / (sum * keep + fast_exp2(sk - top));
+        }
+        if (row < n_rows)
+#pragma unroll
+            for (int nb = 0; nb < DV / 8; ++nb)
+                *reinterpret_cast<unsigned*>(out + ((size_t)(t0 + row) * H + h) * DV + nb * 8 + 2 * t4) =
+                    vm_pack_bf16(o[nb][2 * j] * inv, o[nb][2 * j + 1] * inv);
     }
 }
 
@@ -432,7 +446,7 @@ VM_API int vm_attention_sink_prefill_bf16(const void* q, int q_row_stride, const
     if (n_tiles <= 0 || B <= 0) return 0;
     if (H <= 0 || Hkv <= 0 || H % Hkv != 0 || (q_row_stride % 8) != 0 || window < 0 || keep_first < 0 || chunk < 0) return VM_ERR_UNSUPPORTED;
     if ((rel != nullptr) != (bucket_of != nullptr) || (rel && (far < 0 || rel_rows <= 0))) return VM_ERR_BAD_ARG;
-    const bool in_keys = vpages == kpages && v_row_stride == Dk && Dv < Dk;
+    const bool in_keys = vpages == kpages && v_row_stride == Dk && (Dv < Dk || (Dk == 128 && Dv == 128));
     if (!in_keys && v_row_stride != 0 && v_row_stride != Dv) return VM_ERR_UNSUPPORTED;
 #define VM_BP(K, V, IN)                                                                                                                        \
     if (Dk == K && Dv == V && in_keys == IN)                                                                                                   \
@@ -445,7 +459,7 @@ VM_API int vm_attention_sink_prefill_bf16(const void* q, int q_row_stride, const
     VM_BP(32, 16, true) VM_BP(48, 16, true) VM_BP(80, 16, true)
     VM_BP(48, 32, true) VM_BP(64, 32, true) VM_BP(96, 32, true)
     VM_BP(80, 64, true) VM_BP(96, 64, true) VM_BP(128, 64, true)
-    VM_BP(144, 128, true) VM_BP(160, 128, true) VM_BP(192, 128, true)
+    VM_BP(128, 128, true) VM_BP(144, 128, true) VM_BP(160, 128, true) VM_BP(192, 128, true)
 #undef VM_BP
     return VM_ERR_UNSUPPORTED;
 }
