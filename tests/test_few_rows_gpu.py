@@ -1,0 +1,128 @@
+"""The kernels of a decode step's few rows against the same in 64 bits: the routers (csrc/expert_router.cu) and the experts on tensor-core tiles
+(csrc/routed_experts_tile.cu)."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _lib():
+    from velomind_b200.kernels.library import library
+    return library()
+
+
+def _p(t):
+    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+
+
+def _i(v):
+    return ctypes.c_int(int(v))
+
+
+def _f(v):
+    return ctypes.c_float(v)
+
+
+def _stream():
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def _choice(z, kind, top, groups, keep, gtop, correction, normalize, scale):
+    if kind == "chosen":
+        v, i = z.topk(top, -1)
+        return i, torch.softmax(v, -1)
+    s = torch.softmax(z, -1) if kind == "softmax" else torch.sigmoid(z)
+    c = s if correction is None else s + correction
+    if groups > 1:
+        by = c.reshape(len(z), groups, -1)
+        best = by.topk(gtop, -1).values.sum(-1).topk(keep, -1).indices
+        mask = torch.zeros(len(z), groups, dtype=torch.bool, device=z.device).scatter_(1, best, True)
+        c = by.masked_fill(~mask[..., None], -1e9).reshape(c.shape)
+    i = c.topk(top, -1).indices
+    w = s.gather(1, i)
+    return i, w / (w.sum(-1, keepdim=True) + 1e-20) * scale if normalize else w * scale
+
+
+@pytest.mark.parametrize("T", [1, 8, 149, 163, 700])
+@pytest.mark.parametrize("hidden,n_out,top,kind", [(1024, 16, 4, "chosen"), (96, 18, 4, "softmax"), (2048, 32, 4, "sigmoid"), (64, 5, 2, "chosen"), (160, 64, 6, "sigmoid"), (72, 9, 3, "softmax")])
+def test_routers(T, hidden, n_out, top, kind):
+    """One block per token and tiles of sixteen tokens, with a gate row behind the outputs (`chosen`) and with groups: the choice, where no two
+    outputs come close, and the weights (float32 sums of `hidden` terms)."""
+    g = torch.Generator().manual_seed(T + hidden)
+    x = torch.randn(T, hidden, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(n_out, hidden, generator=g) * 2.0 / hidden ** 0.5).to(DEV)
+    chosen, weight = torch.full((T, top), -1, dtype=torch.int32, device=DEV), torch.full((T, top), float("nan"), device=DEV)
+    z = x.double() @ w.double().T
+    if kind == "chosen":
+        b, gate = torch.randn(n_out, generator=g).to(DEV), torch.randn(hidden, generator=g).to(DEV) / hidden ** 0.5
+        sg = torch.full((T,), float("nan"), device=DEV)
+        assert _lib().vm_expert_router(_p(x), None, _f(0), _p(w), _p(b), _p(gate), _i(T), _i(hidden), _i(n_out), _i(top), _p(chosen), _p(weight), _p(sg), _i(1), _stream()) == 0
+        want = _choice(z + b.double(), kind, top, 1, 1, 1, None, False, 1.0)
+        assert float((sg.double() - torch.sigmoid(x.double() @ gate.double())).abs().max()) <= 1e-6
+    else:
+        groups = 2 if n_out % 2 == 0 and n_out // 2 >= top else 1
+        corr = (torch.randn(n_out, generator=g) * 0.01).to(DEV) if kind == "softmax" else None
+        gtop = 2 if kind == "sigmoid" and groups > 1 else 1
+        assert _lib().vm_expert_router_groups(_p(x), None, _f(0), _p(w), _p(corr), _i(T), _i(hidden), _i(n_out), _i(top), _i(groups), _i(1), _i(gtop), _f(1.5),
+                                              _i(0 if kind == "softmax" else 1), _i(1 if kind == "sigmoid" else 0), _p(chosen), _p(weight), _i(1), _stream()) == 0
+        want = _choice(z, kind, top, groups, 1, gtop, None if corr is None else corr.double(), kind == "sigmoid", 1.5)
+    same = (chosen.long() == want[0]).all(-1)
+    assert float(same.float().mean()) >= 0.99                       # (near ties may fall either way)
+    assert float((weight.double() - want[1])[same].abs().max()) <= 4e-6
+
+
+@pytest.mark.parametrize("T", [1, 8, 17, 33, 70])
+@pytest.mark.parametrize("hidden,ff,sff,top,E,ident,glu", [(64, 32, 0, 2, 6, 0, 0), (1024, 512, 1024, 4, 16, 0, 0), (128, 288, 0, 4, 16, 2, 1), (96, 64, 32, 3, 5, 0, 2), (2400, 96, 64, 4, 40, 0, 3)])
+def test_experts_tile(T, hidden, ff, sff, top, E, ident, glu):
+    """Few and many tokens of an expert, pieces of the contraction that end early, identity experts, every kind of gate; the unit and the result are
+    rounded to bfloat16."""
+    g = torch.Generator().manual_seed(T + ff)
+    bf = lambda *s, scale=1.0: (torch.randn(*s, generator=g) * scale).to(torch.bfloat16).to(DEV)
+    x, up, down = bf(T, hidden), bf(E, (2 if glu else 1) * ff, hidden, scale=hidden ** -0.5), bf(E, hidden, ff, scale=ff ** -0.5)
+    s_gated = glu >= 2
+    s_up = bf((2 if s_gated else 1) * sff, hidden, scale=hidden ** -0.5) if sff else None
+    s_down = bf(hidden, sff, scale=sff ** -0.5) if sff else None
+    chosen = torch.stack([torch.randperm(E + ident, generator=g)[:top] for _ in range(T)]).int().to(DEV)
+    weight = torch.rand(T, top, generator=g).to(DEV)
+    sg = torch.rand(T, generator=g).to(DEV) if glu == 0 and sff else None
+    limit, alpha = 1.0, 1.702
+    r = lambda t: t.to(torch.bfloat16).double()
+
+    def unit(z, w, gated, kind):
+        if not gated:
+            return r(torch.relu(z) ** 2)
+        a, b = z.chunk(2, -1)
+        if kind == 1:
+            a, b = r(a).clamp(max=limit), r(b).clamp(-limit, limit)
+            return r(a * torch.sigmoid(alpha * a) * (b + 1))
+        a, b = w * r(a), w * r(b)
+        return r(a * torch.sigmoid(a) * b)
+
+    want = torch.zeros(T, hidden, dtype=torch.float64, device=DEV)
+    for t in range(T):
+        for k in range(top):
+            e, w = int(chosen[t, k]), weight[t, k].double()
+            if e >= E:
+                want[t] += w * x[t].double()
+                continue
+            a = unit(up[e].double() @ x[t].double(), w if glu == 2 else 1.0, bool(glu), glu)
+            want[t] += (1.0 if glu == 2 else w) * (down[e].double() @ a)
+        if sff:
+            a = unit(s_up.double() @ x[t].double(), 1.0, s_gated, glu)
+            want[t] += (sg[t].double() if sg is not None else 1.0) * (s_down.double() @ a)
+    cols = top * ff + sff + (hidden if ident else 0)
+    act = torch.full((T, cols), float("nan"), dtype=torch.bfloat16, device=DEV)
+    out = torch.full((T, hidden), float("nan"), dtype=torch.bfloat16, device=DEV)
+    h = torch.randn(T, hidden, generator=g).to(DEV)
+    assert _lib().vm_experts_few_tile_fits(_i(T), _i(hidden), _i(ff), _i(sff), _i(top), _i(E), _i(ident)) == 1
+    for residual in (None, h.clone()):
+        rc = _lib().vm_experts_few_tile(_p(x), _p(up), _p(down), _p(s_up), _p(s_down), _p(chosen), _p(weight), _p(sg), _i(T), _i(hidden), _i(ff), _i(sff), _i(top), _i(2), _i(2),
+                                        _i(E), _i(ident), _i(glu), _f(limit), _f(alpha), _p(act), _p(out), _p(residual), _stream())
+        assert rc == 0
+        got = out.double() if residual is None else (residual - h).double()
+        # one rounding of the result (2^-9 of it), and now and then a unit that falls to the other side of a rounding
+        assert float((got - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-2 * float(want.std())

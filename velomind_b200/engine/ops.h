@@ -245,9 +245,10 @@ inline void mlstm_scan(const float* proj, int ld, const float* bias_i, const flo
 
 // (norm_w given: x is the float32 residual stream and the kernels norm its rows themselves; residual given: the result is added into it)
 inline void expert_router(const void* x, const float* norm_w, float eps, const float* w_router, const float* b_router, const float* w_gate, int T,
-                          int hidden, int E, int top, int* chosen, float* weight, float* shared_gate, DType act, cudaStream_t s) {
+                          int hidden, int E, int top, int* chosen, float* weight, float* shared_gate, void* rows_out, DType act, cudaStream_t s) {
     Timed t("expert_router", s);
-    check(vm_expert_router(x, norm_w, eps, w_router, b_router, w_gate, T, hidden, E, top, chosen, weight, shared_gate, code(act), s), "expert_router", s);
+    check(vm_expert_router_rows(x, norm_w, eps, w_router, b_router, w_gate, T, hidden, E, top, chosen, weight, shared_gate, rows_out, code(act), s),
+          "expert_router", s);
 }
 
 inline void experts_few_tokens(const void* x, const float* norm_w, float eps, const DeviceTensor& up, const DeviceTensor& down, const void* up_shared,
@@ -271,10 +272,10 @@ struct ExpertKind {
 
 inline void expert_router_scored(const void* x, const float* norm_w, float eps, const float* w_router, const float* correction, int T, int hidden,
                                  int n_out, int top, int group_count, int group_keep, int group_top, float scale, int score_kind, bool normalize, int* chosen,
-                                 float* weight, DType act, cudaStream_t s) {
+                                 float* weight, void* rows_out, DType act, cudaStream_t s) {
     Timed t("expert_router", s);
-    check(vm_expert_router_groups(x, norm_w, eps, w_router, correction, T, hidden, n_out, top, group_count, group_keep, group_top, scale, score_kind,
-                                  normalize ? 1 : 0, chosen, weight, code(act), s),
+    check(vm_expert_router_groups_rows(x, norm_w, eps, w_router, correction, T, hidden, n_out, top, group_count, group_keep, group_top, scale, score_kind,
+                                       normalize ? 1 : 0, chosen, weight, rows_out, code(act), s),
           "expert_router", s);
 }
 
@@ -286,6 +287,17 @@ inline void experts_few_tokens_glu(const void* x, const float* norm_w, float eps
     check(vm_experts_few_tokens_glu(x, norm_w, eps, up.ptr, down.ptr, up_shared, down_shared, code(up.dtype), chosen, weight, shared_gate, T, hidden, ff,
                                     ff_shared, top, k.act_kind, act_kind_shared, k.E, k.n_identity, k.glu, k.limit, k.alpha, act, out, residual,
                                     code(act_dtype), s),
+          "experts_few_tokens", s);
+    ++counters().own_launches;          // two kernels
+}
+
+// bfloat16 rows x (normed), every expert's weights once for all its tokens (vm_experts_few_tile_fits)
+inline void experts_few_tile(const void* x, const DeviceTensor& up, const DeviceTensor& down, const void* up_shared, const void* down_shared, const int* chosen,
+                             const float* weight, const float* shared_gate, int T, int hidden, int ff, int ff_shared, int top, int act_kind_shared,
+                             const ExpertKind& k, void* act, void* out, float* residual, cudaStream_t s) {
+    Timed t("experts_few_tokens", s);
+    check(vm_experts_few_tile(x, up.ptr, down.ptr, up_shared, down_shared, chosen, weight, shared_gate, T, hidden, ff, ff_shared, top, k.act_kind,
+                              act_kind_shared, k.E, k.n_identity, k.glu, k.limit, k.alpha, act, out, residual, s),
           "experts_few_tokens", s);
     ++counters().own_launches;          // two kernels
 }

@@ -114,11 +114,21 @@ int vm_mlstm_step(const float* proj, int ld, const float* bias_i, const float* b
                   const int* cu_tokens, const int* slots, void* out, float* scratch, int B, int H, int D, int V, float cap, float eps,
                   int act_dtype, cudaStream_t stream);
 
-// ---- routed_experts.cu: a routed feed-forward for few tokens
+// ---- expert_router.cu, routed_experts.cu, routed_experts_tile.cu: a routed feed-forward for few tokens (the routers serve any number)
 // x [T, hidden] in the activation dtype, or (norm_w given) the float32 residual stream, whose rows the kernels then norm themselves;
 // residual given: the experts' result is added into it instead of being written to `out`
 int vm_expert_router(const void* x, const float* norm_w, float eps, const float* w_router, const float* b_router, const float* w_gate, int T,
                      int hidden, int E, int top, int* chosen, float* weight, float* shared_gate, int act_dtype, cudaStream_t stream);
+// the same; rows_out (with norm_w; null: none) receives the normed rows [T, hidden] in the activation dtype
+int vm_expert_router_rows(const void* x, const float* norm_w, float eps, const float* w_router, const float* b_router, const float* w_gate, int T,
+                          int hidden, int E, int top, int* chosen, float* weight, float* shared_gate, void* rows_out, int act_dtype, cudaStream_t stream);
+// the experts in bfloat16 on tensor-core tiles, every expert's weights once for all its tokens: x are bfloat16 rows (normed), E the number of real
+// experts (chosen indices >= E name identity experts); the rest as vm_experts_few_tokens_glu
+int vm_experts_few_tile_fits(int T, int hidden, int ff, int ff_shared, int top, int E, int n_identity);
+int vm_experts_few_tile(const void* x, const void* w_up, const void* w_down, const void* w_up_shared, const void* w_down_shared, const int* chosen,
+                        const float* weight, const float* shared_gate, int T, int hidden, int ff, int ff_shared, int top, int act_kind,
+                        int act_kind_shared, int E, int n_identity, int glu, float limit, float alpha, void* act, void* out, float* residual,
+                        cudaStream_t stream);
 int vm_experts_few_tokens(const void* x, const float* norm_w, float eps, const void* w_up, const void* w_down, const void* w_up_shared,
                           const void* w_down_shared, int weight_dtype, const int* chosen, const float* weight, const float* shared_gate, int T,
                           int hidden, int ff, int ff_shared, int top, int act_kind, int act_kind_shared, void* act, void* out,
@@ -145,6 +155,9 @@ int vm_expert_router_scores(const void* x, const float* norm_w, float eps, const
 int vm_expert_router_groups(const void* x, const float* norm_w, float eps, const float* w_router, const float* correction, int T, int hidden,
                             int n_out, int top, int group_count, int group_keep, int group_top, float scale, int score_kind, int normalize, int* chosen,
                             float* weight, int act_dtype, cudaStream_t stream);
+int vm_expert_router_groups_rows(const void* x, const float* norm_w, float eps, const float* w_router, const float* correction, int T, int hidden,
+                                 int n_out, int top, int group_count, int group_keep, int group_top, float scale, int score_kind, int normalize, int* chosen,
+                                 float* weight, void* rows_out, int act_dtype, cudaStream_t stream);      // rows_out as in vm_expert_router_rows
 
 // ---- attention_biased.cu: windowed attention with kept first tokens and a learned bias by bucketed distance; keys of Dk, values of Dv
 // qkv [T, ld]: H query heads and Hkv key heads of Dk, Hkv value heads of Dv; queries and keys get a unit-rms norm per head (weights wq, wk

@@ -145,17 +145,17 @@ public:
     }
 
     // chosen experts and weights of every token (and the shared expert's gate), by the part's form of routing
-    void route(StepContext& ctx, const void* x, const float* nw, float eps, int* chosen, float* weight, float* sgate) {
+    void route(StepContext& ctx, const void* x, const float* nw, float eps, int* chosen, float* weight, float* sgate, void* rows_out = nullptr) {
         if (r_.scored) {
             if (gate_) throw Error("routed_experts: the scored router has no gate for a shared expert");
             ops::expert_router_scored(x, nw, eps, static_cast<const float*>(router_.ptr), r_.correction ? static_cast<const float*>(router_b_.ptr) : nullptr,
                                       ctx.T, hidden_, E_ + r_.identity, top_, r_.groups, r_.groups_keep, r_.groups_top, r_.scale, r_.score_kind, r_.normalize, chosen, weight,
-                                      ctx.act_dtype, ctx.stream);
+                                      rows_out, ctx.act_dtype, ctx.stream);
             return;
         }
         ops::expert_router(x, nw, eps, static_cast<const float*>(router_.ptr), static_cast<const float*>(router_b_.ptr),
-                           gate_ ? static_cast<const float*>(s_gate_.ptr) : nullptr, ctx.T, hidden_, E_, top_, chosen, weight, sgate, ctx.act_dtype,
-                           ctx.stream);
+                           gate_ ? static_cast<const float*>(s_gate_.ptr) : nullptr, ctx.T, hidden_, E_, top_, chosen, weight, sgate, rows_out,
+                           ctx.act_dtype, ctx.stream);
     }
 
     // the few-token path: x in the activation dtype, or (nw given) the float32 residual stream; `residual` given: added into
@@ -163,15 +163,22 @@ public:
         int* chosen = static_cast<int*>(ctx.take_tokens(top_, DType::I32));
         float* weight = static_cast<float*>(ctx.take_tokens(top_, DType::F32));
         float* sgate = gate_ ? static_cast<float*>(ctx.take_tokens(1, DType::F32)) : nullptr;
-        route(ctx, x, nw, eps, chosen, weight, sgate);
+        // in bfloat16 each expert's weights once for all its tokens, from rows that the router has normed; else token by token
+        const bool tile = ctx.act_dtype == DType::BF16 && up_.dtype == DType::BF16 && vm_experts_few_tile_fits(ctx.T_cap, hidden_, ff_, sff_, top_, E_, r_.identity);
+        void* normed = tile && nw ? ctx.take_tokens(hidden_, ctx.act_dtype) : nullptr;
+        route(ctx, x, nw, eps, chosen, weight, sgate, normed);
         void* act = ctx.take_tokens(vm_experts_act_cols(hidden_, ff_, sff_, top_, r_.identity), ctx.act_dtype);
-        if (general())
+        if (tile)
+            ops::experts_few_tile(normed ? normed : x, up_, down_, sff_ > 0 ? s_up_.ptr : nullptr, sff_ > 0 ? s_down_.ptr : nullptr, chosen, weight, sgate, ctx.T,
+                                  hidden_, ff_, sff_, top_, sact_, kind(), act, out, residual, ctx.stream);
+        else if (general())
             ops::experts_few_tokens_glu(x, nw, eps, up_, down_, sff_ > 0 ? s_up_.ptr : nullptr, sff_ > 0 ? s_down_.ptr : nullptr, chosen, weight, sgate,
                                         ctx.T, hidden_, ff_, sff_, top_, sact_, kind(), act, out, residual, ctx.act_dtype, ctx.stream);
         else
             ops::experts_few_tokens(x, nw, eps, up_, down_, sff_ > 0 ? s_up_.ptr : nullptr, sff_ > 0 ? s_down_.ptr : nullptr, chosen, weight, sgate, ctx.T,
                                     hidden_, ff_, sff_, top_, act_, sact_, act, out, residual, ctx.act_dtype, ctx.stream);
         ctx.give(act);
+        ctx.give(normed);
         ctx.give(sgate);
         ctx.give(weight);
         ctx.give(chosen);
