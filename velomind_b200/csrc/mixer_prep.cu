@@ -200,6 +200,183 @@ static int launch_heads(const float* proj, int ld, const float* bias, float eps,
     return vm_launch_status();
 }
 
+// The preparation with a convolution, rotary positions or a norm over the whole projection: a warp takes the heads `item`, item + gridDim.y * 8, .. of one token, so
+// that a token's rotation is worked out once per warp; two neighbouring values per lane and turn, a head's row passes through the warp's own shared memory
+// only to meet its rotary partners.  Few tokens: a warp per head, many blocks per token; with the norm one block
+// per token and a warp per head, whose sums of squares meet once.  (With a block per token and passes over the row in shared
+// memory, a decode step of 4 tokens of 24 heads and three taps took 13 us, 2,300 prompt tokens 27 us: a chain of passes, most of the GPU idle.
+// Now 5.6 and 18 us.)
+template <typename T, int NP, bool NORMED>
+__global__ void __launch_bounds__(NORMED ? 1024 : HEADS_THREADS)
+mixer_turned_heads_kernel(const float* __restrict__ proj, int ld, const float* __restrict__ bias, const float* __restrict__ taps, int K,
+                          float* __restrict__ state, long long state_stride, int state_offset, const float* __restrict__ q_norm,
+                          const float* __restrict__ k_norm, float eps, const float* __restrict__ inv_freq, int rotary_dim,
+                          int pairing, const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ cu_tokens,
+                          const int* __restrict__ slots, const int* __restrict__ block_table, int max_blocks, T* __restrict__ q_out, T* __restrict__ kpages,
+                          T* __restrict__ vpages, int n_pages, int H, int G, int Dk, int Dv, int values_are_keys, int unit_heads, int keep_here,
+                          int* __restrict__ err) {
+    __shared__ float rows[NORMED ? 32 : HEADS_THREADS / 32][64 * NP];
+    __shared__ float squares[32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x;
+    const int items = H + (values_are_keys ? G : 2 * G), C = (H + G) * Dk + (values_are_keys ? 0 : G * Dv);
+    vm_pdl_launch_dependents();
+    vm_pdl_wait();
+    const int pos = positions[t], seq = seq_of_token[t];
+    const int first = cu_tokens[seq];                     // the step's first token of this sequence, at place pos - (t - first)
+    float* kept = (K > 1 && state) ? state + (size_t)slots[seq] * state_stride + state_offset : nullptr;      // [K - 1, C]: the rows before the step
+    int page = -1;
+    const int blk = pos / VM_PAGE_TOKENS, in_page = pos % VM_PAGE_TOKENS;
+    if (kpages) {
+        page = blk < max_blocks ? block_table[(size_t)seq * max_blocks + blk] : -1;
+        if (page < 0 || page >= n_pages) {
+            if (threadIdx.x == 0 && blockIdx.y == 0 && err) atomicExch(err, VM_ERRWORD_CACHE_WRITE);
+            page = -1;
+        }
+    }
+    // this token's rotation of the lane's values: value d is turned with its partner by (cos, +-sin)
+    float cs[NP][2], sn[NP][2];
+    int partner[NP][2];
+    const int half = inv_freq ? rotary_dim / 2 : 0;
+#pragma unroll
+    for (int n = 0; n < NP; ++n)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int d = 2 * (lane + 32 * n) + e;
+            cs[n][e] = 1.f; sn[n][e] = 0.f; partner[n][e] = d;
+            if (d < 2 * half) {
+                const bool low = pairing == VM_PAIR_INTERLEAVED ? e == 0 : d < half;
+                const int i = pairing == VM_PAIR_INTERLEAVED ? d >> 1 : (low ? d : d - half);
+                partner[n][e] = pairing == VM_PAIR_INTERLEAVED ? d ^ 1 : (low ? d + half : d - half);
+                float s;
+                sincosf((float)pos * inv_freq[i], &s, &cs[n][e]);
+                sn[n][e] = low ? -s : s;                  // u cos - v sin; v cos + u sin
+            }
+        }
+    float* row = rows[warp];
+    const int warps = blockDim.x / 32;
+    for (int item = blockIdx.y * warps + warp; item < items; item += gridDim.y * warps) {
+        const bool is_v = item >= H + G;
+        const int D = is_v ? Dv : Dk, col = is_v ? (H + G) * Dk + (item - H - G) * Dv : item * Dk;
+        float x[NP][2];
+        float ss = 0.f;
+#pragma unroll
+        for (int n = 0; n < NP; ++n) {
+            const int d = 2 * (lane + 32 * n), c = col + d;
+            x[n][0] = x[n][1] = 0.f;
+            if (d < D) {
+                const float2 b = bias ? *reinterpret_cast<const float2*>(bias + c) : make_float2(0.f, 0.f);
+                const float2 own = *reinterpret_cast<const float2*>(proj + (size_t)t * ld + c);
+                if (K >= 1 && taps) {
+                    for (int j = 0; j < K; ++j) {
+                        const int back = K - 1 - j;       // tap j weighs the token `back` places before this one
+                        if (pos - back < 0) continue;     // nothing lies before a sequence's start
+                        float2 u = own;
+                        if (back > 0) {
+                            if (t - back >= first) u = *reinterpret_cast<const float2*>(proj + (size_t)(t - back) * ld + c);
+                            else {
+                                const float* k = kept + (size_t)((K - 1) - (back - (t - first))) * C + c;      // row K - 1 - d holds the token d places before the step
+                                u = make_float2(k[0], k[1]);
+                            }
+                        }
+                        x[n][0] = fmaf(taps[(size_t)c * K + j], u.x + b.x, x[n][0]);
+                        x[n][1] = fmaf(taps[(size_t)(c + 1) * K + j], u.y + b.y, x[n][1]);
+                    }
+                    if (keep_here && kept) {              // the kept rows move on by this token (one token per sequence: no other warp reads or writes them)
+                        for (int j = 1; j < K - 1; ++j) {
+                            kept[(size_t)(j - 1) * C + c] = kept[(size_t)j * C + c];
+                            kept[(size_t)(j - 1) * C + c + 1] = kept[(size_t)j * C + c + 1];
+                        }
+                        kept[(size_t)(K - 2) * C + c] = own.x;
+                        kept[(size_t)(K - 2) * C + c + 1] = own.y;
+                    }
+                } else {
+                    x[n][0] = own.x + b.x;
+                    x[n][1] = own.y + b.y;
+                }
+                ss += x[n][0] * x[n][0] + x[n][1] * x[n][1];
+            }
+        }
+        float norm = 1.0f;
+        if (NORMED && item == warp) {                     // the block's first turn holds all heads of q and k: the norm over each whole projection
+            ss = vm_warp_sum(ss);
+            if (lane == 0) squares[warp] = ss;
+            __syncthreads();
+            const bool is_q = item < H, in = lane < warps && (is_q ? lane < H : lane >= H && lane < H + G);
+            norm = 1.0f / sqrtf(vm_warp_sum(in ? squares[lane] : 0.f) / (float)((is_q ? H : G) * Dk) + eps);
+        }
+        if (is_v) {
+            if (page >= 0)
+#pragma unroll
+                for (int n = 0; n < NP; ++n) {
+                    const int d = 2 * (lane + 32 * n);
+                    if (d < Dv) store2(vpages + (((size_t)page * G + item - H - G) * VM_PAGE_TOKENS + in_page) * Dv + d, x[n][0], x[n][1]);
+                }
+            continue;
+        }
+        if (values_are_keys && item >= H && page >= 0 && vpages)      // the keys as they left the convolution
+#pragma unroll
+            for (int n = 0; n < NP; ++n) {
+                const int d = 2 * (lane + 32 * n);
+                if (d < Dv) store2(vpages + (((size_t)page * G + item - H) * VM_PAGE_TOKENS + in_page) * Dv + d, x[n][0], x[n][1]);
+            }
+        const float f = !NORMED && unit_heads ? 1.0f / sqrtf(vm_warp_sum(ss) / (float)Dk + eps) : 1.0f;
+#pragma unroll
+        for (int n = 0; n < NP; ++n) {
+            if (NORMED) {
+                const int d = 2 * (lane + 32 * n);
+                const float* w = item < H ? q_norm + col + d : k_norm + (col - H * Dk) + d;
+                if (d < Dk) { x[n][0] = x[n][0] * norm * w[0]; x[n][1] = x[n][1] * norm * w[1]; }
+            } else {
+                x[n][0] *= f; x[n][1] *= f;
+            }
+            if (half) *reinterpret_cast<float2*>(row + 2 * (lane + 32 * n)) = make_float2(x[n][0], x[n][1]);
+        }
+        if (half) {
+            __syncwarp();
+#pragma unroll
+            for (int n = 0; n < NP; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    if (2 * (lane + 32 * n) + e < 2 * half) x[n][e] = x[n][e] * cs[n][e] + row[partner[n][e]] * sn[n][e];
+            __syncwarp();                                 // the next head's row takes this one's place
+        }
+        T* dst = item < H ? q_out + (size_t)t * H * Dk + (size_t)item * Dk : kpages + (((size_t)page * G + item - H) * VM_PAGE_TOKENS + in_page) * Dk;
+        if (item >= H && page < 0) continue;
+#pragma unroll
+        for (int n = 0; n < NP; ++n) {
+            const int d = 2 * (lane + 32 * n);
+            if (d < Dk) store2(dst + d, x[n][0], x[n][1]);
+        }
+    }
+}
+
+template <typename T>
+static int launch_turned_heads(const float* proj, int ld, const float* bias, const float* taps, int K, float* state, long long state_stride, int state_offset,
+                               const float* q_norm, const float* k_norm, float eps, const float* inv_freq, int rotary_dim, int pairing, const int* positions, const int* seq_of_token,
+                               const int* cu_tokens, const int* slots, const int* block_table, int max_blocks, T* q_out, T* kpages, T* vpages, int n_pages,
+                               int n_tokens, int H, int G, int Dk, int Dv, int values_are_keys, int unit_heads, int keep_here, int* err, cudaStream_t stream) {
+    // blocks per token: enough for a warp per head while the GPU has room for them (eight blocks an SM), one from there on
+    const int all = (H + 2 * G + HEADS_THREADS / 32 - 1) / (HEADS_THREADS / 32);
+    const long long room = 8ll * vm_sm_count() / n_tokens;
+    const dim3 grid(n_tokens, (unsigned)(room < 1 ? 1 : room < all ? room : all));
+    const int widest = Dk > Dv ? Dk : Dv;
+    const int heads = H + (values_are_keys ? G : 2 * G);
+#define VM_TURNED(NP_)                                                                                                                                  \
+    if (q_norm)                                            /* one block a token, a warp per head (the caller has seen to it that H + G <= 32) */        \
+        vm_launch_pdl(mixer_turned_heads_kernel<T, NP_, true>, dim3(n_tokens), dim3(32 * (heads < 32 ? heads : 32)), 0, stream, proj, ld, bias, taps, K,    \
+                      state, state_stride, state_offset, q_norm, k_norm, eps, inv_freq, rotary_dim, pairing, positions, seq_of_token, cu_tokens, slots,     \
+                      block_table, max_blocks, q_out, kpages, vpages, n_pages, H, G, Dk, Dv, values_are_keys, unit_heads, keep_here, err);                  \
+    else                                                                                                                                                    \
+        vm_launch_pdl(mixer_turned_heads_kernel<T, NP_, false>, grid, dim3(HEADS_THREADS), 0, stream, proj, ld, bias, taps, K, state, state_stride,         \
+                      state_offset, q_norm, k_norm, eps, inv_freq, rotary_dim, pairing, positions, seq_of_token, cu_tokens, slots, block_table, max_blocks, \
+                      q_out, kpages, vpages, n_pages, H, G, Dk, Dv, values_are_keys, unit_heads, keep_here, err)
+    if (widest <= 64) { VM_TURNED(1); }
+    else if (widest <= 128) { VM_TURNED(2); }
+    else { VM_TURNED(4); }
+#undef VM_TURNED
+    return vm_launch_status();
+}
+
 // the kept rows of every sequence move on by the step's tokens: row K - 1 - d holds the projected row d places before the next step
 __global__ void mixer_keep_rows_kernel(const float* __restrict__ proj, int ld, int C, int K, float* __restrict__ state, long long state_stride,
                                        int state_offset, const int* __restrict__ cu_tokens, const int* __restrict__ slots) {
@@ -250,7 +427,20 @@ VM_API int vm_mixer_prepare(const float* proj, int ld, const float* bias, const 
     const int threads = C >= 2048 ? 512 : 256;
     const int keep_here = (one_token_each && K > 1) ? 1 : 0;
     cudaError_t e = cudaSuccess;
-    if (act_dtype == VM_F32) {
+    // heads that depend on nothing but themselves, or one norm a block can hold (and the pages are the row's own, or there are none): warps take them apart
+    const bool apart = (!q_norm || H + G <= 32) && (G == 0 || (kpages && vpages)) && Dk % 2 == 0 && Dv % 2 == 0 && ld % 2 == 0 && Dk <= 256 && Dv <= 256 &&
+                       ((uintptr_t)proj | (uintptr_t)bias) % 8 == 0 && ((uintptr_t)q_out | (uintptr_t)kpages | (uintptr_t)vpages) % 8 == 0;
+    if (apart && act_dtype == VM_F32) {
+        const int st = launch_turned_heads<float>(proj, ld, bias, taps, K, state, state_stride, state_offset, q_norm, k_norm, eps, inv_freq, rotary_dim, pairing,
+                                                  positions, seq_of_token, cu_tokens, slots, block_table, max_blocks, (float*)q_out, (float*)kpages, (float*)vpages,
+                                                  n_pages, T, H, G, Dk, Dv, values_are_keys, unit_heads, keep_here, err, stream);
+        if (st) return st;
+    } else if (apart && act_dtype == VM_BF16) {
+        const int st = launch_turned_heads<__nv_bfloat16>(proj, ld, bias, taps, K, state, state_stride, state_offset, q_norm, k_norm, eps, inv_freq, rotary_dim,
+                                                          pairing, positions, seq_of_token, cu_tokens, slots, block_table, max_blocks, (__nv_bfloat16*)q_out, (__nv_bfloat16*)kpages,
+                                                          (__nv_bfloat16*)vpages, n_pages, T, H, G, Dk, Dv, values_are_keys, unit_heads, keep_here, err, stream);
+        if (st) return st;
+    } else if (act_dtype == VM_F32) {
         if (smem > 48 * 1024) e = cudaFuncSetAttribute(mixer_prepare_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         vm_launch_pdl(mixer_prepare_kernel<float>, dim3(T), dim3(threads), smem, stream, proj, ld, bias, taps, K, state, state_stride, state_offset, q_norm,
