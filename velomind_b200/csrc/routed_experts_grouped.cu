@@ -222,6 +222,54 @@ __global__ void experts_combine_kernel(const float* __restrict__ y, const int* _
     }
 }
 
+// the same with four neighbouring columns a thread and up to four experts' rows in flight together (one value a thread and one row after the other:
+// 22.5 us for 2,556 tokens of width 1,024 and 4 experts, 43 MB, and 22.9 us for 4,096 tokens; now 11.6 and 15.3 us)
+__global__ void __launch_bounds__(256)
+experts_combine_vec_kernel(const float* __restrict__ y, const int* __restrict__ row_of_pair, const float* __restrict__ weight,
+                           const float* __restrict__ shared_y, const float* __restrict__ shared_gate, int T, int hidden, int top,
+                           const __nv_bfloat16* __restrict__ x, const int* __restrict__ chosen, int E, __nv_bfloat16* __restrict__ out) {
+    const int per = hidden / 4;
+    const long long n = (long long)T * per;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const int t = (int)(i / per), c = (int)(i - (long long)t * per) * 4;
+        const int* rows = row_of_pair + (size_t)t * top;
+        const size_t at = (size_t)t * hidden + c;
+        float4 sy = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (shared_y) sy = *reinterpret_cast<const float4*>(shared_y + at);
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k0 = 0; k0 < top; k0 += 4) {
+            float4 v[4];
+            float w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                w[k] = 0.f;
+                v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (k0 + k >= top) continue;
+                const int row = rows[k0 + k];
+                if (row >= 0) {
+                    w[k] = weight ? weight[(size_t)t * top + k0 + k] : 1.0f;
+                    v[k] = *reinterpret_cast<const float4*>(y + (size_t)row * hidden + c);
+                } else if (x && chosen[(size_t)t * top + k0 + k] >= E) {
+                    w[k] = weight[(size_t)t * top + k0 + k];
+                    const uint2 u = *reinterpret_cast<const uint2*>(x + at);
+                    const float2 p = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+                    v[k] = make_float4(p.x, p.y, q.x, q.y);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                acc.x = fmaf(w[k], v[k].x, acc.x); acc.y = fmaf(w[k], v[k].y, acc.y);
+                acc.z = fmaf(w[k], v[k].z, acc.z); acc.w = fmaf(w[k], v[k].w, acc.w);
+            }
+        }
+        if (shared_y) {
+            const float f = shared_gate ? shared_gate[t] : 1.0f;
+            acc.x = fmaf(f, sy.x, acc.x); acc.y = fmaf(f, sy.y, acc.y); acc.z = fmaf(f, sy.z, acc.z); acc.w = fmaf(f, sy.w, acc.w);
+        }
+        *reinterpret_cast<uint2*>(out + at) = make_uint2(vm_pack_bf16(acc.x, acc.y), vm_pack_bf16(acc.z, acc.w));
+    }
+}
+
 // x_sorted[row] = x[token_of_row[row]], zeros for a row of padding; 16 bytes per thread
 __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ token_of_row, int rows, int hidden,
                                    __nv_bfloat16* __restrict__ x_sorted) {
@@ -342,11 +390,17 @@ VM_API int vm_experts_grouped_glu(const void* x, const void* w_up, const void* w
         if (st) return st;
     }
     const size_t n = (size_t)T * hidden;
-    const size_t want = (n + 255) / 256;
     // (a weight that went into the expert's input is not applied again)
-    experts_combine_kernel<<<(int)(want < 148 * 16 ? want : 148 * 16), 256, 0, stream>>>(y, row_of_pair, glu == VM_GLU_SILU_WEIGHTED_INPUT ? nullptr : weight,
-                                                                                         shared_y, shared_gate, T, hidden, top,
-                                                                                         n_identity > 0 ? (const __nv_bfloat16*)x : nullptr, chosen, E,
+    const float* w = glu == VM_GLU_SILU_WEIGHTED_INPUT ? nullptr : weight;
+    const __nv_bfloat16* own = n_identity > 0 ? (const __nv_bfloat16*)x : nullptr;
+    const uintptr_t rows_at = (uintptr_t)y | (uintptr_t)shared_y | (uintptr_t)own | (uintptr_t)out;
+    if (hidden % 4 == 0 && rows_at % 16 == 0) {
+        experts_combine_vec_kernel<<<(unsigned)((n / 4 + 255) / 256), 256, 0, stream>>>(y, row_of_pair, w, shared_y, shared_gate, T, hidden, top, own, chosen, E,
+                                                                                        (__nv_bfloat16*)out);
+        return vm_launch_status();
+    }
+    const size_t want = (n + 255) / 256;
+    experts_combine_kernel<<<(int)(want < 148 * 16 ? want : 148 * 16), 256, 0, stream>>>(y, row_of_pair, w, shared_y, shared_gate, T, hidden, top, own, chosen, E,
                                                                                          (__nv_bfloat16*)out);
     return vm_launch_status();
 }
