@@ -1,5 +1,5 @@
-"""The kernels of a decode step's few rows against the same in 64 bits: the routers (csrc/expert_router.cu) and the experts on tensor-core tiles
-(csrc/routed_experts_tile.cu)."""
+"""The kernels of a decode step's few rows against the same in 64 bits: float32 products (csrc/skinny_f32.cu), the routers (csrc/expert_router.cu)
+and the experts on tensor-core tiles (csrc/routed_experts_tile.cu)."""
 import ctypes
 
 import numpy as np
@@ -29,6 +29,43 @@ def _f(v):
 
 def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("N,K", [(1, 4), (5, 36), (7, 576), (960, 576), (33, 1028), (64, 4096)])
+def test_skinny_f32(T, N, K):
+    """A row of a product does not depend on the others; error: K terms of 2^-24 of values of rms 1."""
+    g = torch.Generator().manual_seed(T * K)
+    x, w = torch.randn(T, K + 8, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    out = torch.full((T, N), float("nan"), device=DEV)
+    assert _lib().vm_skinny_f32(_p(x), ctypes.c_longlong(K + 8), _p(w), _p(out), _i(T), _i(N), _i(K), _stream()) == 0
+    want = x[:, :K].double() @ w.double().T
+    assert float((out.double() - want).abs().max()) <= 1e-6 * K ** 0.5 * 4
+    one = torch.empty(1, N, device=DEV)
+    assert _lib().vm_skinny_f32(_p(x[T - 1:]), ctypes.c_longlong(K + 8), _p(w), _p(one), _i(1), _i(N), _i(K), _stream()) == 0
+    assert float((one - out[T - 1:]).abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 8])
+@pytest.mark.parametrize("N,K", [(6, 36), (1152, 576), (130, 1028)])
+def test_skinny_f32_with_its_neighbours(T, N, K):
+    """The norm in front, the sum into a residual stream and the gated unit behind."""
+    g = torch.Generator().manual_seed(T + K)
+    x, w, nw, h = (torch.randn(*s, generator=g).to(DEV) for s in ((T, K), (N, K), (K,), (T, N)))
+    xn = x.double() / torch.sqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-5) * nw.double()
+    for norm in (True, False):
+        y = (xn if norm else x.double()) @ w.double().T
+        args = (_p(x), ctypes.c_longlong(K), _p(nw if norm else None), _f(1e-5), _p(w))
+        tol = 1e-6 * K ** 0.5 * 8
+        for add in (0, 1):
+            out = h.clone()
+            assert _lib().vm_skinny_f32_fused(*args, _p(out), _i(T), _i(N), _i(K), _i(add), _i(0), _stream()) == 0
+            assert float((out.double() - (y + h.double() if add else y)).abs().max()) <= tol
+        out = torch.full((T, N // 2), float("nan"), device=DEV)
+        assert _lib().vm_skinny_f32_fused(*args, _p(out), _i(T), _i(N), _i(K), _i(0), _i(1), _stream()) == 0
+        gate, up = y.chunk(2, -1)
+        want = torch.nn.functional.silu(gate) * up
+        assert float((out.double() - want).abs().max()) <= tol * float(y.abs().max())
 
 
 def _choice(z, kind, top, groups, keep, gtop, correction, normalize, scale):

@@ -291,6 +291,17 @@ inline void experts_few_tokens_glu(const void* x, const float* norm_w, float eps
     ++counters().own_launches;          // two kernels
 }
 
+// a few float32 rows (a step of at most FEW_F32_ROWS rows of capacity) through one product with the neighbouring work in it: x rows of `K` values, normed
+// if norm_w is given; add: into `out`; swiglu: W = [gate; up], out [T, rows / 2]
+constexpr int FEW_F32_ROWS = 8;
+inline void few_f32(const void* x, const float* norm_w, float eps, const DeviceTensor& W, void* out, int T, bool add, bool swiglu, cudaStream_t s) {
+    if (T <= 0) return;
+    Timed t("linear", s);
+    check(vm_skinny_f32_fused(static_cast<const float*>(x), W.cols(), norm_w, eps, static_cast<const float*>(W.ptr), static_cast<float*>(out), T,
+                              static_cast<int>(W.rows()), static_cast<int>(W.cols()), add ? 1 : 0, swiglu ? 1 : 0, s),
+          "linear", s);
+}
+
 // bfloat16 rows x (normed), every expert's weights once for all its tokens (vm_experts_few_tile_fits)
 inline void experts_few_tile(const void* x, const DeviceTensor& up, const DeviceTensor& down, const void* up_shared, const void* down_shared, const int* chosen,
                              const float* weight, const float* shared_gate, int T, int hidden, int ff, int ff_shared, int top, int act_kind_shared,

@@ -245,6 +245,12 @@ int vm_rope_kv_write(void* qkv, const int* positions, const int* seq_of_token, c
                      int n_pages, int act_dtype, int* err, cudaStream_t stream);
 
 // ---- attention
+// ---- skinny_f32.cu: out[T, N] = x[T, K] W[N, K]^T in float32 for up to eight rows
+int vm_skinny_f32_fits(const void* x, long long ldx, const void* w, int T, int K);
+int vm_skinny_f32(const float* x, long long ldx, const float* w, float* out, int T, int N, int K, cudaStream_t stream);
+// norm_w [K] given: the rows of x are normed; add: out += ...; swiglu: w = [gate; up] stacked, out [T, N / 2] = silu(gate) up
+int vm_skinny_f32_fused(const float* x, long long ldx, const float* norm_w, float eps, const float* w, float* out, int T, int N, int K, int add, int swiglu,
+                        cudaStream_t stream);
 // ---- attention_rows.cu: the float32 arithmetic of the plain kernels with a query's keys spread over a CTA (arguments as vm_attention_sink_generic;
 // v_stride is given); vm_attention_generic and vm_attention_sink_generic call it where it takes the sizes
 int vm_attention_rows_fits(const void* kpages, const void* vpages, int H, int Hkv, int Dk, int Dv, int v_stride);

@@ -61,7 +61,9 @@ public:
     bool can_fuse(const StepContext& ctx, const Norm& norm) const override {
         const float* nw;
         float eps;
-        if (!norm.as_rms(&nw, &eps) || ctx.act_dtype != DType::BF16) return false;
+        if (!norm.as_rms(&nw, &eps)) return false;
+        if (few_f32(ctx)) return true;
+        if (ctx.act_dtype != DType::BF16) return false;
         if (qkv_.weight.dtype != DType::BF16 || out_.weight.dtype != DType::BF16) return false;
         if (hidden_ % 8 || (H_ * D_) % 8) return false;
         const bool fused_rotary = rotary_.rotary_dim == 0 || (rotary_.rotary_dim == D_ && rotary_.pairing == VM_PAIR_HALF_SPLIT);
@@ -70,12 +72,30 @@ public:
         return true;
     }
 
+    // a few rows in float32: norm + q k v, rotary + cache write, attention, out added into h
+    bool few_f32(const StepContext& ctx) const {
+        return ctx.act_dtype == DType::F32 && ctx.T_cap <= ops::FEW_F32_ROWS && qkv_.weight.dtype == DType::F32 && out_.weight.dtype == DType::F32 &&
+               hidden_ % 4 == 0 && (H_ * D_) % 4 == 0;
+    }
+
     // h += attention(norm(h)): three or four launches, five on the library path.
     void forward_fused(StepContext& ctx, float* h, Norm& norm) override {
         const float* nw = nullptr;
         float eps = 0.f;
         norm.as_rms(&nw, &eps);
         const KVView kv = ctx.kv();
+        if (few_f32(ctx)) {
+            const long long width = static_cast<long long>(H_ + 2 * Hkv_) * D_;
+            void* qkv = ctx.take_tokens(width, DType::F32);
+            ops::few_f32(h, nw, eps, qkv_.weight, qkv, ctx.T, false, false, ctx.stream);
+            ops::rope_kv_write(qkv, ctx, kv, rotary_, H_, Hkv_, D_, DType::F32);
+            void* att = ctx.take_tokens(static_cast<long long>(H_) * D_, DType::F32);
+            ops::attention(ctx, qkv, static_cast<int>(width), kv, att, H_, Hkv_, D_, scale_, window_);
+            ctx.give(qkv);
+            ops::few_f32(att, nullptr, 0.f, out_.weight, h, ctx.T, true, false, ctx.stream);
+            ctx.give(att);
+            return;
+        }
         const bool skinny = ctx.T_cap <= max_rows();
         const bool fused_rotary = rotary_.rotary_dim == 0 || (rotary_.rotary_dim == D_ && rotary_.pairing == VM_PAIR_HALF_SPLIT);
         const bool tc = !skinny && fused_rotary && ops::tc_fused_rows(ctx) && (D_ == 64 || D_ == 128);

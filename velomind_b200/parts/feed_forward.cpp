@@ -43,10 +43,18 @@ public:
     bool can_fuse(const StepContext& ctx, const Norm& norm) const override {
         const float* nw;
         float eps;
-        if (!norm.as_rms(&nw, &eps) || ctx.act_dtype != DType::BF16) return false;
+        if (!norm.as_rms(&nw, &eps)) return false;
+        if (few_f32(ctx)) return true;
+        if (ctx.act_dtype != DType::BF16) return false;
         if (gate_up_.weight.dtype != DType::BF16 || down_.weight.dtype != DType::BF16) return false;
         if (ctx.T_cap <= max_rows()) return hidden_ % 32 == 0 && I_ % 32 == 0;
         return hidden_ % 8 == 0 && I_ % 8 == 0;
+    }
+
+    // a few rows in float32: norm + gate and up + SwiGLU, down added into h
+    bool few_f32(const StepContext& ctx) const {
+        return ctx.act_dtype == DType::F32 && ctx.T_cap <= ops::FEW_F32_ROWS && gate_up_.weight.dtype == DType::F32 && down_.weight.dtype == DType::F32 &&
+               act_ == VM_ACT_SILU && !clamped() && hidden_ % 4 == 0 && I_ % 4 == 0;
     }
 
     // h += down(silu(gate(norm(h))) * up(norm(h))): two or three launches.
@@ -54,6 +62,13 @@ public:
         const float* nw = nullptr;
         float eps = 0.f;
         norm.as_rms(&nw, &eps);
+        if (few_f32(ctx)) {
+            void* act = ctx.take_tokens(I_, DType::F32);
+            ops::few_f32(h, nw, eps, gate_up_.weight, act, ctx.T, false, true, ctx.stream);
+            ops::few_f32(act, nullptr, 0.f, down_.weight, h, ctx.T, true, false, ctx.stream);
+            ctx.give(act);
+            return;
+        }
         const bool skinny = ctx.T_cap <= max_rows();
         const bool tc = !skinny && act_ == VM_ACT_SILU && !clamped() && ops::tc_fused_rows(ctx) && I_ % 64 == 0;      // (that epilogue knows SiLU)
         if (!skinny && !tc) {
