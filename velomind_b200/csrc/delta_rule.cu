@@ -878,7 +878,11 @@ VM_API int vm_delta_chunks(const float* rows, const float* gates, float* state, 
     if (T <= 0 || B <= 0 || n_chunks <= 0) return 0;
     if (!sizes_ok(H, G, Dk, Dv, 1) || !state || !scratch) return VM_ERR_BAD_ARG;
     if (!vm_delta_chunk_tokens(Dk, Dv) || H > 65535) return VM_ERR_UNSUPPORTED;
-    const int stages = carry_smem(Dk, 2) <= SMEM_MAX ? 2 : 1;
+    // Two stages hide a chunk's loads behind the one before; but where that gives more blocks than SMs, at one block an SM, blocks of one stage that
+    // share an SM do (measured, two prompts of 1,400 and 2,000 tokens, 16 heads of 128 x 128, 256 blocks: 256 us in two waves, 202 us side by side).
+    const long long blocks = (long long)B * H * ((Dv + CCOLS - 1) / CCOLS);
+    const bool beside = blocks > vm_sm_count() && 2 * (carry_smem(Dk, 1) + 2048) <= SMEM_MAX;
+    const int stages = carry_smem(Dk, 2) <= SMEM_MAX && !beside ? 2 : 1;
     cudaError_t e = allow_smem(delta_local_kernel, local_smem(Dk));
     if (e == cudaSuccess) e = allow_smem(delta_finish_kernel, finish_smem(Dk));
     if (e == cudaSuccess) e = stages == 2 ? allow_smem(delta_carry_kernel<2>, carry_smem(Dk, 2)) : allow_smem(delta_carry_kernel<1>, carry_smem(Dk, 1));
