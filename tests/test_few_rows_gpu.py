@@ -163,3 +163,22 @@ def test_experts_tile(T, hidden, ff, sff, top, E, ident, glu):
         got = out.double() if residual is None else (residual - h).double()
         # one rounding of the result (2^-9 of it), and now and then a unit that falls to the other side of a rounding
         assert float((got - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-2 * float(want.std())
+
+
+@pytest.mark.parametrize("sizes", [[(1, 0)], [(3, 1), (40000, 0), (5, 3)], [(7, 0)] * 33])
+def test_clear_areas(sizes):
+    """State areas of any size and start become zeros, and nothing beside them does."""
+    pool = torch.ones(sum(n + off + 8 for n, off in sizes), device=DEV)
+    at, left = [], torch.ones_like(pool)
+    start = 0
+    for n, off in sizes:
+        at.append((start + off, n))
+        left[start + off:start + off + n] = 0
+        start += n + off + 8
+    for k in range(0, len(at), 32):
+        part = at[k:k + 32]
+        where = (ctypes.c_void_p * len(part))(*[pool.data_ptr() + 4 * a for a, _ in part])
+        n = (ctypes.c_longlong * len(part))(*[n for _, n in part])
+        assert _lib().vm_clear_areas(where, n, _i(len(part)), _stream()) == 0
+    assert torch.equal(pool, left)
+    assert _lib().vm_clear_areas(None, None, _i(33), _stream()) != 0

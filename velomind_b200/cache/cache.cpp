@@ -247,14 +247,26 @@ SequenceCache::SequenceCache(const std::vector<CacheNeed>& needs, const std::vec
 
 int SequenceCache::open() {
     const int slot = book.open();
+    // the state areas of all runs, as many as one launch takes at a time
+    float* at[VM_CLEAR_AREAS];
+    long long n[VM_CLEAR_AREAS];
+    int count = 0;
+    auto clear = [&] {
+        const bool ok = vm_clear_areas(at, n, count, stream_) == 0;
+        count = 0;
+        if (!ok) {
+            book.close(slot);
+            throw KernelError("could not clear a sequence's state area");
+        }
+    };
     for (size_t i = 0; i < state.size(); ++i)
         if (state[i] && book.state_owner[i] == static_cast<int>(i)) {
-            const size_t row = static_cast<size_t>(book.state_floats[i]) * sizeof(float);
-            if (cudaMemsetAsync(static_cast<char*>(state[i]->ptr) + row * slot, 0, row, stream_) != cudaSuccess) {
-                book.close(slot);
-                throw KernelError("could not clear a sequence's state area");
-            }
+            n[count] = book.state_floats[i];
+            at[count] = static_cast<float*>(state[i]->ptr) + n[count] * slot;
+            ++count;
+            if (count == VM_CLEAR_AREAS) clear();
         }
+    if (count) clear();
     return slot;
 }
 

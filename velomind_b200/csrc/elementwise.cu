@@ -378,3 +378,38 @@ VM_API int vm_soft_cap(float* x, long long n, float cap, cudaStream_t stream) {
     vm_launch_pdl(soft_cap_kernel, dim3(grid), dim3(256), 0, stream, x, n, cap, (uintptr_t)x % 16 == 0 ? 1 : 0);
     return vm_launch_status();
 }
+
+// ------------------------------------------------------------------------------------------------ clearing a sequence's state areas
+// One launch for all areas of a slot (a memory set per area costs the stream 2 us each, 40 of them in front of a batch of eight prompts of a model
+// with five; all areas of a sequence in one launch 2 us).  blockIdx.y names the area; whole 16-byte pieces where the area's start and size allow it.
+namespace {
+struct ClearList {
+    float* at[VM_CLEAR_AREAS];
+    long long n[VM_CLEAR_AREAS];
+};
+__global__ void __launch_bounds__(256) clear_areas_kernel(ClearList list) {
+    float* at = list.at[blockIdx.y];
+    const long long n = list.n[blockIdx.y], step = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool vec = (reinterpret_cast<uintptr_t>(at) & 15) == 0;
+    const long long quads = vec ? n / 4 : 0;
+    for (long long i = first; i < quads; i += step) reinterpret_cast<float4*>(at)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (long long i = 4 * quads + first; i < n; i += step) at[i] = 0.f;
+}
+}  // namespace
+
+// zeros into `count` (at most VM_CLEAR_AREAS) areas of n[i] floats
+VM_API int vm_clear_areas(float* const* at, const long long* n, int count, cudaStream_t stream) {
+    if (count <= 0) return 0;
+    if (count > VM_CLEAR_AREAS) return VM_ERR_BAD_ARG;
+    ClearList list = {};
+    long long most = 0;
+    for (int i = 0; i < count; ++i) {
+        list.at[i] = at[i];
+        list.n[i] = n[i];
+        most = n[i] > most ? n[i] : most;
+    }
+    if (most <= 0) return 0;
+    const long long want = (most + 4095) / 4096;           // a block clears four runs of 256 quads
+    clear_areas_kernel<<<dim3((unsigned)(want < 256 ? want : 256), count), 256, 0, stream>>>(list);
+    return vm_launch_status();
+}

@@ -47,6 +47,9 @@ int vm_add_rmsnorm(float* h, const void* delta, const float* w, void* out, const
 int vm_residual_add(float* h, const void* delta, long long n, int act_dtype, cudaStream_t stream);
 int vm_swiglu(const void* gate_up, void* out, int T, int I, int act_dtype, cudaStream_t stream);
 int vm_convert(const void* in, int in_dtype, void* out, int out_dtype, long long n, cudaStream_t stream);
+// zeros into up to VM_CLEAR_AREAS areas of n[i] floats, one launch
+enum { VM_CLEAR_AREAS = 32 };
+int vm_clear_areas(float* const* at, const long long* n, int count, cudaStream_t stream);
 // out[t, i] = act(gate_up[t, i]) * gate_up[t, I + i] for the activation `kind` (VM_ACT_*)
 int vm_gated_activation(const void* gate_up, void* out, int T, int I, int kind, int act_dtype, cudaStream_t stream);
 // the clamped gated unit: g = min(gate, limit), u = clamp(up, -limit, limit), out = g sigmoid(alpha g) (u + 1)
