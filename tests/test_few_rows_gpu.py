@@ -165,6 +165,35 @@ def test_experts_tile(T, hidden, ff, sff, top, E, ident, glu):
         assert float((got - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-2 * float(want.std())
 
 
+@pytest.mark.parametrize("T,top", [(895, 8), (896, 8), (1024, 8), (2048, 4), (512, 16)])
+def test_experts_tile_of_large_decode_batches(T, top):
+    """As many (token, expert) pairs as the list of a block holds, around the sizes from which it needs more shared memory than a launch gets
+    unasked; one more token is refused."""
+    g = torch.Generator().manual_seed(T)
+    hidden, ff, E = 64, 32, 18
+    bf = lambda *s, scale=1.0: (torch.randn(*s, generator=g) * scale).to(torch.bfloat16).to(DEV)
+    x, up, down = bf(T, hidden), bf(E, ff, hidden, scale=hidden ** -0.5), bf(E, hidden, ff, scale=ff ** -0.5)
+    chosen = torch.rand(T, E, generator=g).topk(top, -1).indices.int().to(DEV)
+    weight = torch.rand(T, top, generator=g).to(DEV)
+    z = torch.einsum("efh,th->tef", up.double(), x.double())
+    a = (torch.relu(z) ** 2).to(torch.bfloat16).double()
+    y = torch.einsum("ehf,tef->teh", down.double(), a)
+    want = (y.gather(1, chosen.long()[..., None].expand(-1, -1, hidden)) * weight.double()[..., None]).sum(1)
+    act = torch.full((T, top * ff), float("nan"), dtype=torch.bfloat16, device=DEV)
+    out = torch.full((T, hidden), float("nan"), dtype=torch.bfloat16, device=DEV)
+
+    def run(T):
+        sizes = _i(T), _i(hidden), _i(ff), _i(0), _i(top)
+        fits = _lib().vm_experts_few_tile_fits(*sizes, _i(E), _i(0))
+        return fits, _lib().vm_experts_few_tile(_p(x), _p(up), _p(down), None, None, _p(chosen), _p(weight), None, *sizes, _i(2), _i(2), _i(E), _i(0), _i(0), _f(0),
+                                                _f(0), _p(act), _p(out), None, _stream())
+    assert run(T) == (1, 0)
+    # one rounding of the result (2^-9 of it), and now and then a unit that falls to the other side of a rounding
+    assert float((out.double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-2 * float(want.std())
+    fits, rc = run(8192 // top + 1)                                # (refused before anything is launched)
+    assert fits == 0 and rc != 0
+
+
 @pytest.mark.parametrize("sizes", [[(1, 0)], [(3, 1), (40000, 0), (5, 3)], [(7, 0)] * 33])
 def test_clear_areas(sizes):
     """State areas of any size and start become zeros, and nothing beside them does."""

@@ -24,7 +24,7 @@ constexpr int UP_ROWS = 16;
 constexpr int DOWN_WARPS = 16;
 constexpr int DOWN_KB = 8;               // blocks of 32 of a piece
 constexpr int DOWN_TOKENS = 32;          // tokens of a block
-constexpr int MAX_PAIRS = 8192;          // (token, expert) pairs whose list an up block keeps in shared memory
+constexpr int MAX_PAIRS = 8192;          // (token, expert) pairs whose list an up block keeps in shared memory (32 KB behind 20 KB of sums: asked for below)
 
 __device__ __forceinline__ float tile_act(float z, int kind) {
     if (kind == VM_ACT_RELU_SQUARED) { const float r = fmaxf(z, 0.f); return r * r; }
@@ -322,9 +322,10 @@ VM_API int vm_experts_few_tile(const void* x, const void* w_up, const void* w_do
                         (int)vm_experts_act_cols(hidden, ff, ff_shared, top, n_identity), limit, alpha};
     const int nt = down_tiles(hidden);
     const size_t smem = down_smem(ff, ff_shared, top, E, nt);
+    static const cudaError_t r0 = cudaFuncSetAttribute(experts_up_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_PAIRS * (int)sizeof(int));
     static const cudaError_t r1 = cudaFuncSetAttribute(experts_down_tile_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     static const cudaError_t r2 = cudaFuncSetAttribute(experts_down_tile_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (r1 != cudaSuccess || r2 != cudaSuccess) return (int)(r1 != cudaSuccess ? r1 : r2);
+    if (r0 != cudaSuccess || r1 != cudaSuccess || r2 != cudaSuccess) return (int)(r0 != cudaSuccess ? r0 : r1 != cudaSuccess ? r1 : r2);
     vm_launch_pdl(experts_up_tile_kernel, dim3(E * (ff / UP_ROWS) + ff_shared / UP_ROWS), dim3(UP_WARPS * 32), (size_t)T * top * sizeof(int), stream,
                   (const __nv_bfloat16*)x, (const __nv_bfloat16*)w_up, (const __nv_bfloat16*)w_up_shared, chosen, weight, z, T * top >= E ? 1 : 0,
                   (__nv_bfloat16*)act);
