@@ -175,6 +175,26 @@ def test_an_infinite_value_stays_infinite():
     assert bool(torch.isposinf(got[0, :, 3]).all()) and bool(torch.isfinite(got[0, :, 4:]).all()) and bool(torch.isfinite(got[0, :, :3]).all())
 
 
+@pytest.mark.parametrize("name", ["tile", "rows"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_biases_at_the_ends_of_the_type(name, dtype):
+    """The lowest float as a mask: on the far keys (they get no weight), on every key (they all get the same, as in float32 arithmetic), and a sink of
+    the lowest and the largest float."""
+    if name == "tile" and dtype == torch.float32:
+        pytest.skip("bfloat16 only")
+    least = torch.finfo(torch.float32).min
+    for rel, sink in ((torch.arange(7)[:, None].expand(7, 4) > 2, None), (torch.ones(7, 4, dtype=torch.bool), None), (None, least), (None, -least)):
+        s = Step(4, 1, 64, 64, [0, 40, 300], [1] * 3, dtype)
+        if rel is not None:
+            s.rel = torch.where(rel, torch.full((7, 4), least), s.rel)
+            s.bucket = (torch.arange(s.far + 1) * 7 // (s.far + 1)).int()
+        if sink is not None:
+            s.sink = torch.full((4,), sink)
+        options = (0, 0, 0, rel is not None, sink is not None, False, 0.125)
+        got, want = s.run(name, *options), s.want(*options)
+        assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all())
+
+
 def test_a_missing_page_is_reported():
     s = Step(4, 1, 64, 64, [200], [1], torch.bfloat16)
     s.table[0, 1] = -1

@@ -37,6 +37,13 @@ __device__ __forceinline__ void store_to(int rank, float* local, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
 }
 
+// a bias, slope or sink in the softmax's base-2 units; a finite one stays finite (the lowest float, as masks use it, times log2(e) is not, and a row whose
+// keys all carry it would have no largest score)
+__device__ __forceinline__ float base2(float v) {
+    const float y = v * 1.4426950408889634f;
+    return isinf(y) && !isinf(v) ? copysignf(3.402823466e38f, v) : y;
+}
+
 // two bfloat16 with every infinity and NaN replaced by zero
 __device__ __forceinline__ unsigned finite_only(unsigned v) {
     const unsigned bad = __vcmpeq2(v & 0x7f807f80u, 0x7f807f80u);
@@ -65,7 +72,6 @@ attn_decode_tile_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, c
                         __nv_bfloat16* __restrict__ out, int H, int Hkv, float scale_log2, int window, int keep_first, int chunk, int n_pages,
                         const float* __restrict__ sink, const float* __restrict__ slopes, int v_stride, int* __restrict__ err) {
     constexpr int RF = row_floats<DV>(), KB = DK / 32, VH = DV / 64;
-    constexpr float LOG2E = 1.4426950408889634f;
     extern __shared__ __align__(16) float part[];          // [WARPS][ROWS][RF]; with splits also [splits][share of the outputs]
     __shared__ float fac[WARPS][ROWS], row_top[MAX_SPLITS][ROWS], row_sum[MAX_SPLITS][ROWS];
     const int split = blockIdx.x, splits = gridDim.x, b = blockIdx.z;
@@ -97,7 +103,7 @@ attn_decode_tile_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, c
             qb[kb] = g + 8 < ng ? *reinterpret_cast<const uint4*>(row + (size_t)(g + 8) * DK + kb * 32) : make_uint4(0u, 0u, 0u, 0u);
         }
     }
-    const float slope_a = slopes && g < ng ? slopes[h0 + g] * LOG2E : 0.f, slope_b = slopes && g + 8 < ng ? slopes[h0 + g + 8] * LOG2E : 0.f;
+    const float slope_a = slopes && g < ng ? base2(slopes[h0 + g]) : 0.f, slope_b = slopes && g + 8 < ng ? base2(slopes[h0 + g + 8]) : 0.f;
     float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.f, l_b = 0.f;
     float o[VH * 8][4];
 #pragma unroll
@@ -144,8 +150,8 @@ attn_decode_tile_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, c
                 for (int e = 0; e < 2; ++e) {
                     const int away = pos - (base + nb * 8 + 2 * t4 + e);
                     const float* row = rel + (size_t)bucket_of[min(max(away, 0), far)] * H + h0;
-                    bias[nb][e] = g < ng ? row[g] * LOG2E : 0.f;
-                    bias[nb][2 + e] = g + 8 < ng ? row[g + 8] * LOG2E : 0.f;
+                    bias[nb][e] = g < ng ? base2(row[g]) : 0.f;
+                    bias[nb][2 + e] = g + 8 < ng ? base2(row[g + 8]) : 0.f;
                 }
         }
         page = c + splits * WARPS < n_chunks ? page_of(base_of(c + splits * WARPS)) : -1;
@@ -289,7 +295,7 @@ attn_decode_tile_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, c
         }
         float keep = 1.f;
         if (sink) {                                        // exp(sink): one more term of the denominator, without a value
-            const float sk = sink[h0 + r] * LOG2E, top = fmaxf(M, sk);
+            const float sk = base2(sink[h0 + r]), top = fmaxf(M, sk);
             keep = exp2f(M - top);
             L = L * keep + exp2f(sk - top);
         }
