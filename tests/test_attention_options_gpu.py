@@ -101,12 +101,14 @@ class Step:
         few.H, few.Hkv = n, max(1, n // (self.H // self.Hkv)) if n < self.H else self.Hkv
         return few.want(*options)
 
-    def run(self, name, window, keep, chunk, rel, sink, slopes, scale, tokens=None):
+    def call(self, name, window, keep, chunk, rel, sink, slopes, scale, tokens=None, n_seqs=0, width=None):
+        """The kernel's outputs, its status and the error word; width: columns of the block table."""
         at = slice(0, self.T) if tokens is None else tokens
         n = len(range(*at.indices(self.T)))
         out = torch.full((n, self.H, self.Dv), float("nan"), dtype=self.dtype, device=DEV)
         err = torch.zeros(1, dtype=torch.int32, device=DEV)
-        dev = [t.to(DEV) for t in (self.q[at].contiguous(), self.table, self.positions[at].contiguous(), self.seq[at].contiguous(), self.rel, self.bucket, self.sink, self.slopes)]
+        blocks = self.table if width is None else torch.nn.functional.pad(self.table, (0, max(0, width - self.table.shape[1])), value=-1)[:, :width].contiguous()
+        dev = [t.to(DEV) for t in (self.q[at].contiguous(), blocks, self.positions[at].contiguous(), self.seq[at].contiguous(), self.rel, self.bucket, self.sink, self.slopes)]
         q, table, pos, seq, r, b, sk, sl = dev
         head = [_p(q), _i(self.stride), _p(self.kp), _p(self.vp), _p(table), _i(table.shape[1]), _p(pos)]
         opts = [_p(r if rel else None), _p(b if rel else None), _i(self.far if rel else 0), _p(sk if sink else None), _p(sl if slopes else None),
@@ -117,12 +119,15 @@ class Step:
             cu = torch.tensor([0] + list(np.cumsum(new)), dtype=torch.int32, device=DEV)
             rc = _lib().vm_attention_sink_prefill_bf16(*head, _p(cu), _i(len(new)), _i(sum(-(-m // 64) for m in new)), *opts[:3], _i(7 if rel else 0), *opts[3:], *sizes, _p(err), _stream())
         elif name == "rows":
-            rc = _lib().vm_attention_sink_generic(*head, _p(seq), *opts, _i(n), *sizes, _i(0 if self.dtype == torch.float32 else 1), _p(err), _stream())
+            rc = _lib().vm_attention_sink_generic_seqs(*head, _p(seq), *opts, _i(n), *sizes, _i(0 if self.dtype == torch.float32 else 1), _p(err), _i(n_seqs), _stream())
         else:
             rc = _lib().vm_attention_sink_decode_bf16(*head, *opts, _i(n), *sizes, _p(err), _stream())
-        assert rc == 0
-        assert int(err.item()) == 0
-        return out.cpu()
+        return out.cpu(), rc, int(err.item())
+
+    def run(self, *args, **more):
+        out, rc, err = self.call(*args, **more)
+        assert (rc, err) == (0, 0)
+        return out
 
 
 # window, kept first tokens, chunk, bias, sink, slopes
@@ -146,6 +151,23 @@ def test_rows_do_not_depend_on_the_batch_or_the_cut():
     whole = s.run("rows", 50, 3, 0, False, True, False, 0.125)
     for a, b in ((0, 1), (149, 152), (140, 160), (245, 246)):
         assert torch.equal(whole[a:b], s.run("rows", 50, 3, 0, False, True, False, 0.125, slice(a, b)))
+
+
+@pytest.mark.parametrize("H,Hkv,D", [(32, 32, 64), (9, 3, 64), (16, 1, 128), (12, 12, 20)])
+@pytest.mark.parametrize("before,new,widths", [([0, 7, 31, 32, 50, 62, 63] * 6, [1] * 42, (1, 2, 3)), ([0, 33, 64, 100, 126, 127] * 6, [1] * 36, (2, 3)),
+                                               ([70, 128, 300, 511, 90] * 8, [1] * 40, (8, 9)), ([0, 20, 3] * 12, [3, 40, 1] * 12, (1, 2, 3)), ([0, 1, 60], [30, 2, 4], (1, 4))])
+def test_rows_of_many_sequences(H, Hkv, D, before, new, widths):
+    """Decode batches and prompts side by side, in tables of one page, two and more: however tokens are dealt out to CTAs and keys to
+    warps, the same bits; and the right ones."""
+    s = Step(H, Hkv, D, D, before, new, torch.float32)
+    options = (0, 0, 0, False, False, False, D ** -0.5)
+    got = s.run("rows", *options, n_seqs=len(new), width=widths[0])
+    for width in widths:
+        for n_seqs in (0, len(new)):
+            assert torch.equal(got, s.run("rows", *options, n_seqs=n_seqs, width=width)), (width, n_seqs)
+    some = torch.arange(0, s.T, max(1, s.T // 40))
+    heads = slice(0, H // Hkv) if Hkv > 1 else slice(0, H)             # (heads compared: the reference is slow)
+    assert float((got[some][:, heads].double() - s.want_some(some, heads, *options)).abs().max()) <= 1e-5
 
 
 @pytest.mark.parametrize("H,Hkv,Dk,Dv,in_keys", [(8, 8, 64, 64, False), (16, 4, 64, 64, False), (4, 2, 64, 128, False), (6, 2, 96, 64, False), (4, 4, 128, 64, False), (3, 1, 96, 128, False),

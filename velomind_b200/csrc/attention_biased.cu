@@ -316,11 +316,11 @@ VM_API int vm_attention_biased_generic(const void* q, int q_row_stride, const vo
 // The same with a sink and values that may lie inside the key rows.  sink float32 [H] (null: none): exp(sink[h]) is one more term
 // of head h's softmax denominator, without a key or a value, not scaled.  v_row_stride: elements from one token's value row to the
 // next in `vpages` (0: Dv); with vpages == kpages and v_row_stride == Dk a token's value is the first Dv values of its key row.
-// slopes float32 [H] (null: none): slopes[h] * (i - j) is taken off head h's score of key j.  chunk > 0: a chunked mask.
-VM_API int vm_attention_sink_generic(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
-                                     const int* positions, const int* seq_of_token, const float* rel, const int* bucket_of, int far, const float* sink,
-                                     const float* slopes, int v_row_stride, void* out, int n_tokens, int H, int Hkv, int Dk, int Dv, float scale, int window, int keep_first,
-                                     int chunk, int n_pages, int act_dtype, int* err, cudaStream_t stream) {
+// slopes float32 [H] (null: none): slopes[h] * (i - j) is taken off head h's score of key j.  chunk > 0: a chunked mask.  n_seqs as in vm_attention_rows.
+VM_API int vm_attention_sink_generic_seqs(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
+                                          const int* positions, const int* seq_of_token, const float* rel, const int* bucket_of, int far, const float* sink,
+                                          const float* slopes, int v_row_stride, void* out, int n_tokens, int H, int Hkv, int Dk, int Dv, float scale,
+                                          int window, int keep_first, int chunk, int n_pages, int act_dtype, int* err, int n_seqs, cudaStream_t stream) {
     const int v_stride = v_row_stride > 0 ? v_row_stride : Dv;
     if (v_stride < Dv) return VM_ERR_BAD_ARG;
     if (n_tokens <= 0) return 0;
@@ -328,7 +328,7 @@ VM_API int vm_attention_sink_generic(const void* q, int q_row_stride, const void
     if ((rel != nullptr) != (bucket_of != nullptr) || (rel && far < 0)) return VM_ERR_BAD_ARG;
     if ((act_dtype == VM_F32 || act_dtype == VM_BF16) && vm_attention_rows_fits(kpages, vpages, H, Hkv, Dk, Dv, v_stride))
         return vm_attention_rows(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, rel, bucket_of, far, sink, slopes, v_stride,
-                                 out, n_tokens, H, Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, act_dtype, err, stream);
+                                 out, n_tokens, H, Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, act_dtype, err, n_seqs, stream);
     if (act_dtype == VM_F32)
         return launch_biased<float>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, rel, bucket_of, far, out, n_tokens, H,
                                     Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, sink, slopes, v_stride, err, stream);
@@ -336,4 +336,12 @@ VM_API int vm_attention_sink_generic(const void* q, int q_row_stride, const void
         return launch_biased<__nv_bfloat16>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, rel, bucket_of, far, out,
                                             n_tokens, H, Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, sink, slopes, v_stride, err, stream);
     return VM_ERR_UNSUPPORTED;
+}
+
+VM_API int vm_attention_sink_generic(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
+                                     const int* positions, const int* seq_of_token, const float* rel, const int* bucket_of, int far, const float* sink,
+                                     const float* slopes, int v_row_stride, void* out, int n_tokens, int H, int Hkv, int Dk, int Dv, float scale, int window, int keep_first,
+                                     int chunk, int n_pages, int act_dtype, int* err, cudaStream_t stream) {
+    return vm_attention_sink_generic_seqs(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, rel, bucket_of, far, sink, slopes,
+                                          v_row_stride, out, n_tokens, H, Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, act_dtype, err, 0, stream);
 }

@@ -107,16 +107,16 @@ static int launch_generic(const void* q, int q_row_stride, const void* kpages, c
     return vm_launch_status();
 }
 
-// q: [n_tokens, H, D] rows with stride q_row_stride elements; out: [n_tokens, H*D] contiguous.
-VM_API int vm_attention_generic(const void* q, int q_row_stride, const void* kpages, const void* vpages,
-                                const int* block_table, int max_blocks, const int* positions, const int* seq_of_token,
-                                void* out, int n_tokens, int H, int Hkv, int D, float scale, int window, int n_pages,
-                                int act_dtype, int* err, cudaStream_t stream) {
+// q: [n_tokens, H, D] rows with stride q_row_stride elements; out: [n_tokens, H*D] contiguous.  n_seqs as in vm_attention_rows.
+VM_API int vm_attention_generic_seqs(const void* q, int q_row_stride, const void* kpages, const void* vpages,
+                                     const int* block_table, int max_blocks, const int* positions, const int* seq_of_token,
+                                     void* out, int n_tokens, int H, int Hkv, int D, float scale, int window, int n_pages,
+                                     int act_dtype, int* err, int n_seqs, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (H <= 0 || Hkv <= 0 || H % Hkv != 0 || D <= 0 || D > 512) return VM_ERR_UNSUPPORTED;
     if ((act_dtype == VM_F32 || act_dtype == VM_BF16) && vm_attention_rows_fits(kpages, vpages, H, Hkv, D, D, D))
         return vm_attention_rows(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, nullptr, nullptr, 0, nullptr, nullptr, D,
-                                 out, n_tokens, H, Hkv, D, D, scale, window, 0, 0, n_pages, act_dtype, err, stream);
+                                 out, n_tokens, H, Hkv, D, D, scale, window, 0, 0, n_pages, act_dtype, err, n_seqs, stream);
     if (act_dtype == VM_F32)
         return launch_generic<float>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, out,
                                      n_tokens, H, Hkv, D, scale, window, n_pages, err, stream);
@@ -124,4 +124,11 @@ VM_API int vm_attention_generic(const void* q, int q_row_stride, const void* kpa
         return launch_generic<__nv_bfloat16>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token,
                                              out, n_tokens, H, Hkv, D, scale, window, n_pages, err, stream);
     return VM_ERR_UNSUPPORTED;
+}
+
+VM_API int vm_attention_generic(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
+                                const int* positions, const int* seq_of_token, void* out, int n_tokens, int H, int Hkv, int D, float scale, int window,
+                                int n_pages, int act_dtype, int* err, cudaStream_t stream) {
+    return vm_attention_generic_seqs(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, out, n_tokens, H, Hkv, D, scale, window,
+                                     n_pages, act_dtype, err, 0, stream);
 }

@@ -5,11 +5,13 @@
 // What bounds it is latency: a decode step of a few sequences is a chain of loads.  With one warp per (token, head) that chain was as
 // long as the context (120 us for four tokens of 9 heads at 190 cached tokens, 122 us for 446 tokens of four prompts).  Here a CTA owns up to
 // eight query rows that share a kv head (the heads of its group, of one or more neighbouring tokens), and its eight warps share the
-// keys: a chunk of 32 keys, one key per lane, belongs to the warp with its number modulo eight.  The key rows come as whole lines, all in
+// keys: a chunk of 32 keys, one key per lane, belongs to the warp with its number modulo eight (a table of one or two pages has two or four chunks, and
+// the CTA as many warps).  The key rows come as whole lines, all in
 // flight, and pass through the warp's own shared memory (a lane that reads its row from global memory touches a line of its own with every
 // load: 5 us a chunk instead of 2); a value row is one line; the probabilities come from shared memory four at a time; the warps' sums meet
 // in warp order at the end.
-// Measured at those sizes: 10.5 us and 59 us; one prompt of 190, 446 and 2,048 tokens 25, 75 and 800 us (90, 322 and 5,049 before), one of 8 tokens 7.0 (5.7).
+// Measured at those sizes: 6.2 us and 59 us; one prompt of 8, 190, 446 and 2,048 tokens 4.7, 24, 75 and 800 us (5.7, 90, 322 and 5,049 before).  Where there
+// are hardly any keys the join costs more than it saves: a first token alone 4.3 us (3.9 before), sixteen prompts of 8 tokens and 9 heads 8.5 (6.8).
 //
 // The result for a query depends on its own place alone: chunks start at absolute multiples of 32, which warp takes one follows from its
 // absolute number, every dot product is summed in index order by one lane, and the other rows of a CTA never enter a row's arithmetic.
@@ -18,7 +20,6 @@
 
 namespace {
 
-constexpr int WARPS = 8;
 constexpr int MAX_ROWS = 8;
 constexpr int KEYS = 32;                 // keys of a warp's turn
 constexpr int SLICE = 64;                // columns of the keys in shared memory at a time
@@ -36,8 +37,8 @@ __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
 __device__ __forceinline__ float2 load2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ float2 load2(const __nv_bfloat16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
 
-// R: query rows of a CTA (a power of two); VP: pairs of value columns per lane, 2 lane + 64 i and the next
-template <typename T, int R, int VP>
+// R: query rows of a CTA (a power of two); VP: pairs of value columns per lane, 2 lane + 64 i and the next; WARPS: 8, or as many as the table has chunks
+template <typename T, int R, int VP, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
 attn_rows_kernel(const T* __restrict__ q, int q_row_stride, const T* __restrict__ kpages, const T* __restrict__ vpages,
                  const int* __restrict__ block_table, int max_blocks, const int* __restrict__ positions, const int* __restrict__ seq_of_token,
@@ -77,6 +78,17 @@ attn_rows_kernel(const T* __restrict__ q, int q_row_stride, const T* __restrict_
             }
             if (++h == h0 + heads) { h = h0; ++t; }
         }
+        // this warp's first chunk (not between the kept tokens and the window) and its page, asked for before the queries' barrier
+        auto next_chunk = [&](int c) {
+            if (c * 32 >= kept_most && c < lowest / 32) c += (lowest / 32 - c + WARPS - 1) / WARPS * WARPS;
+            return c;
+        };
+        auto page_of = [&](int c) {
+            const int blk = c * 32 / VM_PAGE_TOKENS;
+            return c * 32 <= highest && blk < max_blocks ? block_table[(size_t)seq * max_blocks + blk] : -1;
+        };
+        int c = next_chunk(warp), page = page_of(c);
+        const int first = c * 32;
         for (int i = threadIdx.x; i < R * Dk; i += WARPS * 32) {
             const int r = i / Dk, d = i - r * Dk;
             sq[i] = r < rows ? vm_to_float(q[(size_t)(t0 + r / heads) * q_row_stride + (size_t)(h0 + r % heads) * Dk + d]) * scale : 0.f;
@@ -90,14 +102,9 @@ attn_rows_kernel(const T* __restrict__ q, int q_row_stride, const T* __restrict_
             for (int i = 0; i < VP; ++i) acc[r][i][0] = acc[r][i][1] = 0.f;
         }
         float* mine = sp + warp * R * 32;
-        for (int c = warp; c * 32 <= highest; c += WARPS) {
+        for (; c * 32 <= highest; c = next_chunk(c + WARPS)) {
             const int base = c * 32;
-            if (base >= kept_most && c < lowest / 32) {              // between the kept tokens and the window: on to this warp's first chunk there
-                c += (lowest / 32 - c - 1) / WARPS * WARPS;
-                continue;
-            }
-            const int blk = base / VM_PAGE_TOKENS;
-            const int page = (blk < max_blocks) ? block_table[(size_t)seq * max_blocks + blk] : -1;
+            if (base != first) page = page_of(c);
             if (page < 0 || page >= n_pages) {             // a page the step needs is not there: report, skip
                 if (lane == 0 && err) atomicExch(err, VM_ERRWORD_CACHE_READ);
                 continue;
@@ -276,18 +283,18 @@ attn_rows_kernel(const T* __restrict__ q, int q_row_stride, const T* __restrict_
     }
 }
 
-template <typename T, int R, int VP>
+template <typename T, int R, int VP, int WARPS>
 int launch_rows(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks, const int* positions,
                 const int* seq_of_token, const float* rel, const int* bucket_of, int far, void* out, int n_tokens, int tile_tokens, int H, int Hkv,
                 int Dk, int Dv, float scale, int window, int keep_first, int chunk, int n_pages, const float* sink, const float* slopes, int v_stride,
                 int* err, cudaStream_t stream) {
     const size_t keys = (size_t)WARPS * KEYS * pitch<T>() * sizeof(T), sums = (size_t)WARPS * R * (Dv + 2) * sizeof(float);
     const size_t smem = ((size_t)R * Dk + (size_t)WARPS * R * 32) * sizeof(float) + (keys > sums ? keys : sums);
-    static const cudaError_t raised = cudaFuncSetAttribute(attn_rows_kernel<T, R, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+    static const cudaError_t raised = cudaFuncSetAttribute(attn_rows_kernel<T, R, VP, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
     if (raised != cudaSuccess) return (int)raised;
     const int G = H / Hkv;
     const dim3 grid((n_tokens + tile_tokens - 1) / tile_tokens, Hkv * ((G + R - 1) / R));
-    attn_rows_kernel<T, R, VP><<<grid, WARPS * 32, smem, stream>>>((const T*)q, q_row_stride, (const T*)kpages, (const T*)vpages, block_table, max_blocks,
+    attn_rows_kernel<T, R, VP, WARPS><<<grid, WARPS * 32, smem, stream>>>((const T*)q, q_row_stride, (const T*)kpages, (const T*)vpages, block_table, max_blocks,
                                                                    positions, seq_of_token, rel, bucket_of, far, (T*)out, n_tokens, tile_tokens, H, Hkv,
                                                                    Dk, Dv, scale, window, keep_first, chunk, n_pages, sink, slopes, v_stride, err);
     return vm_launch_status();
@@ -297,22 +304,33 @@ template <typename T>
 int dispatch_rows(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks, const int* positions,
                   const int* seq_of_token, const float* rel, const int* bucket_of, int far, void* out, int n_tokens, int H, int Hkv, int Dk, int Dv,
                   float scale, int window, int keep_first, int chunk, int n_pages, const float* sink, const float* slopes, int v_stride, int* err,
-                  cudaStream_t stream) {
-    // Rows of a CTA: a token's heads of one group; of several neighbouring tokens (as many as make eight rows) once there are more CTAs
-    // than two per SM without that.  None of it changes a row's result.
-    const int G = H / Hkv;
-    int tile = 1;
-    if (G < MAX_ROWS && (long long)n_tokens * Hkv > 2ll * vm_sm_count()) tile = MAX_ROWS / G;
-    int R = 1;
-    while (R < MAX_ROWS && R < G * tile) R *= 2;
+                  int n_seqs, cudaStream_t stream) {
+    // None of what is chosen here changes a row's result, so all of it may follow from the step's shape.
+    // Warps: eight, or a table's two or four chunks of keys and no more: 64 tokens or fewer leave two warps with work, and the CTAs are smaller (30 tokens
+    // of 9 heads 5.4 us with two warps, 8.2 with eight; 16 sequences of 60 tokens, 32 heads 6.2 / 19.7).
+    // Rows: as few as keep the CTAs within what the SMs hold side by side (a CTA's chain grows with its rows: one sequence of 190 tokens and
+    // 9 heads 6.4 / 7.2 / 8.9 us with 1 / 2 / 4 rows), then as many as a kv head has, up to eight (64 sequences of 500 tokens and 9 heads 26.7 us
+    // with 4 rows, 29.7 with 2, 34.4 with 1; a prompt of 446 tokens 75 us with 8, 158 with 1).
+    // Neighbouring tokens share a CTA only as far as sequences bring several: those of different sequences are taken one after another (16 sequences of 190
+    // tokens, 32 heads without groups: 21.7 us a CTA per token, 81 us with eight tokens in a CTA).
+    const int G = H / Hkv, warps = max_blocks <= 1 ? 2 : max_blocks <= 2 ? 4 : 8;
+    const int together = n_seqs > 0 ? (n_tokens / n_seqs > 1 ? n_tokens / n_seqs : 1) : n_tokens;
+    const long long room = (long long)vm_sm_count() * 8 / warps;
+    int R = 1, tile = 1;
+    for (;; R *= 2) {
+        tile = R / G < 1 ? 1 : R / G < together ? R / G : together;
+        if (R == MAX_ROWS || R >= (long long)G * together || (n_tokens + tile - 1ll) / tile * Hkv * ((G + R - 1) / R) <= room) break;
+    }
     const int vp = (Dv + 63) / 64;
-#define VM_ROWS(RR, P)                                                                                                                          \
-    if (R == RR && vp <= P)                                                                                                                     \
-        return launch_rows<T, RR, P>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, rel, bucket_of, far, out, \
-                                     n_tokens, tile, H, Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, sink, slopes, v_stride, err, stream);
+#define VM_ROWS_WARPS(RR, P, W)                                                                                                                 \
+    if (R == RR && vp <= P && warps == W)                                                                                                       \
+        return launch_rows<T, RR, P, W>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, rel, bucket_of, far, out, \
+                                        n_tokens, tile, H, Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, sink, slopes, v_stride, err, stream);
+#define VM_ROWS(RR, P) VM_ROWS_WARPS(RR, P, 2) VM_ROWS_WARPS(RR, P, 4) VM_ROWS_WARPS(RR, P, 8)
     VM_ROWS(1, 1) VM_ROWS(2, 1) VM_ROWS(4, 1) VM_ROWS(8, 1)
     VM_ROWS(1, 2) VM_ROWS(2, 2) VM_ROWS(4, 2) VM_ROWS(8, 2)
 #undef VM_ROWS
+#undef VM_ROWS_WARPS
     return VM_ERR_UNSUPPORTED;
 }
 
@@ -326,17 +344,18 @@ VM_API int vm_attention_rows_fits(const void* kpages, const void* vpages, int H,
                : 0;
 }
 
+// n_seqs: sequences of the step (0: not known, its tokens are taken for a prompt's)
 VM_API int vm_attention_rows(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
                              const int* positions, const int* seq_of_token, const float* rel, const int* bucket_of, int far, const float* sink,
                              const float* slopes, int v_stride, void* out, int n_tokens, int H, int Hkv, int Dk, int Dv, float scale, int window,
-                             int keep_first, int chunk, int n_pages, int act_dtype, int* err, cudaStream_t stream) {
+                             int keep_first, int chunk, int n_pages, int act_dtype, int* err, int n_seqs, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (!vm_attention_rows_fits(kpages, vpages, H, Hkv, Dk, Dv, v_stride)) return VM_ERR_UNSUPPORTED;
     if (act_dtype == VM_F32)
         return dispatch_rows<float>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, rel, bucket_of, far, out, n_tokens, H,
-                                    Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, sink, slopes, v_stride, err, stream);
+                                    Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, sink, slopes, v_stride, err, n_seqs, stream);
     if (act_dtype == VM_BF16)
         return dispatch_rows<__nv_bfloat16>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, rel, bucket_of, far, out,
-                                            n_tokens, H, Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, sink, slopes, v_stride, err, stream);
+                                            n_tokens, H, Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, sink, slopes, v_stride, err, n_seqs, stream);
     return VM_ERR_UNSUPPORTED;
 }

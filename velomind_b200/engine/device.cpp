@@ -548,8 +548,8 @@ void attention(StepContext& ctx, const void* q, int q_row_stride, const KVView& 
         return;
     }
     Timed t("attention_generic", s);
-    check(vm_attention_generic(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, ctx.seq_of_token, out, ctx.T, H,
-                               Hkv, D, scale, window, kv.n_pages, code(ctx.act_dtype), ctx.err, s),
+    check(vm_attention_generic_seqs(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, ctx.seq_of_token, out, ctx.T, H,
+                                    Hkv, D, scale, window, kv.n_pages, code(ctx.act_dtype), ctx.err, ctx.B, s),
           "attention_generic", s);
 }
 
@@ -590,9 +590,9 @@ void attention_biased(StepContext& ctx, const void* q, int q_row_stride, const K
         return;
     }
     Timed t("attention_biased_generic", s);
-    check(vm_attention_sink_generic(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, ctx.seq_of_token, mask.rel,
-                                    mask.bucket_of, mask.far, mask.sink, mask.slopes, mask.v_row_stride, out, ctx.T, H, Hkv, Dk, Dv, scale, mask.window, mask.keep_first, mask.chunk,
-                                    kv.n_pages, code(ctx.act_dtype), ctx.err, s),
+    check(vm_attention_sink_generic_seqs(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, ctx.seq_of_token, mask.rel,
+                                         mask.bucket_of, mask.far, mask.sink, mask.slopes, mask.v_row_stride, out, ctx.T, H, Hkv, Dk, Dv, scale, mask.window,
+                                         mask.keep_first, mask.chunk, kv.n_pages, code(ctx.act_dtype), ctx.err, ctx.B, s),
           "attention_biased_generic", s);
 }
 

@@ -184,6 +184,11 @@ int vm_attention_sink_generic(const void* q, int q_row_stride, const void* kpage
                               const int* positions, const int* seq_of_token, const float* rel, const int* bucket_of, int far, const float* sink, const float* slopes,
                               int v_row_stride, void* out, int n_tokens, int H, int Hkv, int Dk, int Dv, float scale, int window, int keep_first,
                               int chunk, int n_pages, int act_dtype, int* err, cudaStream_t stream);
+// the same with the number of the step's sequences (0: not known), which decides how many neighbouring tokens share a CTA; results are the same
+int vm_attention_sink_generic_seqs(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
+                                   const int* positions, const int* seq_of_token, const float* rel, const int* bucket_of, int far, const float* sink,
+                                   const float* slopes, int v_row_stride, void* out, int n_tokens, int H, int Hkv, int Dk, int Dv, float scale, int window,
+                                   int keep_first, int chunk, int n_pages, int act_dtype, int* err, int n_seqs, cudaStream_t stream);
 int vm_attention_sink_prefill_fits(int Dk, int Dv, int values_in_keys);
 int vm_attention_sink_prefill_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
                                    const int* positions, const int* cu_tokens, int B, int n_tiles, const float* rel, const int* bucket_of, int far,
@@ -255,15 +260,18 @@ int vm_skinny_f32(const float* x, long long ldx, const float* w, float* out, int
 int vm_skinny_f32_fused(const float* x, long long ldx, const float* norm_w, float eps, const float* w, float* out, int T, int N, int K, int add, int swiglu,
                         cudaStream_t stream);
 // ---- attention_rows.cu: the float32 arithmetic of the plain kernels with a query's keys spread over a CTA (arguments as vm_attention_sink_generic;
-// v_stride is given); vm_attention_generic and vm_attention_sink_generic call it where it takes the sizes
+// v_stride is given, n_seqs as in vm_attention_sink_generic_seqs); vm_attention_generic and vm_attention_sink_generic call it where it takes the sizes
 int vm_attention_rows_fits(const void* kpages, const void* vpages, int H, int Hkv, int Dk, int Dv, int v_stride);
 int vm_attention_rows(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
                       const int* positions, const int* seq_of_token, const float* rel, const int* bucket_of, int far, const float* sink,
                       const float* slopes, int v_stride, void* out, int n_tokens, int H, int Hkv, int Dk, int Dv, float scale, int window,
-                      int keep_first, int chunk, int n_pages, int act_dtype, int* err, cudaStream_t stream);
+                      int keep_first, int chunk, int n_pages, int act_dtype, int* err, int n_seqs, cudaStream_t stream);
 int vm_attention_generic(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
                          int max_blocks, const int* positions, const int* seq_of_token, void* out, int n_tokens, int H, int Hkv,
                          int D, float scale, int window, int n_pages, int act_dtype, int* err, cudaStream_t stream);
+int vm_attention_generic_seqs(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
+                              const int* positions, const int* seq_of_token, void* out, int n_tokens, int H, int Hkv, int D, float scale, int window,
+                              int n_pages, int act_dtype, int* err, int n_seqs, cudaStream_t stream);      // n_seqs as in vm_attention_sink_generic_seqs
 int vm_attention_prefill_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
                               int max_blocks, const int* positions, const int* cu_tokens, int B, int n_tiles, void* out, int H,
                               int Hkv, int D, float scale, int window, int n_pages, int* err, int groups, cudaStream_t stream);
