@@ -84,11 +84,35 @@ def _choice(z, kind, top, groups, keep, gtop, correction, normalize, scale):
     return i, w / (w.sum(-1, keepdim=True) + 1e-20) * scale if normalize else w * scale
 
 
-@pytest.mark.parametrize("T", [1, 8, 149, 163, 700])
+def _check_choice(x, w, z, chosen, kind, groups, gtop, correction):
+    """Every output was the best one left to choose, up to the error of 32-bit sums: hidden / 16 + 16 additions in a row, however the kernels cut
+    them, of 2^-23 (the tensor cores cut off, 2^-24 where they round) of the sum of the products' magnitudes."""
+    n = chosen.long()
+    assert bool((n.sort(-1).values.diff(dim=-1) > 0).all())
+    e = (w.shape[1] / 16 + 16) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T).max(-1, keepdim=True).values
+    s = z if kind == "chosen" else torch.softmax(z, -1) if kind == "softmax" else torch.sigmoid(z)
+    with_corr = s if correction is None else s + correction.double()
+    c = z if kind == "sigmoid" and correction is None else with_corr
+    e = e if c is z else 2.1 * e + 2.0 ** -22                           # a softmax moves by at most twice its logits
+    left = torch.ones_like(c, dtype=torch.bool)
+    if groups > 1:
+        per = c.shape[1] // groups
+        mine = n // per
+        assert bool((mine == mine[:, :1]).all())
+        score = with_corr.reshape(len(c), groups, per).topk(gtop, -1).values.sum(-1)
+        assert bool((score.gather(1, mine[:, :1]) >= score.max(-1, keepdim=True).values - 2 * gtop * e).all())
+        left = torch.arange(c.shape[1], device=c.device) // per == mine[:, :1]
+    for k in range(n.shape[1]):
+        best = c.masked_fill(~left, -1e30).max(-1, keepdim=True).values
+        assert bool((c.gather(1, n[:, k:k + 1]) >= best - 2 * e).all()), k
+        left = left & ~torch.zeros_like(left).scatter_(1, n[:, k:k + 1], True)
+
+
+@pytest.mark.parametrize("T", [1, 8, 149, 163, 700, 905, 1201])
 @pytest.mark.parametrize("hidden,n_out,top,kind", [(1024, 16, 4, "chosen"), (96, 18, 4, "softmax"), (2048, 32, 4, "sigmoid"), (64, 5, 2, "chosen"), (160, 64, 6, "sigmoid"), (72, 9, 3, "softmax")])
 def test_routers(T, hidden, n_out, top, kind):
     """One block per token and tiles of sixteen tokens, with a gate row behind the outputs (`chosen`) and with groups: the choice, where no two
-    outputs come close, and the weights (float32 sums of `hidden` terms)."""
+    outputs come closer than the sums' error, and the weights (float32 sums of `hidden` terms)."""
     g = torch.Generator().manual_seed(T + hidden)
     x = torch.randn(T, hidden, generator=g).to(torch.bfloat16).to(DEV)
     w = (torch.randn(n_out, hidden, generator=g) * 2.0 / hidden ** 0.5).to(DEV)
@@ -110,6 +134,31 @@ def test_routers(T, hidden, n_out, top, kind):
     same = (chosen.long() == want[0]).all(-1)
     assert float(same.float().mean()) >= 0.99                       # (near ties may fall either way)
     assert float((weight.double() - want[1])[same].abs().max()) <= 4e-6
+    if kind == "chosen":
+        _check_choice(x, w, z + b.double(), chosen, kind, 1, 1, None)
+    else:
+        _check_choice(x, w, z, chosen, kind, groups, gtop, corr)
+
+
+@pytest.mark.parametrize("hidden,n_out", [(1024, 16), (2048, 64), (96, 40)])
+def test_a_router_row_in_a_long_step_and_in_short_ones(hidden, n_out):
+    """The same rows in one step (tiles of tokens) and a hundred at a time (a block per token) add their products up in another order: weights agree to 8e-6
+    (4e-6 each against 64 bits), and a choice differs only where the scores are as close as the sums' error."""
+    g = torch.Generator().manual_seed(hidden)
+    T, top = 1500, 4
+    x = torch.randn(T, hidden, generator=g).to(torch.bfloat16).to(DEV)
+    w, b = (torch.randn(n_out, hidden, generator=g) * 2.0 / hidden ** 0.5).to(DEV), torch.randn(n_out, generator=g).to(DEV)
+    out = []
+    for piece in (T, 100):
+        chosen, weight = torch.full((T, top), -1, dtype=torch.int32, device=DEV), torch.full((T, top), float("nan"), device=DEV)
+        for a in range(0, T, piece):
+            assert _lib().vm_expert_router(_p(x[a:]), None, _f(0), _p(w), _p(b), None, _i(min(piece, T - a)), _i(hidden), _i(n_out), _i(top), _p(chosen[a:]), _p(weight[a:]), None,
+                                           _i(1), _stream()) == 0
+        _check_choice(x, w, x.double() @ w.double().T + b.double(), chosen, "chosen", 1, 1, None)
+        out.append((chosen, weight))
+    same = (out[0][0] == out[1][0]).all(-1)
+    assert float(same.float().mean()) >= 0.99
+    assert float((out[0][1] - out[1][1])[same].abs().max()) <= 8e-6
 
 
 @pytest.mark.parametrize("T", [1, 8, 17, 33, 70])

@@ -29,32 +29,33 @@ struct Routing {
 constexpr int AHEAD = 4;                 // pieces of four weights that a lane holds at a time
 
 // a weight row against the input row in shared memory, summed over a warp: lane i takes the pieces of four values i, i + 64, .. and i + 32, i + 96, ..
-// in two chains.  `pre`: the row's first AHEAD pieces, requested earlier (null: none)
-__device__ __forceinline__ float row_dot(const float* __restrict__ w, const float* __restrict__ x, int n, int lane, const float4* pre) {
-    float acc[2] = {0.f, 0.f};
+// in two chains, in a plain loop unrolled UNROLL times with its loads in front (pieces fetched four at a time behind a bound each: 185 -> 255 us for 2,048
+// tokens of width 2,048 and 128 outputs).  `pre`: the row's first AHEAD pieces, requested earlier (null: none)
+template <int UNROLL> __device__ __forceinline__ float row_dot(const float* __restrict__ w, const float* __restrict__ x, int n, int lane, const float4* pre) {
+    float acc = 0.f, acc1 = 0.f;
     if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {
+        const float4* w4 = reinterpret_cast<const float4*>(w);
+        const float4* x4 = reinterpret_cast<const float4*>(x);
+        auto add = [](float& a, const float4& r, const float4& v) { a = fmaf(r.x, v.x, fmaf(r.y, v.y, fmaf(r.z, v.z, fmaf(r.w, v.w, a)))); };
         const int nv = n / 4;
-        for (int j0 = 0; j0 * 32 < nv; j0 += AHEAD) {
-            float4 r[AHEAD];
+        int i = lane;
+        if (pre) {
 #pragma unroll
-            for (int j = 0; j < AHEAD; ++j) {
-                const int i = lane + 32 * (j0 + j);
-                if (i < nv) r[j] = pre && j0 == 0 ? pre[j] : reinterpret_cast<const float4*>(w)[i];
-            }
-#pragma unroll
-            for (int j = 0; j < AHEAD; ++j) {
-                const int i = lane + 32 * (j0 + j);
-                if (i < nv) {
-                    const float4 v = reinterpret_cast<const float4*>(x)[i];
-                    float& a = acc[j & 1];
-                    a = fmaf(r[j].x, v.x, fmaf(r[j].y, v.y, fmaf(r[j].z, v.z, fmaf(r[j].w, v.w, a))));
-                }
-            }
+            for (int j = 0; j < AHEAD; ++j)
+                if (lane + 32 * j < nv) add(j & 1 ? acc1 : acc, pre[j], x4[lane + 32 * j]);
+            i += 32 * AHEAD;
         }
+#pragma unroll UNROLL
+        for (; i + 32 < nv; i += 64) {
+            const float4 a = __ldg(w4 + i), b = __ldg(w4 + i + 32), xa = x4[i], xb = x4[i + 32];
+            add(acc, a, xa);
+            add(acc1, b, xb);
+        }
+        if (i < nv) add(acc, __ldg(w4 + i), x4[i]);
     } else {
-        for (int i = lane; i < n; i += 32) acc[0] = fmaf(w[i], x[i], acc[0]);
+        for (int i = lane; i < n; i += 32) acc = fmaf(w[i], x[i], acc);
     }
-    return vm_warp_sum(acc[0] + acc[1]);
+    return vm_warp_sum(acc + acc1);
 }
 
 // the largest of v[0 .. n) over a warp, the lowest index among equals; 0x7fffffff if none is above -inf
@@ -172,10 +173,11 @@ __device__ void choose_scored(float* sc, float* ch, float* gs, const Routing& r,
 }
 
 // a block per token.  x: rows in the activation dtype T, or (norm_w given) the float32 residual stream: rmsnorm(x) * norm_w, rounded as T would
-// hold it, so that a step gives the same numbers whether the norm ran here or in a kernel of its own
-template <typename T>
-__global__ void __launch_bounds__(1024)
-route_kernel(const void* __restrict__ x, const float* __restrict__ norm_w, float eps, Routing r, int hidden, int* __restrict__ chosen,
+// hold it, so that a step gives the same numbers whether the norm ran here or in a kernel of its own.  PER_SM: blocks that an SM holds.  1: up to 32 warps,
+// first weights ahead of the wait; 4 and 6: 8 warps, more loads in flight or more blocks (1,024 x 16, 512 tokens 7.0 and 8.2 us, 800 tokens 13.1 and 8.2)
+template <typename T, int PER_SM, bool SCORED>
+__global__ void __launch_bounds__(PER_SM == 1 ? 1024 : 256, PER_SM)
+route_kernel(const void* __restrict__ x, const float* __restrict__ norm_w, float eps, const __grid_constant__ Routing r, int hidden, int* __restrict__ chosen,
              float* __restrict__ weight, float* __restrict__ shared_gate, T* __restrict__ rows_out) {
     __shared__ float red[32];
     extern __shared__ __align__(16) float sm[];            // [hidden] input, [n_out] logits, then scores; scored: [n_out] choice scores, [group_count] group scores
@@ -187,7 +189,7 @@ route_kernel(const void* __restrict__ x, const float* __restrict__ norm_w, float
     const int outputs = r.n_out + (r.gate ? 1 : 0);
     auto row = [&](int e) { return e < r.n_out ? r.w + (size_t)e * hidden : r.gate; };
     float4 pre[AHEAD];
-    const bool ahead = warp < outputs && (hidden & 3) == 0 && (reinterpret_cast<uintptr_t>(row(warp)) & 15) == 0;
+    const bool ahead = PER_SM == 1 && warp < outputs && (hidden & 3) == 0 && (reinterpret_cast<uintptr_t>(row(warp)) & 15) == 0;
     if (ahead) {                                           // constants: nothing before this kernel writes them
 #pragma unroll
         for (int j = 0; j < AHEAD; ++j)
@@ -212,7 +214,7 @@ route_kernel(const void* __restrict__ x, const float* __restrict__ norm_w, float
     }
     __syncthreads();
     for (int e = warp; e < outputs; e += nw) {
-        const float d = row_dot(row(e), xs, hidden, lane, ahead && e == warp ? pre : nullptr);
+        const float d = row_dot<PER_SM == 1 ? 4 : PER_SM == 4 ? 2 : 1>(row(e), xs, hidden, lane, ahead && e == warp ? pre : nullptr);
         if (lane == 0) {
             if (e < r.n_out) sc[e] = d + (r.bias ? r.bias[e] : 0.f);
             else shared_gate[t] = 1.0f / (1.0f + expf(-d));
@@ -220,7 +222,7 @@ route_kernel(const void* __restrict__ x, const float* __restrict__ norm_w, float
     }
     __syncthreads();
     if (warp != 0) return;
-    if (r.scored) choose_scored(sc, ch, gs, r, lane, chosen + (size_t)t * r.top, weight + (size_t)t * r.top);
+    if (SCORED) choose_scored(sc, ch, gs, r, lane, chosen + (size_t)t * r.top, weight + (size_t)t * r.top);
     else choose_softmax(sc, r, lane, chosen + (size_t)t * r.top, weight + (size_t)t * r.top);
 }
 
@@ -246,7 +248,7 @@ __device__ __forceinline__ void three_parts(const float4& a, const float4& b, un
 }
 
 __global__ void __launch_bounds__(TILE_WARPS * 32, 2)
-route_tile_kernel(const __nv_bfloat16* __restrict__ x, Routing r, int n_tokens, int hidden, int* __restrict__ chosen, float* __restrict__ weight,
+route_tile_kernel(const __nv_bfloat16* __restrict__ x, const __grid_constant__ Routing r, int n_tokens, int hidden, int* __restrict__ chosen, float* __restrict__ weight,
                   float* __restrict__ shared_gate) {
     extern __shared__ __align__(16) float sm[];            // [TILE_WARPS][TILE tokens][columns] partial logits, then per token n_out scores, n_out choice scores, groups
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3, t0 = blockIdx.x * TILE;
@@ -322,10 +324,12 @@ int launch_route(const void* x, const float* norm_w, float eps, const Routing& r
                  cudaStream_t stream) {
     const size_t smem = (size_t)(r.scored ? hidden + 2 * r.n_out + r.group_count : hidden + r.n_out) * sizeof(float);
     if (smem > 48 * 1024) return VM_ERR_UNSUPPORTED;
-    // sixteen tokens a block once a block per token would be more than one per SM (2,048 tokens: 12.5 us against 25; one wave of blocks of a token
-    // each takes 6 to 9 us)
+    // Sixteen tokens a block once a block per token would be more than the six that an SM holds, or more than three where the weights are 256 KB and more
+    // (1,024 x 16: 800 tokens 8.2 us a block per token, 8.6 in tiles, 1,184 tokens 15 and 8.6; 1,024 x 64: 296 tokens 11 and 14.5, 512 tokens 15.5 and 14.5;
+    // 2,048 x 64: 296 tokens 20 and 22, 400 tokens 30 and 22)
     const int outputs = r.n_out + (r.gate ? 1 : 0);
-    if (sizeof(T) == 2 && !norm_w && n > vm_sm_count() && hidden % 32 == 0 && outputs <= 8 * MAX_TILES && r.group_count <= r.n_out && aligned16(x) && aligned16(r.w) &&
+    const bool many = n > ((long long)outputs * hidden >= 65536 ? 3 : 6) * vm_sm_count();
+    if (sizeof(T) == 2 && !norm_w && many && hidden % 32 == 0 && outputs <= 8 * MAX_TILES && r.group_count <= r.n_out && aligned16(x) && aligned16(r.w) &&
         aligned16(r.gate)) {
         const size_t tile = ((size_t)TILE_WARPS * TILE * ((outputs + 7) / 8 * 8 + 2) + (size_t)TILE * (2 * r.n_out + r.group_count)) * sizeof(float);
         static const cudaError_t raised = cudaFuncSetAttribute(route_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
@@ -333,8 +337,18 @@ int launch_route(const void* x, const float* norm_w, float eps, const Routing& r
         vm_launch_pdl(route_tile_kernel, dim3((n + TILE - 1) / TILE), dim3(TILE_WARPS * 32), tile, stream, (const __nv_bfloat16*)x, r, n, hidden, chosen, weight, shared_gate);
         return vm_launch_status();
     }
-    const int threads = n <= vm_sm_count() && r.n_out > 8 ? 1024 : 256;      // few tokens: a warp for each output or two (the block's latency is the step's)
-    vm_launch_pdl(route_kernel<T>, dim3(n), dim3(threads), smem, stream, x, norm_w, eps, r, hidden, chosen, weight, shared_gate, (T*)rows_out);
+    const int per_sm = n <= vm_sm_count() ? 1 : n <= 4 * vm_sm_count() ? 4 : 6;
+    const int threads = per_sm == 1 && r.n_out > 8 ? 1024 : 256;      // few tokens: a warp for each output or two (the block's latency is the step's)
+#define VM_ROUTE(P, S)                                                                                                                               \
+    if (per_sm == P && (r.scored != 0) == S)                                                                                                         \
+        vm_launch_pdl(route_kernel<T, P, S>, dim3(n), dim3(threads), smem, stream, x, norm_w, eps, r, hidden, chosen, weight, shared_gate, (T*)rows_out)
+    VM_ROUTE(1, true);
+    VM_ROUTE(1, false);
+    VM_ROUTE(4, true);
+    VM_ROUTE(4, false);
+    VM_ROUTE(6, true);
+    VM_ROUTE(6, false);
+#undef VM_ROUTE
     return vm_launch_status();
 }
 
