@@ -202,7 +202,7 @@ static int launch_heads(const float* proj, int ld, const float* bias, float eps,
 
 // The preparation with a convolution, rotary positions or a norm over the whole projection: a warp takes the heads `item`, item + gridDim.y * 8, .. of one token, so
 // that a token's rotation is worked out once per warp; two neighbouring values per lane and turn, a head's row passes through the warp's own shared memory
-// only to meet its rotary partners.  Few tokens: a warp per head, many blocks per token; with the norm one block
+// only to meet its rotary partners.  Few tokens: a warp per head, many blocks per token; with the norm (steps whose blocks the GPU holds at once) one block
 // per token and a warp per head, whose sums of squares meet once.  (With a block per token and passes over the row in shared
 // memory, a decode step of 4 tokens of 24 heads and three taps took 13 us, 2,300 prompt tokens 27 us: a chain of passes, most of the GPU idle.
 // Now 5.6 and 18 us.)
@@ -427,8 +427,12 @@ VM_API int vm_mixer_prepare(const float* proj, int ld, const float* bias, const 
     const int threads = C >= 2048 ? 512 : 256;
     const int keep_here = (one_token_each && K > 1) ? 1 : 0;
     cudaError_t e = cudaSuccess;
-    // heads that depend on nothing but themselves, or one norm a block can hold (and the pages are the row's own, or there are none): warps take them apart
-    const bool apart = (!q_norm || H + G <= 32) && (G == 0 || (kpages && vpages)) && Dk % 2 == 0 && Dv % 2 == 0 && ld % 2 == 0 && Dk <= 256 && Dv <= 256 &&
+    // Heads that depend on nothing but themselves, or one norm a block can hold (and the pages are the row's own, or there are none): warps take them apart.
+    // With the norm a block's warps wait for each other, and blocks of more than eight of them pay as long as the GPU holds them all at once (heads of 64, no
+    // convolution: 16 + 4 heads, 250 tokens 6.6 -> 6.0 us, 300 tokens 6.8 -> 8.2, 2,300 tokens 20 -> 40; 3 + 1 heads, 2,300 tokens 10.9 -> 8.0)
+    const int warps = H + 2 * G < 32 ? H + 2 * G : 32;
+    const bool normed_apart = H + G <= 32 && (warps <= 8 || (long long)T * warps <= 40ll * vm_sm_count());
+    const bool apart = (!q_norm || normed_apart) && (G == 0 || (kpages && vpages)) && Dk % 2 == 0 && Dv % 2 == 0 && ld % 2 == 0 && Dk <= 256 && Dv <= 256 &&
                        ((uintptr_t)proj | (uintptr_t)bias) % 8 == 0 && ((uintptr_t)q_out | (uintptr_t)kpages | (uintptr_t)vpages) % 8 == 0;
     if (apart && act_dtype == VM_F32) {
         const int st = launch_turned_heads<float>(proj, ld, bias, taps, K, state, state_stride, state_offset, q_norm, k_norm, eps, inv_freq, rotary_dim, pairing,
