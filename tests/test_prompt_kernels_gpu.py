@@ -1,5 +1,5 @@
 """Kernels of a prompt's mixers at the places where their launches change form: the preparation with a norm over the whole projection
-(csrc/mixer_prep.cu)."""
+(csrc/mixer_prep.cu), the delta rule's chunks with one or two stages (csrc/delta_rule.cu)."""
 import ctypes
 
 import pytest
@@ -85,3 +85,38 @@ def test_the_normed_preparation(T, K, H, G, D):
         assert float((rows(vp) - y[:, (H + G) * D:].reshape(T, G, D)).abs().max()) <= 2e-5
     if K > 1:
         assert torch.equal(state.reshape(K - 1, C), x[T - K + 1:])
+
+
+@pytest.mark.parametrize("new,H,G,Dk,Dv", [([130, 65, 1, 64], 40, 20, 64, 64), ([200, 30], 10, 10, 128, 128), ([70, 129], 12, 6, 128, 100), ([300], 2, 1, 80, 48), ([64, 3, 90], 30, 15, 80, 32),
+                                           ([100, 140], 13, 13, 96, 96)])
+def test_delta_rule_in_chunks(new, H, G, Dk, Dv):
+    """Blocks of one stage side by side (more blocks than SMs, keys of 96 and 128), two blocks of two stages an SM (64 and 80), and one wave: against the
+    recurrence in 64 bits."""
+    g = torch.Generator().manual_seed(Dk + H)
+    T, B, C = sum(new), len(new), 2 * G * Dk + H * Dv
+    rows = torch.randn(T, C, generator=g)
+    for a in (0, G * Dk):
+        rows[:, a:a + G * Dk] = torch.nn.functional.normalize(rows[:, a:a + G * Dk].reshape(T, G, Dk), dim=-1).reshape(T, G * Dk)
+    gates = torch.cat([torch.rand(T, H, generator=g), -torch.rand(T, H, generator=g) * 0.2], 1)
+    start = torch.randn(B, H, Dk, Dv, generator=g) * 0.3
+    state = start.reshape(B, -1).clone().to(DEV)
+    chunks = sum(-(-n // 64) for n in new)
+    scratch = torch.full((_lib().vm_delta_scratch_floats(_i(chunks), _i(H), _i(Dk), _i(Dv)),), float("nan"), device=DEV)
+    o = torch.full((T, H * Dv), float("nan"), device=DEV)
+    d_rows, d_gates, cu, slots = rows.to(DEV), gates.contiguous().to(DEV), _cu(new), _ints(list(range(B)))
+    assert _lib().vm_delta_chunks(_p(d_rows), _p(d_gates), _p(state), _l(H * Dk * Dv), _i(0), _p(cu), _p(slots), _p(o), _p(scratch), _i(chunks), _i(T), _i(B), _i(H),
+                                  _i(G), _i(Dk), _i(Dv), _stream()) == 0
+    z = d_rows.double()
+    q, k = (z[:, a:a + G * Dk].reshape(T, G, Dk).repeat_interleave(H // G, 1) for a in (0, G * Dk))
+    v, beta, keep = z[:, 2 * G * Dk:].reshape(T, H, Dv), d_gates[:, :H].double(), torch.exp(d_gates[:, H:].double())
+    S, t = start.to(DEV).double(), 0
+    for b, n in enumerate(new):
+        for t in range(t, t + n):
+            s = S[b] * keep[t][:, None, None]
+            u = beta[t][:, None] * (v[t] - torch.einsum("hkv,hk->hv", s, k[t]))
+            S[b] = s + k[t][:, :, None] * u[:, None]
+            want = torch.einsum("hkv,hk->hv", S[b], q[t])
+            if t % 37 == 0 or t + 1 == sum(new[:b + 1]):
+                assert float((o[t].reshape(H, Dv).double() - want).abs().max()) <= 2e-5, t
+        t += 1
+    assert float((state.reshape(S.shape).double() - S).abs().max()) <= 2e-5

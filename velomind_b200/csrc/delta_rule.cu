@@ -880,8 +880,9 @@ VM_API int vm_delta_chunks(const float* rows, const float* gates, float* state, 
     if (!vm_delta_chunk_tokens(Dk, Dv) || H > 65535) return VM_ERR_UNSUPPORTED;
     // Two stages hide a chunk's loads behind the one before; but where that gives more blocks than SMs, at one block an SM, blocks of one stage that
     // share an SM do (measured, two prompts of 1,400 and 2,000 tokens, 16 heads of 128 x 128, 256 blocks: 256 us in two waves, 202 us side by side).
+    // Keys of up to 80 leave two blocks of two stages an SM, and those stay ahead (64 x 64, 320 blocks: the three launches 326 us, 345 us with one stage).
     const long long blocks = (long long)B * H * ((Dv + CCOLS - 1) / CCOLS);
-    const bool beside = blocks > vm_sm_count() && 2 * (carry_smem(Dk, 1) + 2048) <= SMEM_MAX;
+    const bool beside = blocks > vm_sm_count() && 2 * (carry_smem(Dk, 2) + 2048) > SMEM_MAX && 2 * (carry_smem(Dk, 1) + 2048) <= SMEM_MAX;
     const int stages = carry_smem(Dk, 2) <= SMEM_MAX && !beside ? 2 : 1;
     cudaError_t e = allow_smem(delta_local_kernel, local_smem(Dk));
     if (e == cudaSuccess) e = allow_smem(delta_finish_kernel, finish_smem(Dk));
