@@ -332,3 +332,25 @@ def test_long_prompt_takes_the_tcgen05_attention(model_folders):
     engine.raise_if_error()
     assert engine.counters["tc_attention_calls"] > 0
     _compare(got, S.expected_rows(steps, requests, plain), TOL["bfloat16"])
+
+
+def test_prompts_of_middling_length_take_it_where_there_are_many(model_folders):
+    """Twelve prompts of some 800 tokens fill the GPU with tiles that see ten key blocks and more: the tcgen05 attention.  As many tiles of short prompts
+    beside one of 1,000 do not take it.  Logits against the plain model."""
+    import velomind_b200 as vm
+    folder = model_folders["tiny_c"]
+    requests = S.make_requests(CONFIGS["tiny_c"]["vocab_size"], (800, 771, 1000), seed=29)
+    plain = S.plain_logits(folder, requests)
+    scale = max(1.0, max(float(np.abs(v).max()) for v in plain.values()))
+    engine = _engine(folder, "bfloat16", max_tokens=64 * 200, max_slots=96, max_step_tokens=16384)
+    for lengths, taken in ((["r0"] * 6 + ["r1"] * 6, 2), (["r2"] + [60] * 80, 0)):
+        parts = [("r0", requests["r0"][:n]) if isinstance(n, int) else (n, requests[n]) for n in lengths]
+        before = engine.counters["tc_attention_calls"]
+        slots = [engine.open() for _ in parts]
+        got = engine.step([vm.Entry(s, t, [0, len(t) // 2, len(t) - 1]) for s, (_, t) in zip(slots, parts)]).float().cpu().numpy().reshape(len(parts), 3, -1)
+        assert engine.counters["tc_attention_calls"] - before == taken            # (two layers)
+        for row, (rid, t) in zip(got, parts):
+            assert np.abs(row - plain[rid][[0, len(t) // 2, len(t) - 1]]).max() <= TOL["bfloat16"] * scale
+        for s in slots:
+            engine.close(s)
+    engine.raise_if_error()

@@ -434,7 +434,8 @@ constexpr int MAX_DECODE_SPLITS = 16;
 constexpr int DECODE_ONE_CTA_BLOCKS = 16;     // block tables up to this wide (1,024 tokens): at most two rounds of pages for ten warps
 constexpr int TC_ATTENTION_MIN_BLOCKS = 20;   // head size 64: the tcgen05 prefill attention when a tile may see this many key blocks
 constexpr int TC_ATTENTION_CTAS_PER_SM = 3;   // CTAs of that kernel an SM holds at once (registers and shared memory)
-constexpr int WS_ATTENTION_MANY_BLOCKS = 16;  // the same for steps of many tiles
+constexpr int WS_ATTENTION_MANY_BLOCKS = 16;  // the same for steps of many long tiles
+constexpr int WS_ATTENTION_MEAN_BLOCKS = 10;  // ... that see this many key blocks of new tokens on average
 int WS_ATTENTION_MIN_BLOCKS = 32;             // head size 64: the warp-specialised tcgen05 attention when a tile may see this many key blocks
 
 int* decode_counters() {
@@ -493,15 +494,17 @@ void attention(StepContext& ctx, const void* q, int q_row_stride, const KVView& 
         // from its lengths: a recorded step keeps its choice.  The table width bounds the key blocks a tile may walk.
         int most_blocks = kv.table_width;
         if (window > 0) most_blocks = std::min(most_blocks, window / VM_PAGE_TOKENS + 2);
-        long long tiles128 = 0, tiles64 = 0;
+        long long tiles128 = 0, tiles64 = 0, blocks128 = 0;      // blocks128: over the tiles of 128, the key blocks of their sequence's new tokens
         for (int b = 0; b < ctx.B; ++b) {
             const int n = ctx.host_cu_tokens[b + 1] - ctx.host_cu_tokens[b];
             tiles128 += (n + 127) / 128;
             tiles64 += (n + 63) / 64;
+            blocks128 += static_cast<long long>((n + 127) / 128) * std::min(most_blocks, (n + 63) / 64);
         }
-        // (many tiles of middling length keep that kernel's CTAs busy too: eight prompts of 576 to 1,024 tokens and 15 heads 44 us against 61 us for the
-        //  mma.sync kernel, four of 1,024 and 32 heads 75 / 90; one of 1,024 and 9 heads 22 / 17, eight of 512 33 / 22)
-        const bool many = most_blocks >= WS_ATTENTION_MANY_BLOCKS && tiles128 * H >= 3ll * sm_count();
+        // (many tiles of middling length keep that kernel's CTAs busy too: 15 heads, four prompts of 1,024 tokens 43 us against 51 us for the mma.sync kernel, eight of
+        //  800 59 / 60; 32 heads, three of 1,024 61 / 71; one of 1,024 and 9 heads 22 / 17, eight of 512 33 / 22.  Short prompts beside long ones do not, each
+        //  pays for a CTA's set-up: 15 heads, one of 1,024 beside sixteen of 100 42 / 31, eight of 800 beside 32 of 60 72 / 66)
+        const bool many = most_blocks >= WS_ATTENTION_MANY_BLOCKS && tiles128 * H >= 3ll * sm_count() && blocks128 >= WS_ATTENTION_MEAN_BLOCKS * tiles128;
         if (D == 64 && (most_blocks >= WS_ATTENTION_MIN_BLOCKS || many) && ctx.err != nullptr) {
             // the longest prompts: softmax warps, a copy warp and product warps, clusters dealt out to pairs of tile groups
             // (measured, 9 heads: 4,096 tokens 78 us against 88 us for the kernel below, 8,192: 224 / 262; 2,048: 32 / 33;
