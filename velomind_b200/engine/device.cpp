@@ -541,9 +541,10 @@ void attention(StepContext& ctx, const void* q, int q_row_stride, const KVView& 
                   "attention_prefill_bf16", s);
             return;
         }
-        // two groups of warps share a tile's keys where the tiles are long and too few to fill the GPU (measured, 9 heads of 64: one prompt of 2,048 tokens
-        // 40.0 us with two groups, 43.8 us with one, of 1,024 tokens 17.3 / 20.2; of 300 tokens 8.2 / 7.9, sixteen of 40 to 295 16.4 / 12.2, eight of 512 25.1 / 22.2)
-        const int groups = most_blocks >= 16 && tiles64 * H <= 2ll * sm_count() ? 2 : 1;
+        // two groups of warps share a tile's keys where the tiles are long and too few to fill the GPU: two an SM where tiles may see 1,024 keys and more, one an SM
+        // above 512 (measured, with two groups / with one: 9 heads of 64, one prompt of 2,048 tokens 40.0 / 43.8 us, of 1,000 16.4 / 19.5, of 512 10.1 / 11.3, of 300
+        // 7.6 / 7.8, two of 700 18.0 / 17.6, sixteen of 40 to 295 16.4 / 12.2, eight of 512 25.1 / 22.2; 16 heads of 128, one of 512 15.2 / 18.3, of 700 26 / 29)
+        const int groups = most_blocks >= 8 && tiles64 * H <= (most_blocks >= 16 ? 2ll : 1ll) * sm_count() ? 2 : 1;
         Timed t("attention_prefill_bf16", s);
         check(vm_attention_prefill_bf16(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, ctx.cu_tokens, ctx.B,
                                         static_cast<int>(tiles64), out, H, Hkv, D, scale, window, kv.n_pages, ctx.err, groups, s),
