@@ -163,8 +163,11 @@ public:
         int* chosen = static_cast<int*>(ctx.take_tokens(top_, DType::I32));
         float* weight = static_cast<float*>(ctx.take_tokens(top_, DType::F32));
         float* sgate = gate_ ? static_cast<float*>(ctx.take_tokens(1, DType::F32)) : nullptr;
-        // in bfloat16 each expert's weights once for all its tokens, from rows that the router has normed; else token by token
-        const bool tile = ctx.act_dtype == DType::BF16 && up_.dtype == DType::BF16 && vm_experts_few_tile_fits(ctx.T_cap, hidden_, ff_, sff_, top_, E_, r_.identity);
+        // In bfloat16 each expert's weights once for all its tokens, from rows that the router has normed; else token by token, as for more than a few tokens of
+        // experts so small that reading them again costs less than a tile's chain (64 x 32, 64 tokens: 8.8 us token by token, 12.4 in tiles; 128 x 64, 128 tokens
+        // with a shared expert 14.5 / 20.2; 256 x 128 15.0 / 13.4)
+        const bool tile = ctx.act_dtype == DType::BF16 && up_.dtype == DType::BF16 && (ctx.T_cap <= 16 || static_cast<long long>(hidden_) * ff_ >= 256 * 128) &&
+                          vm_experts_few_tile_fits(ctx.T_cap, hidden_, ff_, sff_, top_, E_, r_.identity);
         void* normed = tile && nw ? ctx.take_tokens(hidden_, ctx.act_dtype) : nullptr;
         route(ctx, x, nw, eps, chosen, weight, sgate, normed);
         void* act = ctx.take_tokens(vm_experts_act_cols(hidden_, ff_, sff_, top_, r_.identity), ctx.act_dtype);
