@@ -206,7 +206,7 @@ def _run_attention(kind, dtype, H, Hkv, D, lens_before, new, window, seed=0, gro
                                     window, err, groups)
     else:
         B = len(new)
-        n_splits = o.decode_splits(B, Hkv, H // Hkv, table.shape[1])
+        n_splits = o.decode_splits(B, Hkv, H // Hkv, D, table.shape[1])
         for splits in sorted({1, n_splits, min(3, table.shape[1])}):
             partial = torch.full((B * H * splits * (D + 2),), float("nan"), device=DEV)
             counters = torch.zeros(B * H, dtype=torch.int32, device=DEV)

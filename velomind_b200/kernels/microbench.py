@@ -158,7 +158,7 @@ def main(argv=None) -> int:
         bytes_read = ws[0].numel() * 2
     elif a.kernel == "attn_decode":
         q = torch.randn(M, H * D, device=dev).to(bf)
-        splits = a.splits or ops.decode_splits(M, Hkv, H // Hkv, width)
+        splits = a.splits or ops.decode_splits(M, Hkv, H // Hkv, D, width)
         partial = torch.empty(M * H * ops.MAX_DECODE_SPLITS * (D + 2), device=dev)
         out = torch.empty(M, H * D, device=dev, dtype=bf)
         fn = lambda: ops.attention_decode_bf16(q, H * D, kp, vp, table, pos, out, partial, ops.decode_counters(dev), H, Hkv, D,

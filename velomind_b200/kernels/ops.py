@@ -223,7 +223,7 @@ def decode_counters(device) -> torch.Tensor:
 DECODE_ONE_CTA_BLOCKS = 16     # block tables up to this wide (1,024 tokens): at most two rounds of pages for ten warps
 
 
-def decode_splits(B: int, Hkv: int, G: int, table_width: int, device=None, D: int = 64) -> int:
+def decode_splits(B: int, Hkv: int, G: int, D: int, table_width: int, device=None) -> int:
     """How many CTAs share the keys of one (sequence, kv head): enough to fill the GPU, a function of the
     step's SHAPE only (so that a captured launch stays valid as sequences grow)."""
     groups = B * Hkv * (-(-G // 16))          # a CTA serves up to 16 query heads of one kv head
