@@ -372,7 +372,8 @@ void linear(const void* x, DType x_dtype, long long ldx, const DeviceTensor& W, 
     if (!(out_dtype == x_dtype || out_dtype == DType::F32)) throw KernelError("linear: the result has the input's dtype or float32");
     Timed t("linear", s);
     if (x_dtype == DType::F32 && vm_skinny_f32_fits(x, ldx, W.ptr, T, static_cast<int>(W.cols()))) {
-        // a few rows in float32: this library's own kernel (measured, 4 rows: 2.7 to 5.5 us where the matrix-product library takes 9.4 to 14 us)
+        // a few rows in float32: this library's own kernel (measured against the matrix-product library, 4 rows: 576 x 576 1.9 / 5.0 us, 2,048 x 8,192
+        // 19 / 63, 49,152 x 2,048 76 / 118; 8 rows: 2.3 / 8.0, 27 / 65, 102 / 125; no size from 64 x 64 on was slower)
         check(vm_skinny_f32(static_cast<const float*>(x), ldx, static_cast<const float*>(W.ptr), static_cast<float*>(out), T, static_cast<int>(W.rows()),
                             static_cast<int>(W.cols()), s),
               "linear", s);
@@ -453,8 +454,9 @@ int decode_splits(int B, int Hkv, int G, int D, int table_width) {
     const int groups = B * Hkv * ((G + 15) / 16);           // a CTA serves up to 16 query heads of one kv head
     const int sms = sm_count();
     if (groups <= sms && table_width <= DECODE_ONE_CTA_BLOCKS) return 1;   // short sequences: one CTA of ten warps holds all pages
-    // More than half the SMs have a CTA of their own: ten warps (whose pages fit shared memory up to heads of 64) walk the pages, and nothing is joined across CTAs (measured, 80 groups of 3 heads of
-    // 64: 1,100 tokens 7.2 us against 11.2 us in two splits of four warps, 2,000 tokens 11.6 / 14.8; 128 groups, 2,000 tokens 12.3 / 14.1).
+    // More than half the SMs have a CTA of their own: ten warps (whose pages fit shared memory up to heads of 64) walk the pages, and nothing is joined across CTAs
+    // (measured, 80 groups of 3 heads of 64: 1,100 tokens 7.4 us against 11.3 us in two splits of four warps, 2,000 tokens 11.9 / 14.9, 8,000 39 / 44, 16,000
+    // 73 / 80; 128 groups, 2,000 tokens 12.3 / 14.1, 16,000 85 / 88).
     if (D <= 64 && groups <= sms && 2 * groups > sms) return 1;
     // Else about one CTA per SM, in powers of two (24 groups, 2,000 tokens: 8 splits 7.2 us, 7 splits 8.4 us; 64 groups: 4 splits 9.0 us, 3 splits
     // 10.7 us) ...
