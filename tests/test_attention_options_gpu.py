@@ -217,16 +217,17 @@ def test_biases_at_the_ends_of_the_type(name, dtype):
         assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all())
 
 
-def test_a_missing_page_is_reported():
-    s = Step(4, 1, 64, 64, [200], [1], torch.bfloat16)
-    s.table[0, 1] = -1
-    with pytest.raises(AssertionError):
-        s.run("tile", 0, 0, 0, False, False, False, 0.125)
+@pytest.mark.parametrize("name,dtype,page", [("tile", torch.bfloat16, -1), ("rows", torch.bfloat16, -1), ("rows", torch.float32, 4096), ("prompt", torch.bfloat16, -1)])
+def test_a_missing_page_is_reported(name, dtype, page):
+    """A page that is not there, or outside the pool: the launch is accepted, and the error word says that a page was missing."""
+    s = Step(4, 1, 64, 64, [200], [1], dtype)
+    s.table[0, 1] = page
+    assert s.call(name, 0, 0, 0, False, False, False, 0.125)[1:] == (0, 3)
 
 
 @pytest.mark.parametrize("H,Hkv,Dk,Dv,in_keys", [(4, 2, 64, 64, False), (80, 20, 64, 64, False), (3, 1, 96, 64, True), (2, 1, 160, 128, True), (70, 1, 128, 128, True), (2, 2, 64, 128, False),
                                                  (4, 4, 32, 16, False)])
-@pytest.mark.parametrize("options", OPTIONS[1:] + [(0, 0, 0, True, False, True)])
+@pytest.mark.parametrize("options", OPTIONS + [(0, 0, 0, True, False, True)])
 def test_prompt(H, Hkv, Dk, Dv, in_keys, options):
     """Prompts around the edges of the 64-row tiles and of the masks: blocks that every row of a warp sees whole and blocks that it does not.  Probabilities are rounded to
     bfloat16 (2^-9 each of values around 1) and so is the result."""

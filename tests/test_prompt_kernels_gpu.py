@@ -1,5 +1,6 @@
 """Kernels of a prompt's mixers at the places where their launches change form: the preparation with a norm over the whole projection
-(csrc/mixer_prep.cu), the delta rule's chunks with one or two stages (csrc/delta_rule.cu)."""
+(csrc/mixer_prep.cu), the delta rule's chunks with one or two stages (csrc/delta_rule.cu), the matrix memory's chunks with and without 16-byte loads
+(csrc/mlstm.cu)."""
 import ctypes
 
 import pytest
@@ -120,3 +121,39 @@ def test_delta_rule_in_chunks(new, H, G, Dk, Dv):
                 assert float((o[t].reshape(H, Dv).double() - want).abs().max()) <= 2e-5, t
         t += 1
     assert float((state.reshape(S.shape).double() - S).abs().max()) <= 2e-5
+
+
+@pytest.mark.parametrize("new,H,D,V", [([64, 1, 63, 100], 4, 128, 256), ([129], 2, 64, 128), ([130, 7], 2, 32, 64), ([200], 3, 20, 36), ([65, 65], 1, 48, 40), ([127], 8, 24, 100)])
+def test_matrix_memory_in_chunks_however_its_rows_lie(new, H, D, V):
+    """With 16-byte loads where the rows allow them and without (the same rows one value further on): the same bits; and what the memory read and
+    written token by token gives, up to sums in another order."""
+    g = torch.Generator().manual_seed(D + V)
+    T, B = sum(new), len(new)
+    ld = 2 * H * D + 2 * H * V + 2 * H
+    ld += -ld % 4
+    proj = torch.randn(T, ld, generator=g)
+    bi, bf = torch.randn(H, generator=g).to(DEV), (torch.randn(H, generator=g) + 3).to(DEV)
+    nw = torch.rand(H * V, generator=g).to(DEV) + 0.5
+    words = H * (D * V + D + 1)
+    slots, cu = _ints(list(range(B))), _cu(new)
+    got = []
+    for kind in ("aligned", "one on", "token by token"):
+        pool = torch.full((T * ld + 4,), float("nan"), device=DEV)
+        rows = pool[1:1 + T * ld] if kind == "one on" else pool[:T * ld]
+        rows.copy_(proj.reshape(-1))
+        state = torch.zeros(B, words, device=DEV)
+        out = torch.full((T, H * V), float("nan"), device=DEV)
+        head = (_p(rows), _i(ld), _p(bi), _p(bf), _p(nw), _p(state), _p(cu), _p(slots), _p(out))
+        sizes = (_i(B), _i(H), _i(D), _i(V), _f(15.0), _f(1e-6), _i(0), _stream())
+        if kind == "token by token":
+            if not _lib().vm_mlstm_scan_fits(_i(D), _i(V)):
+                continue
+            assert _lib().vm_mlstm_scan(*head, *sizes) == 0
+        else:
+            scratch = torch.full((_lib().vm_mlstm_chunk_scratch_floats(_i(T), _i(B), _i(H), _i(D), _i(V)),), float("nan"), device=DEV)
+            assert _lib().vm_mlstm_chunks(*head, _p(scratch), _i(T), *sizes) == 0
+        got.append((out, state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    # (sums of up to 228 tokens and 128 channels in another order, 2^-24 each of their largest term, through a norm over the head: a few hundred of them)
+    for out, _ in got[2:]:
+        assert float((out - got[0][0]).abs().max()) <= 5e-5 * float(out.abs().max())
