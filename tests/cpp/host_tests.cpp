@@ -10,6 +10,7 @@
 #include <set>
 
 #include "velomind_b200/kernels.h"
+#include "velomind_b200/once_per_device.h"
 #include "velomind_b200/velomind.h"
 
 using namespace vmb;
@@ -516,6 +517,18 @@ TEST(parts_and_architectures_are_looked_up_by_name) {
     THROWS(ConfigError, "does not come before", plan.validate());
     const WeightTable table = weight_table(llama_plan(LlamaConfig::from_json(json::parse(SMOLLM2_135M_CONFIG, "built-in"))));
     CHECK(table.size() == 30 * 9 + 3 && table.at("lm_head.weight").alias_of == "model.embed_tokens.weight");
+}
+
+// ------------------------------------------------------------------------------------------------ once per device
+TEST(something_is_done_once_on_each_device) {
+    VmOncePerDevice once;
+    int runs[3] = {0, 0, 0};
+    const auto on = [&](int device, int status) { return once(device, [&] { ++runs[device % 3]; return status; }); };
+    CHECK(on(0, 0) == 0 && on(0, 0) == 0 && runs[0] == 1);
+    CHECK(on(1, 0) == 0 && runs[1] == 1);             // another device: again
+    CHECK(on(2, 700) == 700 && on(2, 0) == 0 && on(2, 0) == 0 && runs[2] == 2);      // after a failure: again
+    CHECK(on(0, 0) == 0 && on(1, 0) == 0 && runs[0] == 1 && runs[1] == 1);
+    CHECK(on(64, 0) == 0 && on(64, 0) == 0 && runs[1] == 3);      // (64 % 3 = 1)
 }
 
 }  // namespace

@@ -36,7 +36,7 @@ CASES = ["free_list_never_loses_or_doubles", "slots_and_pages_come_back", "group
          "arena_plan_packs_by_liveness", "loop_unequal_prompts_stop_tokens_and_early_ends", "loop_runs_batch_after_batch_and_reuses_slots",
          "batches_are_cut_by_pages_and_slots", "loop_closes_slots_when_a_step_fails", "loop_with_queued_decode_runs_gives_the_same_tokens",
          "pretokenizer_pieces", "bpe_round_trip_and_special_ids", "streamer_emits_deltas_and_waits_for_whole_characters",
-         "json_reads_and_writes", "parts_and_architectures_are_looked_up_by_name"]
+         "json_reads_and_writes", "parts_and_architectures_are_looked_up_by_name", "something_is_done_once_on_each_device"]
 
 
 def test_every_case_is_listed(host_tests):

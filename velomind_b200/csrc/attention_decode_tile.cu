@@ -320,9 +320,9 @@ int launch_tile(const void* q, int q_row_stride, const void* kpages, const void*
     int splits = 1;
     while (splits < MAX_SPLITS && 2 * splits * tiles <= (splits == 4 ? 64 : vm_sm_count()) && (long long)splits * WARPS * KEYS < keys) splits *= 2;
     const size_t smem = ((size_t)WARPS * ROWS * row_floats<DV>() + (splits > 1 ? ROWS * DV + splits : 0)) * sizeof(float);
-    static const cudaError_t raised = cudaFuncSetAttribute(attn_decode_tile_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                           (int)((WARPS * ROWS * row_floats<DV>() + ROWS * DV + MAX_SPLITS) * sizeof(float)));
-    if (raised != cudaSuccess) return (int)raised;
+    static VmOncePerDevice once;
+    const cudaError_t allowed = vm_allow_smem(once, attn_decode_tile_kernel<DK, DV>, (WARPS * ROWS * row_floats<DV>() + ROWS * DV + MAX_SPLITS) * sizeof(float));
+    if (allowed != cudaSuccess) return (int)allowed;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(splits, groups, B);
     cfg.blockDim = dim3(WARPS * 32);

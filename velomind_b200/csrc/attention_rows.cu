@@ -290,8 +290,9 @@ int launch_rows(const void* q, int q_row_stride, const void* kpages, const void*
                 int* err, cudaStream_t stream) {
     const size_t keys = (size_t)WARPS * KEYS * pitch<T>() * sizeof(T), sums = (size_t)WARPS * R * (Dv + 2) * sizeof(float);
     const size_t smem = ((size_t)R * Dk + (size_t)WARPS * R * 32) * sizeof(float) + (keys > sums ? keys : sums);
-    static const cudaError_t raised = cudaFuncSetAttribute(attn_rows_kernel<T, R, VP, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-    if (raised != cudaSuccess) return (int)raised;
+    static VmOncePerDevice once;
+    const cudaError_t e = vm_allow_smem(once, attn_rows_kernel<T, R, VP, WARPS>, 100 * 1024);
+    if (e != cudaSuccess) return (int)e;
     const int G = H / Hkv;
     const dim3 grid((n_tokens + tile_tokens - 1) / tile_tokens, Hkv * ((G + R - 1) / R));
     attn_rows_kernel<T, R, VP, WARPS><<<grid, WARPS * 32, smem, stream>>>((const T*)q, q_row_stride, (const T*)kpages, (const T*)vpages, block_table, max_blocks,

@@ -7,6 +7,7 @@
 // The launchers' declarations, dtype and status codes, the page size and the rotary pairings: one header shared
 // with the host library, so that a launcher's definition here is checked against what its callers see.
 #include "../include/velomind_b200/kernels.h"
+#include "../include/velomind_b200/once_per_device.h"
 
 #define VM_API extern "C" __attribute__((visibility("default")))
 
@@ -86,6 +87,15 @@ static inline int vm_sm_count() {
         if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) cached[dev] = n;
     }
     return cached[dev];
+}
+
+// `kernel` may use up to `bytes` of dynamic shared memory on the current device (`once`: the call site's own static)
+template <typename... KArgs>
+static inline cudaError_t vm_allow_smem(VmOncePerDevice& once, void (*kernel)(KArgs...), size_t bytes) {
+    int dev = -1;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return static_cast<cudaError_t>(once(dev, [&] { return static_cast<int>(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes))); }));
 }
 
 static inline int vm_launch_status() {

@@ -332,8 +332,9 @@ int launch_route(const void* x, const float* norm_w, float eps, const Routing& r
     if (sizeof(T) == 2 && !norm_w && many && hidden % 32 == 0 && outputs <= 8 * MAX_TILES && r.group_count <= r.n_out && aligned16(x) && aligned16(r.w) &&
         aligned16(r.gate)) {
         const size_t tile = ((size_t)TILE_WARPS * TILE * ((outputs + 7) / 8 * 8 + 2) + (size_t)TILE * (2 * r.n_out + r.group_count)) * sizeof(float);
-        static const cudaError_t raised = cudaFuncSetAttribute(route_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-        if (raised != cudaSuccess) return (int)raised;
+        static VmOncePerDevice once;
+        const cudaError_t e = vm_allow_smem(once, route_tile_kernel, 100 * 1024);
+        if (e != cudaSuccess) return (int)e;
         vm_launch_pdl(route_tile_kernel, dim3((n + TILE - 1) / TILE), dim3(TILE_WARPS * 32), tile, stream, (const __nv_bfloat16*)x, r, n, hidden, chosen, weight, shared_gate);
         return vm_launch_status();
     }

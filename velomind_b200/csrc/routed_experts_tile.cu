@@ -322,10 +322,10 @@ VM_API int vm_experts_few_tile(const void* x, const void* w_up, const void* w_do
                         (int)vm_experts_act_cols(hidden, ff, ff_shared, top, n_identity), limit, alpha};
     const int nt = down_tiles(hidden);
     const size_t smem = down_smem(ff, ff_shared, top, E, nt);
-    static const cudaError_t r0 = cudaFuncSetAttribute(experts_up_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_PAIRS * (int)sizeof(int));
-    static const cudaError_t r1 = cudaFuncSetAttribute(experts_down_tile_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    static const cudaError_t r2 = cudaFuncSetAttribute(experts_down_tile_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (r0 != cudaSuccess || r1 != cudaSuccess || r2 != cudaSuccess) return (int)(r0 != cudaSuccess ? r0 : r1 != cudaSuccess ? r1 : r2);
+    static VmOncePerDevice once[3];
+    cudaError_t e = vm_allow_smem(once[0], experts_up_tile_kernel, MAX_PAIRS * sizeof(int));
+    if (e == cudaSuccess) e = nt == 2 ? vm_allow_smem(once[2], experts_down_tile_kernel<2>, 200 * 1024) : vm_allow_smem(once[1], experts_down_tile_kernel<1>, 200 * 1024);
+    if (e != cudaSuccess) return (int)e;
     vm_launch_pdl(experts_up_tile_kernel, dim3(E * (ff / UP_ROWS) + ff_shared / UP_ROWS), dim3(UP_WARPS * 32), (size_t)T * top * sizeof(int), stream,
                   (const __nv_bfloat16*)x, (const __nv_bfloat16*)w_up, (const __nv_bfloat16*)w_up_shared, chosen, weight, z, T * top >= E ? 1 : 0,
                   (__nv_bfloat16*)act);
