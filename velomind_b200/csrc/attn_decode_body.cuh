@@ -27,10 +27,10 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
     __nv_bfloat16* sKV = sQ + DEC_ROWS * DP;                                            // [warps][K,V][64][DP]
     float* res = reinterpret_cast<float*>(sKV + DEC_WARPS * 2 * BN * DP);               // [warps][16][RW]
     if (PDL) vm_pdl_launch_dependents();
-    // Before the wait this kernel reads what OLDER steps and kernels wrote: positions, the block table and the cache
-    // rows of earlier tokens.  That is sound because the kernel launched directly before it (the one that writes the
-    // new token's row) lets its dependents start only after its own wait, when everything older is complete.  The
-    // new row and the queries, which that kernel writes, are fetched after the wait.
+    // Before the wait this kernel reads what OLDER steps wrote: positions, the block table and the cache rows of earlier
+    // tokens.  That is sound because a step's first kernel lets its dependents start only after its own wait, when
+    // everything older than the step is complete (common.cuh).  The new row and the queries, which the step itself
+    // writes, are fetched after the wait.
     const int G = H / Hkv;
     const int groups_per_kv = (G + DEC_ROWS - 1) / DEC_ROWS;
     const int hk = group_y / groups_per_kv, gg = group_y - hk * groups_per_kv;

@@ -54,10 +54,10 @@ __device__ __forceinline__ int vm_first_seen(int pos, int window, int chunk) {
 // vm_pdl_launch_dependents() lets the successor start its own preamble.  Without the launch attribute both
 // are no-ops.
 // One kernel reads more than constants in its preamble: the decode attention fetches positions, the block table
-// and the cache rows of EARLIER tokens there.  The rule that makes this sound: the kernel launched directly
-// before it (the one that writes the new token's key and value) calls vm_pdl_launch_dependents() only AFTER its
-// own vm_pdl_wait(), so when the attention's preamble runs, everything older than that kernel is complete and
-// visible; what that kernel itself writes (the new row, the queries) is read after the attention's wait.
+// and the cache rows of EARLIER tokens there, all of them written before this step began.  The rule that makes this
+// sound: a step's FIRST kernel (the embedding) calls vm_pdl_launch_dependents() only AFTER its own vm_pdl_wait(), so no
+// later kernel of the step starts before everything older than the step is complete and visible; what the step itself
+// writes (the new rows, the queries) is read after the attention's wait.
 // Kernels launched without the attribute (and library kernels) never release their successor early.
 __device__ __forceinline__ void vm_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void vm_pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

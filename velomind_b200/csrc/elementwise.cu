@@ -13,8 +13,8 @@ VM_API void vm_set_pdl(int on) { vm_pdl_enabled = on ? 1 : 0; }
 template <typename W>
 __global__ void embed_gather_kernel(const W* __restrict__ table, const int* __restrict__ tokens,
                                     float* __restrict__ out, int T, int hid, int vocab, float scale, int* __restrict__ err) {
-    vm_pdl_launch_dependents();
     vm_pdl_wait();
+    vm_pdl_launch_dependents();                             // (a step's first kernel: common.cuh says why in this order)
     const int t = blockIdx.x;
     const int id = tokens[t];
     const bool ok = (id >= 0 && id < vocab);

@@ -213,8 +213,8 @@ __global__ void embed_pairs_kernel(const W* __restrict__ table, const W* __restr
                                    const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ cu_tokens,
                                    const int* __restrict__ slots, int* __restrict__ last, long long last_stride, int keep_here, float* __restrict__ out,
                                    int hid, int vocab, long long buckets, long long mul_prev, long long mul_cur, float scale, int* __restrict__ err) {
-    vm_pdl_launch_dependents();
     vm_pdl_wait();
+    vm_pdl_launch_dependents();                             // (a step's first kernel: common.cuh says why in this order)
     const int t = blockIdx.x;
     const int id = tokens[t], seq = seq_of_token[t];
     const bool ok = id >= 0 && id < vocab;

@@ -33,6 +33,10 @@ struct SkinnyParams {
     int kc;                      // k chunk staged in shared memory at a time (multiple of 32)
     int row_bytes;               // shared-memory row pitch of the A tile, == 64 mod 128
     int stages;                  // (skinny_stream_kernel) stages of its ring of weight rows
+    // (skinny_direct_kernel) rows that carry a norm's weight: A is x norm_w in bf16, squares [M, parts] the parts of the rows' sums of squares
+    const float* squares; int parts;
+    // ... and what its residual epilogue leaves for the next product: h next_w as bf16 [M, N] and the squares' parts [M, ready_parts]
+    const float* next_w; __nv_bfloat16* ready; float* ready_squares; int ready_parts;
 };
 
 // `item` is the work item (what item_index is for the stand-alone kernel); `smem` the CTA's dynamic shared memory.
@@ -52,6 +56,12 @@ __device__ __forceinline__ float skinny_unit(const SkinnyParams& p, float g, flo
     g = fminf(g, p.limit);
     return g * (1.0f / (1.0f + expf(-p.alpha * g))) * (fminf(fmaxf(u, -p.limit), p.limit) + 1.0f);
 }
+
+}  // namespace vmsk
+
+int vm_skinny_direct(const vmsk::SkinnyParams& p, int items, cudaStream_t stream);      // skinny_direct.cu: products whose rows lie ready
+
+namespace vmsk {
 
 struct SkinnyCols { int nA, nB, head; };
 __device__ __forceinline__ SkinnyCols skinny_cols(const SkinnyParams& p, int item_index) {

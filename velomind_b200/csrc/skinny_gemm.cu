@@ -21,7 +21,10 @@
 // it waits for its predecessor; the rope_kv form lets ITS successor, the decode attention, start only after that wait
 // (common.cuh says why).
 //
-// Products that read many megabytes of weights for at most 32 rows take skinny_stream_kernel (skinny_stream.cuh): the same
+// Rows that lie ready in bfloat16 (at most 32 of them) take skinny_direct_kernel (skinny_direct.cu) whatever the size; the kernels here are for the norm
+// as a prologue, for the vocabulary head and for more rows.
+//
+// Products with the norm that read many megabytes of weights for at most 32 rows take skinny_stream_kernel (skinny_stream.cuh): the same
 // work items and epilogues, the weights streamed through shared memory by a warp of their own.
 //
 // Sizes: K % 32 == 0, N % 8 == 0 (16 for the two-tile forms), head size % 16 == 0, I % 8 == 0; M <= 64.
@@ -140,6 +143,8 @@ constexpr long long STREAM_MIN_WEIGHT_BYTES = 9ll << 20;
 constexpr long long STREAM_MIN_WEIGHT_BYTES_TWO_ROWS = 9ll << 19;      // 4.5 MB: with one or two rows there is next to no prologue
 
 int skinny_dispatch(SkinnyParams p, int items, cudaStream_t stream) {
+    if (p.squares || p.next_w) return vm_skinny_direct(p, items, stream);
+    if (skinny_variant == 0 && p.pro == PRO_NONE && p.M <= 32) return vm_skinny_direct(p, items, stream);
     const long long weight_bytes = (long long)p.N * p.K * 2;
     if (skinny_variant >= 2 || (skinny_variant == 0 && p.M <= 32 && weight_bytes >= (p.M <= 2 ? STREAM_MIN_WEIGHT_BYTES_TWO_ROWS : STREAM_MIN_WEIGHT_BYTES))) {
         const int rc = skinny_stream_launch(p, items, stream, skinny_variant == 3 ? 2 : (skinny_variant == 4 ? 1 : 0));
@@ -155,16 +160,41 @@ int skinny_dispatch(SkinnyParams p, int items, cudaStream_t stream) {
 // pipelines per SM / of two CTAs per SM.  For tests and measurements.
 VM_API void vm_skinny_variant(int variant) { skinny_variant = variant; }
 
-// out = A W^T (pro 0) or rmsnorm(h) W^T (pro 1); out bf16 (out_f32 0) or float32 (1); or h += ... (residual 1).
+// pro of the entry points below: 0, A is bf16 [M, K]; 1, A is the float32 residual [M, K] and norm_w the norm's weight; 2, A is bf16 [M, K] with the
+// norm's weight in it (the `ready` rows of vm_skinny_residual_ready) and norm_w the parts of the rows' sums of squares, [M, vm_skinny_ready_parts(K)].
+static void skinny_rows(SkinnyParams& p, const void* A, int pro, const float* norm_w, float eps) {
+    p.A = A; p.eps = eps;
+    p.pro = pro == 1 ? PRO_RMSNORM : PRO_NONE;
+    if (pro == 2) { p.squares = norm_w; p.parts = vm_skinny_ready_parts(p.K); }
+    else p.norm_w = norm_w;
+}
+
+VM_API int vm_skinny_ready_parts(int N) { return ((N % 16 == 0 ? N / 16 : N / 8) + 3) / 4 * 4; }
+
+// h[M, N] += A W^T (A bf16 [M, K]), and the new rows left ready for the product behind the norm that follows: ready bf16 [M, N] = h next_w,
+// squares [M, vm_skinny_ready_parts(N)] float32 with a sum over each row that is the row's sum of squares.
+VM_API int vm_skinny_residual_ready(const void* A, const void* W, int M, int N, int K, float* h, const float* next_w, void* ready, float* squares,
+                                    cudaStream_t stream) {
+    if (N % 8 != 0 || !next_w) return VM_ERR_UNSUPPORTED;
+    SkinnyParams p{};
+    p.A = A; p.W = (const __nv_bfloat16*)W; p.M = M; p.N = N; p.K = K; p.h = h; p.epi = EPI_RESIDUAL;
+    p.next_w = next_w; p.ready = (__nv_bfloat16*)ready; p.ready_squares = squares; p.ready_parts = vm_skinny_ready_parts(N);
+    p.tiles = N % 16 == 0 ? 2 : 1;
+    return skinny_dispatch(p, N / (8 * p.tiles), stream);
+}
+
+// out = A W^T (pro 0, 2) or rmsnorm(h) W^T (pro 1); out bf16 (out_f32 0) or float32 (1); or h += ... (residual 1).
 VM_API int vm_skinny_linear(const void* A, int pro, const float* norm_w, float eps, const void* W, int M, int N, int K,
                             void* out, int out_stride, int out_f32, float* residual_h, int* err, cudaStream_t stream) {
     if (N % 8 != 0) return VM_ERR_UNSUPPORTED;
     SkinnyParams p{};
     p.err = err;
-    p.A = A; p.pro = pro; p.norm_w = norm_w; p.eps = eps; p.W = (const __nv_bfloat16*)W; p.M = M; p.N = N; p.K = K;
+    p.W = (const __nv_bfloat16*)W; p.M = M; p.N = N; p.K = K;
+    skinny_rows(p, A, pro, norm_w, eps);
     p.out = out; p.out_stride = out_stride; p.h = residual_h;
     p.epi = residual_h ? EPI_RESIDUAL : (out_f32 ? EPI_STORE_F32 : EPI_STORE_BF16);
-    p.tiles = (N % 16 == 0 && N / 16 >= 148) ? 2 : 1;
+    const bool direct = skinny_variant == 0 && p.pro == PRO_NONE && M <= 32;      // (that kernel takes pairs of column tiles wherever N has them)
+    p.tiles = (N % 16 == 0 && (direct || N / 16 >= 148)) ? 2 : 1;
     const int items = p.tiles == 2 ? N / 16 : N / 8;
     if (skinny_variant < 2 && pro == PRO_NONE && !residual_h && N >= 4096 && (size_t)((M + 15) / 16 * 16) * (K * 2 + 128) <= 200 * 1024) {
         // many columns (the vocabulary head): warps split N, not K; from K = 768 on the ring kernel is faster (49,152 columns,
@@ -184,9 +214,10 @@ VM_API int vm_skinny_linear_act(const void* A, int pro, const float* norm_w, flo
     if (N % 8 != 0 || act < VM_ACT_SILU || act > VM_ACT_RELU_SQUARED) return VM_ERR_UNSUPPORTED;
     SkinnyParams p{};
     p.err = err;
-    p.A = A; p.pro = pro; p.norm_w = norm_w; p.eps = eps; p.W = (const __nv_bfloat16*)W; p.M = M; p.N = N; p.K = K;
+    p.W = (const __nv_bfloat16*)W; p.M = M; p.N = N; p.K = K;
+    skinny_rows(p, A, pro, norm_w, eps);
     p.out = out; p.out_stride = out_stride; p.epi = EPI_STORE_BF16; p.store_act = act + 1;
-    p.tiles = (N % 16 == 0 && N / 16 >= 148) ? 2 : 1;
+    p.tiles = (N % 16 == 0 && ((skinny_variant == 0 && p.pro == PRO_NONE && M <= 32) || N / 16 >= 148)) ? 2 : 1;
     return skinny_dispatch(p, p.tiles == 2 ? N / 16 : N / 8, stream);
 }
 
@@ -196,7 +227,8 @@ VM_API int vm_skinny_gated(const void* A, int pro, const float* norm_w, float ep
     if (I % 8 != 0 || act < VM_ACT_SILU || act > VM_ACT_RELU_SQUARED) return VM_ERR_UNSUPPORTED;
     SkinnyParams p{};
     p.err = err;
-    p.A = A; p.pro = pro; p.norm_w = norm_w; p.eps = eps; p.W = (const __nv_bfloat16*)W; p.M = M; p.N = 2 * I; p.K = K;
+    p.W = (const __nv_bfloat16*)W; p.M = M; p.N = 2 * I; p.K = K;
+    skinny_rows(p, A, pro, norm_w, eps);
     p.out = out; p.out_stride = I; p.I = I; p.epi = EPI_SWIGLU; p.tiles = 2; p.gate_act = act;
     return skinny_dispatch(p, I / 8, stream);
 }
@@ -208,7 +240,8 @@ VM_API int vm_skinny_clamped(const void* A, int pro, const float* norm_w, float 
     if (!(limit > 0.f)) return VM_ERR_BAD_ARG;
     SkinnyParams p{};
     p.err = err;
-    p.A = A; p.pro = pro; p.norm_w = norm_w; p.eps = eps; p.W = (const __nv_bfloat16*)W; p.M = M; p.N = 2 * I; p.K = K;
+    p.W = (const __nv_bfloat16*)W; p.M = M; p.N = 2 * I; p.K = K;
+    skinny_rows(p, A, pro, norm_w, eps);
     p.out = out; p.out_stride = I; p.I = I; p.epi = EPI_SWIGLU; p.tiles = 2; p.gate_act = GATE_CLAMPED; p.limit = limit; p.alpha = alpha;
     return skinny_dispatch(p, I / 8, stream);
 }
@@ -230,7 +263,8 @@ VM_API int vm_skinny_qkv_rope(const void* A, int pro, const float* norm_w, float
     if (D % 16 != 0 || !(rot_dim == 0 || rot_dim == D) || (rot_dim > 0 && inv_freq == nullptr)) return VM_ERR_UNSUPPORTED;
     if (rot_dim > 0 && pairing != VM_PAIR_HALF_SPLIT) return VM_ERR_UNSUPPORTED;
     SkinnyParams p{};
-    p.A = A; p.pro = pro; p.norm_w = norm_w; p.eps = eps; p.W = (const __nv_bfloat16*)W; p.M = M; p.N = (H + 2 * Hkv) * D; p.K = K;
+    p.W = (const __nv_bfloat16*)W; p.M = M; p.N = (H + 2 * Hkv) * D; p.K = K;
+    skinny_rows(p, A, pro, norm_w, eps);
     p.out = q_out; p.out_stride = H * D; p.epi = EPI_ROPE_KV; p.tiles = 2;
     p.positions = positions; p.seq_of_token = seq_of_token; p.block_table = block_table; p.max_blocks = max_blocks;
     p.inv_freq = inv_freq; p.rot_dim = rot_dim; p.kpages = (__nv_bfloat16*)kpages; p.vpages = (__nv_bfloat16*)vpages;

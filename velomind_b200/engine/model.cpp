@@ -201,6 +201,7 @@ void DecoderModel::forward(StepContext& ctx) {
     for (size_t run = 0; run < plan.schedule.size(); ++run) {
         ctx.run = static_cast<int>(run);
         ctx.state_offset = 0;
+        ctx.following_norm = run + 1 < plan.schedule.size() ? layers[plan.schedule[run + 1].layer].block->takes_ready(ctx) : nullptr;
         pending = layers[plan.schedule[run].layer].block->forward(ctx, h, pending);
         if (dump_stream_path() && !ctx.capturing) {
             if (pending && ctx.pending_mix) {        // (written into the copies now, so that the dumped rows hold it)

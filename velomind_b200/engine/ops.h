@@ -430,42 +430,63 @@ inline int skinny_max_rows(long long weight_bytes) {
 }
 inline bool skinny_ok(int M, long long K, const DeviceTensor& W) { return M > 0 && M <= SKINNY_MAX_ROWS && K % 32 == 0 && W.dtype == DType::BF16; }
 
-inline void skinny_linear(const void* x, const float* norm_w, float eps, const DeviceTensor& W, int M, void* out, int out_stride, bool out_f32,
-                          float* residual, int* err, cudaStream_t s) {
+constexpr int READY_ROWS = 32;     // (the kernel of ready rows takes no more)
+// The rows a weight-streaming product multiplies: plain bfloat16 rows; the float32 stream with the norm in front of the product; or rows that carry the
+// norm's weight already, with the parts of their sums of squares (StepContext::ready).
+struct Rows {
+    Rows(const void* plain) : x(plain) {}
+    Rows(const void* x_, int pro_, const float* w_, float eps_) : x(x_), pro(pro_), w(w_), eps(eps_) {}
+    const void* x;
+    int pro = 0;
+    const float* w = nullptr;
+    float eps = 0.f;
+};
+// the rows of norm(h): those that the sublayer in front left ready, else h with the norm
+inline Rows normed_rows(const StepContext& ctx, const float* h, const float* norm_w, float eps) {
+    if (ctx.ready.weight && ctx.ready.weight == norm_w) return Rows(ctx.ready.rows, 2, ctx.ready.squares, eps);
+    return Rows(h, 1, norm_w, eps);
+}
+
+inline void skinny_linear(const Rows& r, const DeviceTensor& W, int M, void* out, int out_stride, bool out_f32, int* err, cudaStream_t s) {
     Timed t("skinny_linear", s);
-    check(vm_skinny_linear(x, norm_w ? 1 : 0, norm_w, eps, W.ptr, M, static_cast<int>(W.rows()), static_cast<int>(W.cols()), out, out_stride,
-                           out_f32 ? 1 : 0, residual, err, s),
+    check(vm_skinny_linear(r.x, r.pro, r.w, r.eps, W.ptr, M, static_cast<int>(W.rows()), static_cast<int>(W.cols()), out, out_stride, out_f32 ? 1 : 0,
+                           nullptr, err, s),
           "skinny_linear", s);
 }
 
-inline void skinny_linear_act(const void* x, const float* norm_w, float eps, const DeviceTensor& W, int M, int act, void* out, int out_stride, int* err,
-                              cudaStream_t s) {
+// h += x W^T (x plain rows); leaves the new rows ready where the wiring asks for it
+inline void skinny_residual(StepContext& ctx, const void* x, const DeviceTensor& W, float* h) {
+    const int N = static_cast<int>(W.rows()), K = static_cast<int>(W.cols());
+    Timed t("skinny_linear", ctx.stream);
+    if (!ctx.next_norm || ctx.T_cap > READY_ROWS) {
+        check(vm_skinny_linear(x, 0, nullptr, 0.f, W.ptr, ctx.T, N, K, nullptr, N, 0, h, ctx.err, ctx.stream), "skinny_linear", ctx.stream);
+        return;
+    }
+    ctx.made.weight = ctx.next_norm;
+    ctx.made.rows = ctx.take_tokens(N, DType::BF16);
+    ctx.made.squares = static_cast<float*>(ctx.take_tokens(vm_skinny_ready_parts(N), DType::F32));
+    check(vm_skinny_residual_ready(x, W.ptr, ctx.T, N, K, h, ctx.next_norm, ctx.made.rows, ctx.made.squares, ctx.stream), "skinny_linear", ctx.stream);
+}
+
+inline void skinny_linear_act(const Rows& r, const DeviceTensor& W, int M, int act, void* out, int out_stride, int* err, cudaStream_t s) {
     Timed t("skinny_linear_act", s);
-    check(vm_skinny_linear_act(x, norm_w ? 1 : 0, norm_w, eps, W.ptr, M, static_cast<int>(W.rows()), static_cast<int>(W.cols()), act, out, out_stride, err, s),
+    check(vm_skinny_linear_act(r.x, r.pro, r.w, r.eps, W.ptr, M, static_cast<int>(W.rows()), static_cast<int>(W.cols()), act, out, out_stride, err, s),
           "skinny_linear_act", s);
 }
 
-inline void skinny_swiglu(const void* x, const float* norm_w, float eps, const DeviceTensor& W, int M, int I, void* out, int* err, cudaStream_t s) {
-    Timed t("skinny_swiglu", s);
-    check(vm_skinny_swiglu(x, norm_w ? 1 : 0, norm_w, eps, W.ptr, M, I, static_cast<int>(W.cols()), out, err, s), "skinny_swiglu", s);
-}
-
-inline void skinny_gated(const void* x, const float* norm_w, float eps, const DeviceTensor& W, int M, int I, int act, void* out, int* err,
-                         cudaStream_t s) {
+inline void skinny_gated(const Rows& r, const DeviceTensor& W, int M, int I, int act, void* out, int* err, cudaStream_t s) {
     Timed t("skinny_gated", s);
-    check(vm_skinny_gated(x, norm_w ? 1 : 0, norm_w, eps, W.ptr, M, I, static_cast<int>(W.cols()), act, out, err, s), "skinny_gated", s);
+    check(vm_skinny_gated(r.x, r.pro, r.w, r.eps, W.ptr, M, I, static_cast<int>(W.cols()), act, out, err, s), "skinny_gated", s);
 }
 
-inline void skinny_clamped(const void* x, const float* norm_w, float eps, const DeviceTensor& W, int M, int I, float limit, float alpha, void* out, int* err,
-                           cudaStream_t s) {
+inline void skinny_clamped(const Rows& r, const DeviceTensor& W, int M, int I, float limit, float alpha, void* out, int* err, cudaStream_t s) {
     Timed t("skinny_gated", s);
-    check(vm_skinny_clamped(x, norm_w ? 1 : 0, norm_w, eps, W.ptr, M, I, static_cast<int>(W.cols()), limit, alpha, out, err, s), "skinny_gated", s);
+    check(vm_skinny_clamped(r.x, r.pro, r.w, r.eps, W.ptr, M, I, static_cast<int>(W.cols()), limit, alpha, out, err, s), "skinny_gated", s);
 }
 
-inline void skinny_qkv_rope(const void* x, const float* norm_w, float eps, const DeviceTensor& W, void* q_out, const StepContext& ctx, const KVView& kv,
-                            const RotaryTable& rot, int H, int Hkv, int D) {
+inline void skinny_qkv_rope(const Rows& r, const DeviceTensor& W, void* q_out, const StepContext& ctx, const KVView& kv, const RotaryTable& rot, int H, int Hkv, int D) {
     Timed t("skinny_qkv_rope", ctx.stream);
-    check(vm_skinny_qkv_rope(x, norm_w ? 1 : 0, norm_w, eps, W.ptr, ctx.T, static_cast<int>(W.cols()), q_out, ctx.positions, ctx.seq_of_token,
+    check(vm_skinny_qkv_rope(r.x, r.pro, r.w, r.eps, W.ptr, ctx.T, static_cast<int>(W.cols()), q_out, ctx.positions, ctx.seq_of_token,
                              kv.block_table, kv.table_width, rot.inv_freq, rot.rotary_dim, rot.pairing, kv.owns ? kv.k_pages : nullptr,
                              kv.owns ? kv.v_pages : nullptr, H, Hkv, D, kv.owns ? kv.n_pages : 0, ctx.err, ctx.stream),
           "skinny_qkv_rope", ctx.stream);

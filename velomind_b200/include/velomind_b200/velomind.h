@@ -497,6 +497,24 @@ struct StepContext {
     bool takes_two_terms = false;
     void* second_term = nullptr;
     float first_weight = 1.f, second_weight = 0.f;
+    // Few tokens in bfloat16: a sublayer whose last product adds into the stream may leave the new rows ready for the product behind the norm that
+    // reads them next (h x that norm's weight, and the parts of the rows' sums of squares), so that no block of that product norms them again.  The
+    // wiring names the norm in `next_norm` where the sublayer behind it takes such rows, finds them in `made` and hands them on in `ready`, which is
+    // given back when that sublayer has run.
+    struct ReadyRows {
+        const float* weight = nullptr;          // the norm's weight they carry (null: there are none)
+        void* rows = nullptr;                   // bfloat16 [T, hidden]
+        float* squares = nullptr;               // float32 [T, vm_skinny_ready_parts(hidden)]
+    };
+    const float* next_norm = nullptr;
+    const float* following_norm = nullptr;      // the norm whose ready rows the next layer's first sublayer takes (null: none)
+    ReadyRows ready, made;
+    void pass_ready_on() {                      // after a sublayer: what it read is given back, what it made is for the next one
+        if (ready.weight) { give(ready.rows); give(ready.squares); }
+        ready = made;
+        made = ReadyRows();
+        next_norm = nullptr;
+    }
     // Rows per token that a model keeps beside its embedding (all layers' side by side, in one table), or null
     const DeviceTensor* token_rows = nullptr;
     // ... or, in a model with several copies of the stream, through the mixing its layer left with it: copy t becomes
@@ -564,6 +582,8 @@ public:
     // optional: take the norm before the part and the residual sum after it into the part's own kernels
     virtual bool can_fuse(const StepContext&, const Norm&) const { return false; }
     virtual void forward_fused(StepContext&, float* /*h*/, Norm&) {}
+    // optional: whether forward_fused takes ctx.ready instead of norming h itself (of a part that fuses in this step)
+    virtual bool takes_ready(const StepContext&) const { return false; }
 };
 
 class FeedForward : public Part {
@@ -571,6 +591,7 @@ public:
     virtual void forward(StepContext& ctx, const void* x, void* out) = 0;
     virtual bool can_fuse(const StepContext&, const Norm&) const { return false; }
     virtual void forward_fused(StepContext&, float* /*h*/, Norm&) {}
+    virtual bool takes_ready(const StepContext&) const { return false; }
 };
 
 struct BlockParts {
@@ -587,6 +608,8 @@ public:
     // float32 values the wiring itself keeps per sequence (the last inputs of a convolution over time); they lie behind the mixer's
     // own state in the run's state area, at offset mixer->cache_need().state_floats
     virtual int state_floats() const { return 0; }
+    // the weight of the norm whose rows the layer's first sublayer would take ready in this step (null: it norms the stream itself)
+    virtual const float* takes_ready(const StepContext&) const { return nullptr; }
     // whether the wiring knows of several copies of the residual stream (a model that keeps more than one needs it of every layer)
     virtual bool mixes_streams() const { return false; }
 };

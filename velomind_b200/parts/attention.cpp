@@ -72,6 +72,8 @@ public:
         return true;
     }
 
+    bool takes_ready(const StepContext& ctx) const override { return !few_f32(ctx) && ctx.T_cap <= std::min(max_rows(), ops::SKINNY_NORM_ROWS); }
+
     // a few rows in float32: norm + q k v, rotary + cache write, attention, out added into h
     bool few_f32(const StepContext& ctx) const {
         return ctx.act_dtype == DType::F32 && ctx.T_cap <= ops::FEW_F32_ROWS && qkv_.weight.dtype == DType::F32 && out_.weight.dtype == DType::F32 &&
@@ -117,18 +119,18 @@ public:
         }
         void* q = ctx.take_tokens(static_cast<long long>(H_) * D_, DType::BF16);
         if (skinny && ctx.T_cap <= ops::SKINNY_NORM_ROWS) {
-            ops::skinny_qkv_rope(h, nw, eps, qkv_.weight, q, ctx, kv, rotary_, H_, Hkv_, D_);
+            ops::skinny_qkv_rope(ops::normed_rows(ctx, h, nw, eps), qkv_.weight, q, ctx, kv, rotary_, H_, Hkv_, D_);
         } else {
             void* x = ctx.take_tokens(hidden_, DType::BF16);           // many rows: norm once, not once per CTA
             norm.forward(ctx, h, nullptr, x, nullptr, 0);
-            if (skinny) ops::skinny_qkv_rope(x, nullptr, 0.f, qkv_.weight, q, ctx, kv, rotary_, H_, Hkv_, D_);
+            if (skinny) ops::skinny_qkv_rope(x, qkv_.weight, q, ctx, kv, rotary_, H_, Hkv_, D_);
             else ops::tc_qkv_rope(x, hidden_, qkv_.weight, q, ctx, kv, rotary_, H_, Hkv_, D_);
             ctx.give(x);
         }
         void* att = ctx.take_tokens(static_cast<long long>(H_) * D_, DType::BF16);
         ops::attention(ctx, q, H_ * D_, kv, att, H_, Hkv_, D_, scale_, window_);
         ctx.give(q);
-        if (skinny) ops::skinny_linear(att, nullptr, 0.f, out_.weight, ctx.T, nullptr, hidden_, false, h, ctx.err, ctx.stream);
+        if (skinny) ops::skinny_residual(ctx, att, out_.weight, h);
         else ops::tc_linear(att, static_cast<long long>(H_) * D_, out_.weight, ctx.T, nullptr, hidden_, false, h, ctx.err, ctx.stream);
         ctx.give(att);
     }

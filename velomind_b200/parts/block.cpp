@@ -24,6 +24,9 @@ class PreNormBlock : public Arrangement {
 public:
     explicit PreNormBlock(const BlockParts& p, bool feed_forward = true) : p_(p), feed_forward_(feed_forward) {}
     bool graph_safe() const override { return true; }
+    const float* takes_ready(const StepContext& ctx) const override {
+        return p_.mixer->can_fuse(ctx, *p_.mixer_norm) && p_.mixer->takes_ready(ctx) ? weight_of(*p_.mixer_norm) : nullptr;
+    }
 
     void* forward(StepContext& ctx, float* h, void* pending) override {
         const long long hid = hidden(ctx);
@@ -33,7 +36,11 @@ public:
         }
         if (p_.mixer->can_fuse(ctx, *p_.mixer_norm)) {
             settle(ctx, h, pending, hid);
+            if (feed_forward_ && p_.feed_forward->can_fuse(ctx, *p_.feed_forward_norm) && p_.feed_forward->takes_ready(ctx))
+                ctx.next_norm = weight_of(*p_.feed_forward_norm);
+            else if (!feed_forward_) ctx.next_norm = ctx.following_norm;
             p_.mixer->forward_fused(ctx, h, *p_.mixer_norm);
+            ctx.pass_ready_on();
             pending = nullptr;
         } else {
             void* x = ctx.take_tokens(hid, ctx.act_dtype);
@@ -46,7 +53,9 @@ public:
         if (!feed_forward_) return pending;        // a layer that is its mixer alone
         if (p_.feed_forward->can_fuse(ctx, *p_.feed_forward_norm)) {
             settle(ctx, h, pending, hid);
+            ctx.next_norm = ctx.following_norm;
             p_.feed_forward->forward_fused(ctx, h, *p_.feed_forward_norm);
+            ctx.pass_ready_on();
             return nullptr;
         }
         void* x = ctx.take_tokens(hid, ctx.act_dtype);
@@ -60,6 +69,11 @@ public:
 
 private:
     static long long hidden(const StepContext& ctx) { return ctx.hidden; }
+    static const float* weight_of(const Norm& norm) {
+        const float* w = nullptr;
+        float eps = 0.f;
+        return norm.as_rms(&w, &eps) ? w : nullptr;
+    }
     // add a delta that is still pending to the residual stream
     static void settle(StepContext& ctx, float* h, void* pending, long long hid) { settle_pending(ctx, h, pending, hid); }
     BlockParts p_;

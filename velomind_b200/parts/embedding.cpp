@@ -106,7 +106,7 @@ public:
     bool graph_safe() const override { return true; }
     void forward(StepContext& ctx, const void* x, float* logits) override {
         if (ctx.act_dtype == DType::BF16 && ops::skinny_ok(ctx.R, hidden_, proj_.weight) && vocab_ % 8 == 0 && ctx.R_cap <= ops::SKINNY_HEAD_MAX_ROWS)
-            ops::skinny_linear(x, nullptr, 0.f, proj_.weight, ctx.R, logits, vocab_, true, nullptr, ctx.err, ctx.stream);   // few rows: stream the table once
+            ops::skinny_linear(x, proj_.weight, ctx.R, logits, vocab_, true, ctx.err, ctx.stream);   // few rows: stream the table once
         else
             proj_.apply(ctx, x, ctx.act_dtype, logits, DType::F32, ctx.R, ctx.R_cap);
         if (cap_ > 0.f) ops::soft_cap(logits, static_cast<long long>(ctx.R) * vocab_, cap_, ctx.stream);

@@ -51,6 +51,8 @@ public:
         return hidden_ % 8 == 0 && I_ % 8 == 0;
     }
 
+    bool takes_ready(const StepContext& ctx) const override { return !few_f32(ctx) && ctx.T_cap <= std::min(max_rows(), ops::SKINNY_NORM_ROWS); }
+
     // a few rows in float32: norm + gate and up + SwiGLU, down added into h
     bool few_f32(const StepContext& ctx) const {
         return ctx.act_dtype == DType::F32 && ctx.T_cap <= ops::FEW_F32_ROWS && gate_up_.weight.dtype == DType::F32 && down_.weight.dtype == DType::F32 &&
@@ -87,15 +89,15 @@ public:
         }
         void* act = ctx.take_tokens(I_, DType::BF16);
         if (skinny && ctx.T_cap <= ops::SKINNY_NORM_ROWS) {
-            few_rows(ctx, h, nw, eps, act);
+            few_rows(ctx, ops::normed_rows(ctx, h, nw, eps), act);
         } else {
             void* x = ctx.take_tokens(hidden_, DType::BF16);           // many rows: norm once, not once per CTA
             norm.forward(ctx, h, nullptr, x, nullptr, 0);
-            if (skinny) few_rows(ctx, x, nullptr, 0.f, act);
+            if (skinny) few_rows(ctx, x, act);
             else ops::tc_swiglu(x, hidden_, gate_up_.weight, ctx.T, I_, act, ctx.err, ctx.stream);
             ctx.give(x);
         }
-        if (skinny) ops::skinny_linear(act, nullptr, 0.f, down_.weight, ctx.T, nullptr, hidden_, false, h, ctx.err, ctx.stream);
+        if (skinny) ops::skinny_residual(ctx, act, down_.weight, h);
         else ops::tc_linear(act, I_, down_.weight, ctx.T, nullptr, hidden_, false, h, ctx.err, ctx.stream);
         ctx.give(act);
     }
@@ -105,8 +107,8 @@ public:
         if (ctx.act_dtype == DType::BF16 && gate_up_.weight.dtype == DType::BF16 && down_.weight.dtype == DType::BF16 && ctx.T_cap <= max_rows() &&
             hidden_ % 32 == 0 && I_ % 32 == 0 && ctx.T > 0) {
             void* act = ctx.take_tokens(I_, DType::BF16);
-            few_rows(ctx, x, nullptr, 0.f, act);
-            ops::skinny_linear(act, nullptr, 0.f, down_.weight, ctx.T, out, hidden_, false, nullptr, ctx.err, ctx.stream);
+            few_rows(ctx, x, act);
+            ops::skinny_linear(act, down_.weight, ctx.T, out, hidden_, false, ctx.err, ctx.stream);
             ctx.give(act);
             return;
         }
@@ -125,10 +127,10 @@ private:
         if (clamped()) ops::clamped_unit(gu, out, ctx.T, I_, limit_, alpha_, ctx.act_dtype, ctx.stream);
         else ops::gated_activation(gu, out, ctx.T, I_, act_, ctx.act_dtype, ctx.stream);
     }
-    // few rows: both products and the unit in one kernel (nw given: of the norm of the float32 residual rows)
-    void few_rows(StepContext& ctx, const void* x, const float* nw, float eps, void* out) {
-        if (clamped()) ops::skinny_clamped(x, nw, eps, gate_up_.weight, ctx.T, I_, limit_, alpha_, out, ctx.err, ctx.stream);
-        else ops::skinny_gated(x, nw, eps, gate_up_.weight, ctx.T, I_, act_, out, ctx.err, ctx.stream);
+    // few rows: both products and the unit in one kernel
+    void few_rows(StepContext& ctx, const ops::Rows& x, void* out) {
+        if (clamped()) ops::skinny_clamped(x, gate_up_.weight, ctx.T, I_, limit_, alpha_, out, ctx.err, ctx.stream);
+        else ops::skinny_gated(x, gate_up_.weight, ctx.T, I_, act_, out, ctx.err, ctx.stream);
     }
     int hidden_, I_, act_;
     std::string gate_name_, up_name_, down_name_;
@@ -178,6 +180,8 @@ public:
         return hidden_ % 8 == 0 && I_ % 8 == 0;
     }
 
+    bool takes_ready(const StepContext& ctx) const override { return ctx.T_cap <= std::min(max_rows(), ops::SKINNY_NORM_ROWS); }
+
     // h += down(act(up(norm(h)))): the norm in the first product (few tokens), the sum in the second
     void forward_fused(StepContext& ctx, float* h, Norm& norm) override {
         const float* nw = nullptr;
@@ -187,19 +191,19 @@ public:
         void* u = ctx.take_tokens(I_, DType::BF16);
         // (few tokens: the activation rides in the first product's epilogue)
         if (skinny && ctx.T_cap <= ops::SKINNY_NORM_ROWS) {
-            ops::skinny_linear_act(h, nw, eps, up_.weight, ctx.T, act_, u, I_, ctx.err, ctx.stream);
+            ops::skinny_linear_act(ops::normed_rows(ctx, h, nw, eps), up_.weight, ctx.T, act_, u, I_, ctx.err, ctx.stream);
         } else {
             void* x = ctx.take_tokens(hidden_, DType::BF16);
             norm.forward(ctx, h, nullptr, x, nullptr, 0);
             if (skinny) {
-                ops::skinny_linear_act(x, nullptr, 0.f, up_.weight, ctx.T, act_, u, I_, ctx.err, ctx.stream);
+                ops::skinny_linear_act(x, up_.weight, ctx.T, act_, u, I_, ctx.err, ctx.stream);
             } else {
                 ops::linear(x, DType::BF16, hidden_, up_.weight, u, DType::BF16, ctx.T, ctx.stream);
                 ops::activation(u, u, static_cast<long long>(ctx.T) * I_, act_, DType::BF16, ctx.stream);
             }
             ctx.give(x);
         }
-        if (skinny) ops::skinny_linear(u, nullptr, 0.f, down_.weight, ctx.T, nullptr, hidden_, false, h, ctx.err, ctx.stream);
+        if (skinny) ops::skinny_residual(ctx, u, down_.weight, h);
         else ops::linear_residual(u, I_, down_.weight, h, ctx.T, ctx.stream);
         ctx.give(u);
     }
@@ -212,7 +216,7 @@ public:
         if (act_ == VM_ACT_POLYNORM) {
             if (few) {
                 float* z = static_cast<float*>(ctx.take_tokens(I_, DType::F32));
-                ops::skinny_linear(x, nullptr, 0.f, up_.weight, ctx.T, z, I_, true, nullptr, ctx.err, ctx.stream);
+                ops::skinny_linear(x, up_.weight, ctx.T, z, I_, true, ctx.err, ctx.stream);
                 ops::polynorm(z, DType::F32, static_cast<const float*>(coef_.ptr), u, ctx.T, I_, eps_, ctx.act_dtype, ctx.stream);
                 ctx.give(z);
             } else {
@@ -220,12 +224,12 @@ public:
                 ops::polynorm(u, ctx.act_dtype, static_cast<const float*>(coef_.ptr), u, ctx.T, I_, eps_, ctx.act_dtype, ctx.stream);
             }
         } else if (few) {
-            ops::skinny_linear_act(x, nullptr, 0.f, up_.weight, ctx.T, act_, u, I_, ctx.err, ctx.stream);
+            ops::skinny_linear_act(x, up_.weight, ctx.T, act_, u, I_, ctx.err, ctx.stream);
         } else {
             up_.apply(ctx, x, ctx.act_dtype, u, ctx.act_dtype, ctx.T, ctx.T_cap);
             ops::activation(u, u, static_cast<long long>(ctx.T) * I_, act_, ctx.act_dtype, ctx.stream);
         }
-        if (few) ops::skinny_linear(u, nullptr, 0.f, down_.weight, ctx.T, out, hidden_, false, nullptr, ctx.err, ctx.stream);
+        if (few) ops::skinny_linear(u, down_.weight, ctx.T, out, hidden_, false, ctx.err, ctx.stream);
         else down_.apply(ctx, u, ctx.act_dtype, out, ctx.act_dtype, ctx.T, ctx.T_cap);
         ctx.give(u);
     }

@@ -126,24 +126,26 @@ public:
         return hidden_ % 32 == 0 && Rq_ % 32 == 0 && (H_ * V_) % 32 == 0 && down_cols() % 8 == 0 && (H_ * (D_ + R_)) % 8 == 0 && hidden_ % 8 == 0;
     }
 
+    bool takes_ready(const StepContext&) const override { return true; }
+
     void forward_fused(StepContext& ctx, float* h, Norm& norm) override {
         const float* nw = nullptr;
         float eps = 0.f;
         norm.as_rms(&nw, &eps);
         KVView kv = ctx.kv();
         if (kv.owns != own_) throw ConfigError("a latent-attention layer and its schedule disagree about whose latents it reads");
-        void* o = heads(ctx, h, nw, eps, kv, true);
-        ops::skinny_linear(o, nullptr, 0.f, out_.weight, ctx.T, nullptr, hidden_, false, h, ctx.err, ctx.stream);
+        void* o = heads(ctx, ops::normed_rows(ctx, h, nw, eps), kv, true);
+        ops::skinny_residual(ctx, o, out_.weight, h);
         ctx.give(o);
     }
 
-    // x [T, hidden] (or, with norm_w, the float32 stream whose rows the first product norms) -> the heads' gated outputs [T, H*V]
-    void* heads(StepContext& ctx, const void* x, const float* norm_w, float eps, KVView kv, bool skinny_products) {
+    // x [T, hidden] (with skinny_products also the stream's rows behind its norm) -> the heads' gated outputs [T, H*V]
+    void* heads(StepContext& ctx, const ops::Rows& x, KVView kv, bool skinny_products) {
         const DType act = ctx.act_dtype;
         const int cols = down_cols();
         float* down = static_cast<float*>(ctx.take_tokens(cols, DType::F32));
-        if (skinny_products) ops::skinny_linear(x, norm_w, eps, down_.weight, ctx.T, down, cols, true, nullptr, ctx.err, ctx.stream);
-        else down_.apply(ctx, x, act, down, DType::F32, ctx.T, ctx.T_cap);
+        if (skinny_products) ops::skinny_linear(x, down_.weight, ctx.T, down, cols, true, ctx.err, ctx.stream);
+        else down_.apply(ctx, x.x, act, down, DType::F32, ctx.T, ctx.T_cap);
         void* cq = ctx.take_tokens(Rq_, act);
         ops::latent_rope_norm_write(down, cols, Rq_, Rkv_, static_cast<const float*>(q_norm_.ptr), own_ ? static_cast<const float*>(kv_norm_.ptr) : nullptr,
                                     eps_, cq, ctx, kv, own_, R_, rotary_);
@@ -153,7 +155,7 @@ public:
         }
         const long long q_cols = static_cast<long long>(H_) * (D_ + R_);
         void* q = ctx.take_tokens(q_cols, act);
-        if (skinny_products) ops::skinny_linear(cq, nullptr, 0.f, up_q_.weight, ctx.T, q, static_cast<int>(q_cols), false, nullptr, ctx.err, ctx.stream);
+        if (skinny_products) ops::skinny_linear(cq, up_q_.weight, ctx.T, q, static_cast<int>(q_cols), false, ctx.err, ctx.stream);
         else up_q_.apply(ctx, cq, act, q, act, ctx.T, ctx.T_cap);
         ctx.give(cq);
         void* o = attend(ctx, q, kv, gate_ ? down + gate_col() : nullptr, cols);
@@ -251,8 +253,8 @@ public:
             return;
         }
         const bool few = skinny(ctx);                      // (a choice by the step's capacity bucket)
-        void* o = heads(ctx, x, nullptr, 0.f, kv, few);
-        if (few) ops::skinny_linear(o, nullptr, 0.f, out_.weight, ctx.T, out, hidden_, false, nullptr, ctx.err, ctx.stream);
+        void* o = heads(ctx, x, kv, few);
+        if (few) ops::skinny_linear(o, out_.weight, ctx.T, out, hidden_, false, ctx.err, ctx.stream);
         else out_.apply(ctx, o, act, out, act, ctx.T, ctx.T_cap);
         ctx.give(o);
     }

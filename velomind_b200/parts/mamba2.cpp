@@ -88,6 +88,8 @@ public:
         return true;
     }
 
+    bool takes_ready(const StepContext& ctx) const override { return ctx.T_cap <= std::min(max_rows(), ops::SKINNY_NORM_ROWS); }
+
     void forward_fused(StepContext& ctx, float* h, Norm& norm) override {
         const float* nw = nullptr;
         float eps = 0.f;
@@ -95,18 +97,18 @@ public:
         const bool skinny = ctx.T_cap <= max_rows();
         void* proj = ctx.take_tokens(width(), DType::BF16);
         if (skinny && ctx.T_cap <= ops::SKINNY_NORM_ROWS) {
-            ops::skinny_linear(h, nw, eps, in_.weight, ctx.T, proj, static_cast<int>(width()), false, nullptr, ctx.err, ctx.stream);
+            ops::skinny_linear(ops::normed_rows(ctx, h, nw, eps), in_.weight, ctx.T, proj, static_cast<int>(width()), false, ctx.err, ctx.stream);
         } else {
             void* x = ctx.take_tokens(hidden_, DType::BF16);
             norm.forward(ctx, h, nullptr, x, nullptr, 0);
-            if (skinny) ops::skinny_linear(x, nullptr, 0.f, in_.weight, ctx.T, proj, static_cast<int>(width()), false, nullptr, ctx.err, ctx.stream);
+            if (skinny) ops::skinny_linear(x, in_.weight, ctx.T, proj, static_cast<int>(width()), false, ctx.err, ctx.stream);
             else ops::linear(x, DType::BF16, hidden_, in_.weight, proj, DType::BF16, ctx.T, ctx.stream);
             ctx.give(x);
         }
         void* y = ctx.take_tokens(inner(), DType::BF16);
         mix(ctx, proj, y);
         ctx.give(proj);
-        if (skinny) ops::skinny_linear(y, nullptr, 0.f, out_.weight, ctx.T, nullptr, hidden_, false, h, ctx.err, ctx.stream);
+        if (skinny) ops::skinny_residual(ctx, y, out_.weight, h);
         else ops::linear_residual(y, inner(), out_.weight, h, ctx.T, ctx.stream);
         ctx.give(y);
     }

@@ -59,18 +59,20 @@ public:
         return hidden_ % 32 == 0 && (H_ * V_) % 32 == 0 && proj_.weight.rows() % 8 == 0;
     }
 
+    bool takes_ready(const StepContext&) const override { return true; }
+
     void forward_fused(StepContext& ctx, float* h, Norm& norm) override {
         const float* nw = nullptr;
         float eps = 0.f;
         norm.as_rms(&nw, &eps);
         const int cols = static_cast<int>(proj_.weight.rows());
         float* proj = static_cast<float*>(ctx.take_tokens(cols, DType::F32));
-        ops::skinny_linear(h, nw, eps, proj_.weight, ctx.T, proj, cols, true, nullptr, ctx.err, ctx.stream);
+        ops::skinny_linear(ops::normed_rows(ctx, h, nw, eps), proj_.weight, ctx.T, proj, cols, true, ctx.err, ctx.stream);
         void* y = ctx.take_tokens(static_cast<long long>(H_) * V_, DType::BF16);
         ops::mlstm_scan(proj, cols, static_cast<const float*>(bias_i_.ptr), static_cast<const float*>(bias_f_.ptr), static_cast<const float*>(norm_.ptr),
                         ctx, y, H_, D_, V_, cap_, eps_);
         ctx.give(proj);
-        ops::skinny_linear(y, nullptr, 0.f, out_.weight, ctx.T, nullptr, hidden_, false, h, ctx.err, ctx.stream);
+        ops::skinny_residual(ctx, y, out_.weight, h);
         ctx.give(y);
     }
 

@@ -149,6 +149,8 @@ public:
         return true;
     }
 
+    bool takes_ready(const StepContext& ctx) const override { return ctx.T_cap <= std::min(max_rows(), ops::SKINNY_NORM_ROWS); }
+
     void forward_fused(StepContext& ctx, float* h, Norm& norm) override {
         const float* nw = nullptr;
         float eps = 0.f;
@@ -156,18 +158,18 @@ public:
         const bool skinny = ctx.T_cap <= max_rows();
         void* qkv = ctx.take_tokens(width(), DType::BF16);
         if (skinny && ctx.T_cap <= ops::SKINNY_NORM_ROWS) {
-            ops::skinny_linear(h, nw, eps, qkv_.weight, ctx.T, qkv, static_cast<int>(width()), false, nullptr, ctx.err, ctx.stream);
+            ops::skinny_linear(ops::normed_rows(ctx, h, nw, eps), qkv_.weight, ctx.T, qkv, static_cast<int>(width()), false, ctx.err, ctx.stream);
         } else {
             void* x = ctx.take_tokens(hidden_, DType::BF16);
             norm.forward(ctx, h, nullptr, x, nullptr, 0);
-            if (skinny) ops::skinny_linear(x, nullptr, 0.f, qkv_.weight, ctx.T, qkv, static_cast<int>(width()), false, nullptr, ctx.err, ctx.stream);
+            if (skinny) ops::skinny_linear(x, qkv_.weight, ctx.T, qkv, static_cast<int>(width()), false, ctx.err, ctx.stream);
             else ops::linear(x, DType::BF16, hidden_, qkv_.weight, qkv, DType::BF16, ctx.T, ctx.stream);
             ctx.give(x);
         }
         void* att = ctx.take_tokens(static_cast<long long>(H_) * Dv_, DType::BF16);
         attend(ctx, qkv, att);
         ctx.give(qkv);
-        if (skinny) ops::skinny_linear(att, nullptr, 0.f, out_.weight, ctx.T, nullptr, hidden_, false, h, ctx.err, ctx.stream);
+        if (skinny) ops::skinny_residual(ctx, att, out_.weight, h);
         else ops::linear_residual(att, static_cast<long long>(H_) * Dv_, out_.weight, h, ctx.T, ctx.stream);
         ctx.give(att);
     }
