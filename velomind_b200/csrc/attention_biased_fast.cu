@@ -13,12 +13,15 @@
 // maximum, exponentials, products) at the few warps an SM holds: so the query operands stay in registers, a block has one barrier, and a block
 // that every row of a warp sees whole takes no mask.  Measured against two barriers, operands from shared memory and a mask on every score:
 // 1,400 + 2,000 tokens of 32 heads of 64 with slopes 144 -> 116 us, over a latent of 160 values 267 -> 226; eight prompts of 130 to 509 tokens,
-// 16 heads and a table 31.3 -> 26.5; four of 301 to 850 with a sink 39.6 -> 33.2; eight of 512, chunked, 42.3 -> 36.7.
+// 16 heads and a table 31.3 -> 26.5; four of 301 to 850 with a sink 39.6 -> 33.2; eight of 512, chunked, 42.3 -> 36.7.  The tiles are dealt out by their length
+// (tile_order.cuh): without options, 16 heads of 64, 1,400 + 2,000 tokens 82.8 -> 61.6 us, eight of 130 to 508 23.5 -> 17.6, four of 301 to 850 31.5 -> 24.0,
+// eight of 512 34.0 -> 28.0.
 //
 // Decode steps (of sizes that attention_decode_tile.cu does not take).  One CTA per (sequence, query head); its warps take the visible keys in chunks of 32 (a key per lane,
 // float32 dot products from 16-byte loads), keep a float32 online softmax each, and warp 0 joins the warps' results in warp
 // order: the answer does not depend on the batch.
 #include "mma.cuh"
+#include "tile_order.cuh"
 
 namespace {
 
@@ -42,13 +45,13 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // VK: a token's value is the first DV values of its key row (one pool, one tile in shared memory: nothing else is fetched for the values).
 // Registers for as many CTAs an SM as the sizes allow: unrolled without a bound, the kernel for keys of 96 and values of 64 took 187 and left two CTAs
 // instead of three (3,000 tokens, 8 heads in a window of 128: 18.3 us).
-template <int DK, int DV> constexpr int prefill_ctas() { return DK <= 96 && DV <= 32 ? 4 : DK + DV <= 160 ? 3 : 0; }      // (0: two CTAs come by themselves)
+template <int DK, int DV, bool VK> constexpr int prefill_ctas() { return DK <= 96 && DV <= 32 ? 4 : DK + DV <= 160 ? 3 : DK + DV == 256 && !VK ? 2 : 0; }      // (0: two CTAs come by themselves)
 
 template <int DK, int DV, bool VK>
-__global__ void __launch_bounds__(128, prefill_ctas<DK, DV>())
+__global__ void __launch_bounds__(128, prefill_ctas<DK, DV, VK>())
 attn_biased_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __nv_bfloat16* __restrict__ kpages,
                            const __nv_bfloat16* __restrict__ vpages, const int* __restrict__ block_table, int max_blocks,
-                           const int* __restrict__ positions, const int* __restrict__ cu_tokens, int B, const float* __restrict__ rel,
+                           const int* __restrict__ positions, const int* __restrict__ cu_tokens, int B, const __grid_constant__ VmTiles tiles, const float* __restrict__ rel,
                            const int* __restrict__ bucket_of, int far, int rel_rows, __nv_bfloat16* __restrict__ out, int H, int Hkv,
                            float scale_log2, int window, int keep_first, int chunk, int n_pages, const float* __restrict__ sink, const float* __restrict__ slopes,
                            int* __restrict__ err) {
@@ -64,16 +67,10 @@ attn_biased_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride
     const bool biased = rel != nullptr, sloped = slopes != nullptr;
     const bool direct = biased && far + 1 <= DIRECT_TABLE_MAX;
 
-    // ---- which BM tokens of which sequence (the last tiles of a sequence see the most keys: they are started first)
-    int tile = gridDim.x - 1 - blockIdx.x, seq = 0, t0 = 0, n_rows = 0;
-    for (; seq < B; ++seq) {
-        const int a = cu_tokens[seq], b = cu_tokens[seq + 1];
-        const int nt = (b - a + BM - 1) / BM;
-        if (tile < nt) { t0 = a + tile * BM; n_rows = min(BM, b - t0); break; }
-        tile -= nt;
-    }
-    if (seq >= B) return;
-    const int h = blockIdx.y, hk = h / (H / Hkv);
+    // ---- which BM tokens of which sequence, and which head
+    int seq, t0, n_rows, h;
+    if (!vm_tile_of(tiles, cu_tokens, B, BM, seq, t0, n_rows, h)) return;
+    const int hk = h / (H / Hkv);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int pos0 = positions[t0];
     const int hi = pos0 + n_rows - 1;
@@ -94,9 +91,15 @@ attn_biased_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride
         cp_async16_zfill(sQ + r * KP + ch * 8, q + (size_t)(t0 + (r < n_rows ? r : 0)) * q_row_stride + (size_t)h * DK + ch * 8, r < n_rows);
     }
     auto block_of = [&](int step) { return step < kept_blocks ? step : blk_lo + (step - kept_blocks); };
-    auto load_kv = [&](int step, int buf) {
+    // a page is asked for a step ahead of its copies (not by the widest heads, whose registers are taken: keys and values of 128, one prompt of 512 tokens, 16
+    // heads 18.5 us with it, 16.8 without)
+    constexpr bool AHEAD = DK + DV <= 160;
+    auto page_of = [&](int step) {
         const int blk = block_of(step);
-        int page = (blk < max_blocks) ? table[blk] : -1;
+        return step < n_steps && blk < max_blocks ? table[blk] : -1;
+    };
+    auto load_kv = [&](int step, int page, int buf) {
+        const int blk = block_of(step);
         bool ok = (page >= 0 && page < n_pages);
         if (!ok) { if (tid == 0 && err) atomicExch(err, VM_ERRWORD_CACHE_READ); page = 0; }
         const int live = ok ? hi - blk * BN + 1 : 0;       // rows behind the tile's last token hold nothing yet: zeros
@@ -116,8 +119,9 @@ attn_biased_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride
                 cp_async16_zfill(vs + r * VP + ch * 8, vg + r * DV + ch * 8, r < live);
             }
     };
-    load_kv(0, 0);
+    load_kv(0, page_of(0), 0);
     vm_cp_async_commit();
+    int page_next = AHEAD ? page_of(1) : -1;
 
     // ---- per-thread state: rows g and g + 8 of the warp's 16 rows
     const int g = lane >> 2, t4 = lane & 3;
@@ -137,8 +141,9 @@ attn_biased_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride
         const int blk = block_of(step);
         vm_cp_async_wait_all();
         __syncthreads();          // the block is here, and everyone is done with the other buffer
-        if (step + 1 < n_steps) load_kv(step + 1, buf ^ 1);
+        if (step + 1 < n_steps) load_kv(step + 1, AHEAD ? page_next : page_of(step + 1), buf ^ 1);
         vm_cp_async_commit();
+        if (AHEAD) page_next = page_of(step + 2);
         if (step == 0) {
 #pragma unroll
             for (int kk = 0; kk < DK / 16; ++kk)
@@ -259,7 +264,7 @@ attn_biased_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride
 
 template <int DK, int DV, bool VK>
 int launch_biased_prefill(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
-                          const int* positions, const int* cu_tokens, int B, int n_tiles, const float* rel, const int* bucket_of, int far,
+                          const int* positions, const int* cu_tokens, int B, const VmTiles& tiles, int n_tiles, const float* rel, const int* bucket_of, int far,
                           int rel_rows, void* out, int H, int Hkv, float scale, int window, int keep_first, int chunk, int n_pages, const float* sink, const float* slopes,
                           int* err, cudaStream_t stream) {
     const int table = rel ? (far + 1 <= DIRECT_TABLE_MAX ? far + 1 : rel_rows) : 0;
@@ -272,9 +277,10 @@ int launch_biased_prefill(const void* q, int q_row_stride, const void* kpages, c
         if (e != cudaSuccess) return (int)e;
         raised = smem;
     }
+    // (not as a programmatic dependent: CTAs that start while the kernel in front still holds some SMs are not dealt out in turn)
     attn_biased_prefill_kernel<DK, DV, VK><<<dim3(n_tiles, H), 128, smem, stream>>>(
         (const __nv_bfloat16*)q, q_row_stride, (const __nv_bfloat16*)kpages, (const __nv_bfloat16*)vpages, block_table, max_blocks, positions,
-        cu_tokens, B, rel, bucket_of, far, rel_rows, (__nv_bfloat16*)out, H, Hkv, scale * 1.4426950408889634f, window, keep_first, chunk, n_pages, sink,
+        cu_tokens, B, tiles, rel, bucket_of, far, rel_rows, (__nv_bfloat16*)out, H, Hkv, scale * 1.4426950408889634f, window, keep_first, chunk, n_pages, sink,
         slopes, err);
     return vm_launch_status();
 }
@@ -443,8 +449,9 @@ VM_API int vm_attention_biased_prefill_bf16(const void* q, int q_row_stride, con
 // The same with a sink (float32 [H], null: none; exp(sink[h]) joins head h's denominator), slopes (float32 [H], null: none; slopes[h] (i - j)
 // comes off the score), a chunked mask (chunk > 0) and, with vpages == kpages and
 // v_row_stride == Dk, values that are the first Dv values of the key rows (sizes: vm_attention_sink_prefill_fits).
-VM_API int vm_attention_sink_prefill_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
-                                          int max_blocks, const int* positions, const int* cu_tokens, int B, int n_tiles, const float* rel,
+// host_cu_tokens: the same offsets as cu_tokens on the host (the tiles are then dealt out by their length), or null
+VM_API int vm_attention_sink_prefill_seqs_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
+                                          int max_blocks, const int* positions, const int* cu_tokens, const int* host_cu_tokens, int B, int n_tiles, const float* rel,
                                           const int* bucket_of, int far, int rel_rows, const float* sink, const float* slopes, int v_row_stride, void* out, int H, int Hkv,
                                           int Dk, int Dv, float scale, int window, int keep_first, int chunk, int n_pages, int* err, cudaStream_t stream) {
     if (n_tiles <= 0 || B <= 0) return 0;
@@ -452,9 +459,10 @@ VM_API int vm_attention_sink_prefill_bf16(const void* q, int q_row_stride, const
     if ((rel != nullptr) != (bucket_of != nullptr) || (rel && (far < 0 || rel_rows <= 0))) return VM_ERR_BAD_ARG;
     const bool in_keys = vpages == kpages && v_row_stride == Dk && (Dv < Dk || (Dk == 128 && Dv == 128));
     if (!in_keys && v_row_stride != 0 && v_row_stride != Dv) return VM_ERR_UNSUPPORTED;
+    const VmTiles tiles = vm_list_tiles(host_cu_tokens, B, BM, n_tiles);
 #define VM_BP(K, V, IN)                                                                                                                        \
     if (Dk == K && Dv == V && in_keys == IN)                                                                                                   \
-        return launch_biased_prefill<K, V, IN>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, cu_tokens, B, n_tiles, rel, \
+        return launch_biased_prefill<K, V, IN>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, cu_tokens, B, tiles, n_tiles, rel, \
                                                bucket_of, far, rel_rows, out, H, Hkv, scale, window, keep_first, chunk, n_pages, sink, slopes, err, stream);
     VM_BP(32, 16, false) VM_BP(32, 32, false) VM_BP(32, 64, false) VM_BP(32, 128, false)
     VM_BP(64, 16, false) VM_BP(64, 32, false) VM_BP(64, 64, false) VM_BP(64, 128, false)
@@ -466,6 +474,14 @@ VM_API int vm_attention_sink_prefill_bf16(const void* q, int q_row_stride, const
     VM_BP(128, 128, true) VM_BP(144, 128, true) VM_BP(160, 128, true) VM_BP(192, 128, true)
 #undef VM_BP
     return VM_ERR_UNSUPPORTED;
+}
+
+VM_API int vm_attention_sink_prefill_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
+                                          int max_blocks, const int* positions, const int* cu_tokens, int B, int n_tiles, const float* rel,
+                                          const int* bucket_of, int far, int rel_rows, const float* sink, const float* slopes, int v_row_stride, void* out, int H, int Hkv,
+                                          int Dk, int Dv, float scale, int window, int keep_first, int chunk, int n_pages, int* err, cudaStream_t stream) {
+    return vm_attention_sink_prefill_seqs_bf16(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, cu_tokens, nullptr, B, n_tiles, rel, bucket_of,
+                                               far, rel_rows, sink, slopes, v_row_stride, out, H, Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, err, stream);
 }
 
 // one new token per sequence (token s belongs to sequence s); any Dk up to 1,024, Dv up to 256

@@ -10,9 +10,14 @@
 // cp.async into double-buffered shared memory; Q K^T and P V run on mma.sync m16n8k16 (bf16 in, float32
 // accumulate); at the end the groups' partial results are merged through shared memory.
 //
+// What bounds it is the SM with the most key blocks, then the chain of a block (products, maximum, exponentials, products): so the tiles are dealt out by their
+// length (tile_order.cuh), a block has one barrier, and a page's number is asked for a step ahead of its copies.  Measured before / after, heads of 64: 9 heads, one
+// prompt of 512 tokens 10.0 / 9.6 us, 1,000 16.4 / 15.5, 1,536 32.2 / 23.6, eight of 512 21.4 / 16.9, sixteen of 40 to 295 11.8 / 9.4, two of 700 17.7 / 13.6;
+// 15 heads, sixteen of 64 to 1,024 71.9 / 53.4; 16 heads of 128, 2,048 tokens 112 / 67.
+//
 // Sizes: head size D in {16, 32, ..., 128} (template), any head count and group size; the sequences of a
 // step may have any lengths.  Other head sizes are refused (the caller falls back to the generic kernel).
-#include "common.cuh"
+#include "tile_order.cuh"
 
 namespace {
 
@@ -53,10 +58,10 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
 }
 
 template <int D, int NG>
-__global__ void __launch_bounds__(128 * NG)
+__global__ void __launch_bounds__(128 * NG, D <= 64 && NG <= 2 ? 4 / NG : 1)      // (128 registers: as many CTAs an SM as its shared memory leaves)
 attn_prefill_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __nv_bfloat16* __restrict__ kpages,
                         const __nv_bfloat16* __restrict__ vpages, const int* __restrict__ block_table, int max_blocks,
-                        const int* __restrict__ positions, const int* __restrict__ cu_tokens, int B,
+                        const int* __restrict__ positions, const int* __restrict__ cu_tokens, int B, const __grid_constant__ VmTiles tiles,
                         __nv_bfloat16* __restrict__ out, int H, int Hkv, float scale_log2, int window, int n_pages,
                         int* __restrict__ err) {
     constexpr int DP = D + 8;                  // padded row: 2D+16 bytes, an odd number of 16-byte units -> no ldmatrix conflicts
@@ -67,17 +72,10 @@ attn_prefill_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, c
     __nv_bfloat16* sV = sK + 2 * NG * BN * DP;                           // [2][NG][BN][DP]
     constexpr int THREADS = 128 * NG;
 
-    // ---- which 64 tokens of which sequence
-    // (the last tiles of a sequence see the most keys: they are started first)
-    int tile = gridDim.x - 1 - blockIdx.x, seq = 0, t0 = 0, n_rows = 0;
-    for (; seq < B; ++seq) {
-        const int a = cu_tokens[seq], b = cu_tokens[seq + 1];
-        const int nt = (b - a + BM - 1) / BM;
-        if (tile < nt) { t0 = a + tile * BM; n_rows = min(BM, b - t0); break; }
-        tile -= nt;
-    }
-    if (seq >= B) return;
-    const int h = blockIdx.y, hk = h / (H / Hkv);
+    // ---- which 64 tokens of which sequence, and which head
+    int seq, t0, n_rows, h;
+    if (!vm_tile_of(tiles, cu_tokens, B, BM, seq, t0, n_rows, h)) return;
+    const int hk = h / (H / Hkv);
     const int tid = threadIdx.x, lane = tid & 31;
     const int grp = tid >> 7, warp = (tid >> 5) & 3;       // group of four warps; warp inside its group
     const int pos0 = positions[t0];
@@ -92,12 +90,20 @@ attn_prefill_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, c
         const int r = c / CH, ch = c - r * CH;
         cp_async16(sQ + r * DP + ch * 8, q + (size_t)(t0 + (r < n_rows ? r : 0)) * q_row_stride + (size_t)h * D + ch * 8, r < n_rows);
     }
-    auto load_kv = [&](int step, int buf) {                // the NG blocks of one step, by all threads
+    // the pages of a step's NG blocks, asked for a step ahead of their copies
+    int pages[NG];
+    auto ask_pages = [&](int step) {
 #pragma unroll
         for (int gi = 0; gi < NG; ++gi) {
             const int blk = blk_lo + step * NG + gi;
-            if (blk > blk_hi) break;
-            int page = (blk < max_blocks) ? table[blk] : -1;
+            pages[gi] = (blk <= blk_hi && blk < max_blocks) ? table[blk] : -1;
+        }
+    };
+    auto load_kv = [&](int step, int buf) {                // the NG blocks of one step, by all threads
+#pragma unroll
+        for (int gi = 0; gi < NG; ++gi) {
+            if (blk_lo + step * NG + gi > blk_hi) break;
+            int page = pages[gi];
             const bool ok = (page >= 0 && page < n_pages);
             if (!ok) { if (tid == 0 && err) atomicExch(err, 3); page = 0; }
             const __nv_bfloat16* kg = kpages + (size_t)page * page_stride + (size_t)hk * BN * D;
@@ -112,8 +118,10 @@ attn_prefill_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, c
         }
     };
     const int n_steps = (blk_hi - blk_lo + NG) / NG;
+    ask_pages(0);
     load_kv(0, 0);
     cp_async_commit();
+    ask_pages(1);
 
     // ---- per-thread state: rows g and g+8 of the warp's 16 rows
     const int g = lane >> 2, t4 = lane & 3;
@@ -131,10 +139,11 @@ attn_prefill_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, c
     for (int step = 0; step < n_steps; ++step) {
         const int buf = step & 1;
         const int blk = blk_lo + step * NG + grp;          // this group's block of the step
+        cp_async_wait<0>();
+        __syncthreads();          // the blocks are here, and everyone is done with the other buffer
         if (step + 1 < n_steps) load_kv(step + 1, buf ^ 1);
         cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
+        ask_pages(step + 2);
         if (!q_loaded) {
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk)
@@ -211,7 +220,6 @@ attn_prefill_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, c
                 }
             }
         }
-        __syncthreads();          // everyone is done with `buf` before the next iteration's prefetch overwrites it
     }
     cp_async_wait<0>();
 
@@ -267,7 +275,7 @@ attn_prefill_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, c
 
 template <int D, int NG>
 int launch_prefill_ng(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
-                      int max_blocks, const int* positions, const int* cu_tokens, int B, int n_tiles, void* out, int H, int Hkv,
+                      int max_blocks, const int* positions, const int* cu_tokens, int B, const VmTiles& tiles, int n_tiles, void* out, int H, int Hkv,
                       float scale, int window, int n_pages, int* err, cudaStream_t stream) {
     constexpr int DP = D + 8;
     size_t smem = (size_t)(BM + 4 * NG * BN) * DP * sizeof(__nv_bfloat16);
@@ -280,24 +288,25 @@ int launch_prefill_ng(const void* q, int q_row_stride, const void* kpages, const
         configured = true;
     }
     dim3 grid(n_tiles, H);
+    // (not as a programmatic dependent: CTAs that start while the kernel in front still holds some SMs are not dealt out in turn)
     attn_prefill_mma_kernel<D, NG><<<grid, 128 * NG, smem, stream>>>(
         (const __nv_bfloat16*)q, q_row_stride, (const __nv_bfloat16*)kpages, (const __nv_bfloat16*)vpages, block_table,
-        max_blocks, positions, cu_tokens, B, (__nv_bfloat16*)out, H, Hkv, scale * 1.4426950408889634f, window, n_pages, err);
+        max_blocks, positions, cu_tokens, B, tiles, (__nv_bfloat16*)out, H, Hkv, scale * 1.4426950408889634f, window, n_pages, err);
     return vm_launch_status();
 }
 
 // `long_tiles`: some tile of the step sees many key blocks (a long prompt): split its blocks over two warp groups
 template <int D>
 int launch_prefill(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
-                   int max_blocks, const int* positions, const int* cu_tokens, int B, int n_tiles, void* out, int H, int Hkv,
+                   int max_blocks, const int* positions, const int* cu_tokens, int B, const VmTiles& tiles, int n_tiles, void* out, int H, int Hkv,
                    float scale, int window, int n_pages, int* err, int groups, cudaStream_t stream) {
     if (groups >= 4 && D <= 64)
-        return launch_prefill_ng<D, 4>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, cu_tokens, B, n_tiles,
+        return launch_prefill_ng<D, 4>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, cu_tokens, B, tiles, n_tiles,
                                        out, H, Hkv, scale, window, n_pages, err, stream);
     if (groups >= 2)
-        return launch_prefill_ng<D, 2>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, cu_tokens, B, n_tiles,
+        return launch_prefill_ng<D, 2>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, cu_tokens, B, tiles, n_tiles,
                                        out, H, Hkv, scale, window, n_pages, err, stream);
-    return launch_prefill_ng<D, 1>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, cu_tokens, B, n_tiles,
+    return launch_prefill_ng<D, 1>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, cu_tokens, B, tiles, n_tiles,
                                    out, H, Hkv, scale, window, n_pages, err, stream);
 }
 
@@ -305,20 +314,30 @@ int launch_prefill(const void* q, int q_row_stride, const void* kpages, const vo
 
 // n_tiles = sum over the step's sequences of ceil(new tokens / 64), computed by the host.
 // groups: warp groups (1, 2 or 4) that share a tile's key blocks; more for steps whose tiles see many keys.
-VM_API int vm_attention_prefill_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages,
+// host_cu_tokens: the same offsets as cu_tokens on the host (the tiles are then dealt out by their length), or null.
+VM_API int vm_attention_prefill_seqs_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages,
                                      const int* block_table, int max_blocks, const int* positions, const int* cu_tokens,
-                                     int B, int n_tiles, void* out, int H, int Hkv, int D, float scale, int window,
+                                     const int* host_cu_tokens, int B, int n_tiles, void* out, int H, int Hkv, int D, float scale, int window,
                                      int n_pages, int* err, int groups, cudaStream_t stream) {
     if (n_tiles <= 0 || B <= 0) return 0;
     if (H <= 0 || Hkv <= 0 || H % Hkv != 0 || (q_row_stride % 8) != 0) return VM_ERR_UNSUPPORTED;
+    const VmTiles tiles = vm_list_tiles(host_cu_tokens, B, BM, n_tiles);
 #define VM_PREFILL_CASE(DD)                                                                                          \
     case DD:                                                                                                         \
         return launch_prefill<DD>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, cu_tokens, B,  \
-                                  n_tiles, out, H, Hkv, scale, window, n_pages, err, groups, stream);
+                                  tiles, n_tiles, out, H, Hkv, scale, window, n_pages, err, groups, stream);
     switch (D) {
         VM_PREFILL_CASE(16) VM_PREFILL_CASE(32) VM_PREFILL_CASE(48) VM_PREFILL_CASE(64)
         VM_PREFILL_CASE(80) VM_PREFILL_CASE(96) VM_PREFILL_CASE(112) VM_PREFILL_CASE(128)
         default: return VM_ERR_UNSUPPORTED;
     }
 #undef VM_PREFILL_CASE
+}
+
+VM_API int vm_attention_prefill_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages,
+                                     const int* block_table, int max_blocks, const int* positions, const int* cu_tokens,
+                                     int B, int n_tiles, void* out, int H, int Hkv, int D, float scale, int window,
+                                     int n_pages, int* err, int groups, cudaStream_t stream) {
+    return vm_attention_prefill_seqs_bf16(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, cu_tokens, nullptr, B, n_tiles, out, H, Hkv, D,
+                                          scale, window, n_pages, err, groups, stream);
 }

@@ -437,6 +437,7 @@ constexpr int TC_ATTENTION_MIN_BLOCKS = 20;   // head size 64: the tcgen05 prefi
 constexpr int TC_ATTENTION_CTAS_PER_SM = 3;   // CTAs of that kernel an SM holds at once (registers and shared memory)
 constexpr int WS_ATTENTION_MANY_BLOCKS = 16;  // the same for steps of many long tiles
 constexpr int WS_ATTENTION_MEAN_BLOCKS = 10;  // ... that see this many key blocks of new tokens on average
+constexpr int WS_ATTENTION_MEAN_BLOCKS_DEALT = 12;      // ... where the kernel they are taken from deals its tiles out by length
 int WS_ATTENTION_MIN_BLOCKS = 32;             // head size 64: the warp-specialised tcgen05 attention when a tile may see this many key blocks
 
 int* decode_counters() {
@@ -497,17 +498,28 @@ void attention(StepContext& ctx, const void* q, int q_row_stride, const KVView& 
         int most_blocks = kv.table_width;
         if (window > 0) most_blocks = std::min(most_blocks, window / VM_PAGE_TOKENS + 2);
         long long tiles128 = 0, tiles64 = 0, blocks128 = 0;      // blocks128: over the tiles of 128, the key blocks of their sequence's new tokens
+        int newest = 0;
         for (int b = 0; b < ctx.B; ++b) {
             const int n = ctx.host_cu_tokens[b + 1] - ctx.host_cu_tokens[b];
             tiles128 += (n + 127) / 128;
             tiles64 += (n + 63) / 64;
             blocks128 += static_cast<long long>((n + 127) / 128) * std::min(most_blocks, (n + 63) / 64);
+            newest = std::max(newest, (n + 63) / 64);
         }
-        // (many tiles of middling length keep that kernel's CTAs busy too: 15 heads, four prompts of 1,024 tokens 43 us against 51 us for the mma.sync kernel, eight of
-        //  800 59 / 60; 32 heads, three of 1,024 61 / 71; one of 1,024 and 9 heads 22 / 17, eight of 512 33 / 22.  Short prompts beside long ones do not, each
-        //  pays for a CTA's set-up: 15 heads, one of 1,024 beside sixteen of 100 42 / 31, eight of 800 beside 32 of 60 72 / 66)
-        const bool many = most_blocks >= WS_ATTENTION_MANY_BLOCKS && tiles128 * H >= 3ll * sm_count() && blocks128 >= WS_ATTENTION_MEAN_BLOCKS * tiles128;
-        if (D == 64 && (most_blocks >= WS_ATTENTION_MIN_BLOCKS || many) && ctx.err != nullptr) {
+        const long long items = tiles64 * H, sms = sm_count();
+        // Prompts from their start (a table is as wide as its sequences' blocks, rounded up to a power of two) whose tiles of 64 rows fill the GPU go to the mma.sync
+        // kernel below, which deals them out by their length, unless the sequences are long on average.  Measured, mma.sync / warp-specialised / tcgen05: 9 heads, one
+        // prompt of 1,536 tokens 23.6 / 26.2 / 23.8 us, of 2,048 30.2 / 31.6 / 37.7, of 3,000 52.6 / 50.3 / 57.5; 15 heads, 2,048 40.5 / 38.9 / 46, sixteen of 64 to 1,024
+        // 53 / 71 / 86; 16 heads, 1,400 + 2,000 52.8 / 53.4 / 67.  Behind a cached prefix every tile is long, and where there are fewer tiles than that a tile's keys
+        // are dealt out to several CTAs: by the table's width, as far as the two kernels below go.
+        const bool dealt = D == 64 && kv.table_width < 2 * newest && 5 * items > 7 * sms;
+        // (many tiles of middling length keep the warp-specialised kernel's CTAs busy: 15 heads, four prompts of 1,024 tokens 43 us; 32 heads, three of 1,024 61 / 55 for
+        //  the mma.sync kernel, four of 1,000 to 3,000 222 / 271.  Short prompts beside long ones do not, each pays for a CTA's set-up)
+        const bool many = most_blocks >= WS_ATTENTION_MANY_BLOCKS && tiles128 * H >= 3 * sms &&
+                          blocks128 >= (dealt ? WS_ATTENTION_MEAN_BLOCKS_DEALT : WS_ATTENTION_MEAN_BLOCKS) * tiles128;
+        const bool long_ones = dealt ? blocks128 >= WS_ATTENTION_MIN_BLOCKS * tiles128 : most_blocks >= WS_ATTENTION_MIN_BLOCKS;
+        const bool ws = many || long_ones;
+        if (D == 64 && ws && ctx.err != nullptr) {
             // the longest prompts: softmax warps, a copy warp and product warps, clusters dealt out to pairs of tile groups
             // (measured, 9 heads: 4,096 tokens 78 us against 88 us for the kernel below, 8,192: 224 / 262; 2,048: 32 / 33;
             //  2,560: 37 / 48, 3,072: 51 / 58, 1,536: 27 / 24, 1,024: 22 / 18: every CTA pays for its set-up and its cluster's exchange once, whatever its share of the keys;
@@ -519,8 +531,8 @@ void attention(StepContext& ctx, const void* q, int q_row_stride, const KVView& 
                   "attention_prefill_ws_bf16", s);
             return;
         }
-        if (D == 64 && most_blocks >= TC_ATTENTION_MIN_BLOCKS && ctx.err != nullptr) {
-            // long prompts: the tcgen05 kernel, a tile's key blocks dealt out to as many CTAs (2 to 4) as still fit the GPU at once
+        if (D == 64 && !dealt && most_blocks >= TC_ATTENTION_MIN_BLOCKS && ctx.err != nullptr) {
+            // long prompts of few heads, new tokens behind a prefix: the tcgen05 kernel, a tile's key blocks dealt out to as many CTAs (2 to 4) as still fit the GPU at once
             // (measured, 9 heads: 1,536 tokens 23.7 us against 32.2 us for the mma.sync kernel; 2,048: 33.6 / 39.4; 4,096: 89.9 / 123.8;
             //  1,024: 17.6 / 16.6, hence the threshold)
             const long long slots = static_cast<long long>(sm_count()) * TC_ATTENTION_CTAS_PER_SM;
@@ -537,18 +549,20 @@ void attention(StepContext& ctx, const void* q, int q_row_stride, const KVView& 
             // (measured against the kernel below, 16 heads: 30 tokens 5.3 / 5.4 us, 300 11.1 / 12.0, 2,048 90 / 115, 4,096 271 / 357, in a window of 512
             // 81 / 98; eight of 512 52 / 61; 32 heads, 1,024 tokens 53 / 66)
             Timed t("attention_prefill_bf16", s);
-            check(vm_attention_sink_prefill_bf16(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, ctx.cu_tokens, ctx.B,
+            check(vm_attention_sink_prefill_seqs_bf16(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, ctx.cu_tokens, ctx.host_cu_tokens, ctx.B,
                                                  static_cast<int>(tiles64), nullptr, nullptr, 0, 0, nullptr, nullptr, D, out, H, Hkv, D, D, scale, window, 0, 0,
                                                  kv.n_pages, ctx.err, s),
                   "attention_prefill_bf16", s);
             return;
         }
-        // two groups of warps share a tile's keys where the tiles are long and too few to fill the GPU: two an SM where tiles may see 1,024 keys and more, one an SM
-        // above 512 (measured, with two groups / with one: 9 heads of 64, one prompt of 2,048 tokens 40.0 / 43.8 us, of 1,000 16.4 / 19.5, of 512 10.1 / 11.3, of 300
-        // 7.6 / 7.8, two of 700 18.0 / 17.6, sixteen of 40 to 295 16.4 / 12.2, eight of 512 25.1 / 22.2; 16 heads of 128, one of 512 15.2 / 18.3, of 700 26 / 29)
-        const int groups = most_blocks >= 8 && tiles64 * H <= (most_blocks >= 16 ? 2ll : 1ll) * sm_count() ? 2 : 1;
+        // two groups of warps share a tile's keys where the tiles are long and few: up to 3.5 an SM of those dealt out by their length, whose longest
+        // are the longest chains (one group / two: 9 heads of 64, one of 512 10.3 / 9.6 us, of 1,000 17.5 / 15.5, of 2,048 34.0 / 30.2, of 1,024 beside sixteen of
+        // 100 20.8 / 18.6; 15 heads, 2,048 50.0 / 40.5; but eight of 512 16.9 / 19.6, 32 heads, 2,048 70 / 82); elsewhere two an SM where tiles may see 1,024 keys and
+        // more, one an SM above 512 (16 heads of 128, one of 512 18.3 / 15.2, 2,048 67 / 87)
+        const bool few = dealt ? 2 * items <= 7 * sms : items <= (most_blocks >= 16 ? 2ll : 1ll) * sms;
+        const int groups = most_blocks >= 8 && few ? 2 : 1;
         Timed t("attention_prefill_bf16", s);
-        check(vm_attention_prefill_bf16(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, ctx.cu_tokens, ctx.B,
+        check(vm_attention_prefill_seqs_bf16(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, ctx.cu_tokens, ctx.host_cu_tokens, ctx.B,
                                         static_cast<int>(tiles64), out, H, Hkv, D, scale, window, kv.n_pages, ctx.err, groups, s),
               "attention_prefill_bf16", s);
         return;
@@ -589,7 +603,7 @@ void attention_biased(StepContext& ctx, const void* q, int q_row_stride, const K
         long long tiles = 0;
         for (int b = 0; b < ctx.B; ++b) tiles += (ctx.host_cu_tokens[b + 1] - ctx.host_cu_tokens[b] + 63) / 64;
         Timed t("attention_biased_prefill_bf16", s);
-        check(vm_attention_sink_prefill_bf16(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, ctx.cu_tokens, ctx.B,
+        check(vm_attention_sink_prefill_seqs_bf16(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, ctx.cu_tokens, ctx.host_cu_tokens, ctx.B,
                                              static_cast<int>(tiles), mask.rel, mask.bucket_of, mask.far, mask.rows, mask.sink, mask.slopes, mask.v_row_stride, out, H,
                                              Hkv, Dk, Dv, scale, mask.window, mask.keep_first, mask.chunk, kv.n_pages, ctx.err, s),
               "attention_biased_prefill_bf16", s);

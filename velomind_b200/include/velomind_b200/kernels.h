@@ -194,6 +194,10 @@ int vm_attention_sink_prefill_bf16(const void* q, int q_row_stride, const void* 
                                    const int* positions, const int* cu_tokens, int B, int n_tiles, const float* rel, const int* bucket_of, int far,
                                    int rel_rows, const float* sink, const float* slopes, int v_row_stride, void* out, int H, int Hkv, int Dk, int Dv, float scale, int window,
                                    int keep_first, int chunk, int n_pages, int* err, cudaStream_t stream);
+int vm_attention_sink_prefill_seqs_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
+                                   const int* positions, const int* cu_tokens, const int* host_cu_tokens, int B, int n_tiles, const float* rel, const int* bucket_of, int far,
+                                   int rel_rows, const float* sink, const float* slopes, int v_row_stride, void* out, int H, int Hkv, int Dk, int Dv, float scale, int window,
+                                   int keep_first, int chunk, int n_pages, int* err, cudaStream_t stream);
 int vm_attention_sink_decode_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
                                   const int* positions, const float* rel, const int* bucket_of, int far, const float* sink, const float* slopes, int v_row_stride, void* out,
                                   int B, int H, int Hkv, int Dk, int Dv, float scale, int window, int keep_first, int chunk, int n_pages, int* err,
@@ -274,6 +278,10 @@ int vm_attention_generic_seqs(const void* q, int q_row_stride, const void* kpage
                               int n_pages, int act_dtype, int* err, int n_seqs, cudaStream_t stream);      // n_seqs as in vm_attention_sink_generic_seqs
 int vm_attention_prefill_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
                               int max_blocks, const int* positions, const int* cu_tokens, int B, int n_tiles, void* out, int H,
+                              int Hkv, int D, float scale, int window, int n_pages, int* err, int groups, cudaStream_t stream);
+// the same with the offsets on the host too: the tiles are dealt out by their length
+int vm_attention_prefill_seqs_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
+                              int max_blocks, const int* positions, const int* cu_tokens, const int* host_cu_tokens, int B, int n_tiles, void* out, int H,
                               int Hkv, int D, float scale, int window, int n_pages, int* err, int groups, cudaStream_t stream);
 int vm_attention_prefill_tc_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
                                  int max_blocks, const int* positions, const int* cu_tokens, int B, int n_tiles, void* out, int H,
