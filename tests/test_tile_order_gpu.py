@@ -18,8 +18,8 @@ def _i(v):
 
 # one tile; fewer items than SMs; an odd last wave that is not full; sequences without new tokens between others; rows at the edges of a tile; more tiles than the
 # list holds (the walk over the sequences)
-@pytest.mark.parametrize("new,H,Hkv", [([1], 1, 1), ([300], 9, 3), ([2048], 9, 3), ([64, 0, 65, 63, 0, 700], 15, 5), ([130 + 54 * i for i in range(8)], 16, 4), ([5] * 481, 2, 1),
-                                       ([64] * 480, 1, 1)])
+@pytest.mark.parametrize("new,H,Hkv", [([1], 1, 1), ([300], 9, 3), ([2048], 9, 3), ([64, 0, 65, 63, 0, 700], 15, 5), ([130 + 54 * i for i in range(8)], 16, 4), ([5] * 257, 2, 1),
+                                       ([64] * 256, 1, 1), ([64 * 256], 1, 1), ([64 * 256 + 1], 1, 1)])
 def test_same_bits_as_along_the_prompts(new, H, Hkv, D=64):
     from velomind_b200.kernels.library import library
     lib = library()

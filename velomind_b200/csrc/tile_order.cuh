@@ -3,17 +3,16 @@
 // The tiles of a causal prompt see one key block, two, three ...: dealt out in their order along the prompt, one SM gets long tiles only and another short ones
 // (2,048 tokens, 9 heads in tiles of 64 rows: 288 CTAs, all resident, 12 to 52 key blocks an SM, 33 on average).  So the host lists a step's tiles by their number
 // of blocks, the longest first (shape only: new tokens per sequence), and the CTAs, which the GPU deals out to its SMs in turn, take them forwards and
-// backwards from wave to wave.  The list rides along as a kernel argument, so that no CTA walks over the sequences' offsets (a chain of loads) either.  Steps of more
-// tiles than the list holds keep that walk: they are many waves long.
+// backwards from wave to wave.  The list rides along as a kernel argument, two bytes a tile, so that no CTA walks over the sequences' offsets (a chain of loads)
+// either.  Steps of more tiles than it holds keep that walk and take a prompt's last tiles first: they are many waves long.
 #pragma once
 #include "common.cuh"
 
-constexpr int VM_TILES_LISTED = 480;                     // (the arguments of a kernel stay below 4 KB)
+constexpr int VM_TILES_LISTED = 256;
 
 struct VmTiles {
     int n, sms;                                          // n = 0: not listed
-    unsigned at[VM_TILES_LISTED];                        // first token | (rows - 1) << 26
-    unsigned short seq[VM_TILES_LISTED];
+    unsigned short where[VM_TILES_LISTED];               // sequence << 8 | tile of the sequence
 };
 
 // host_cu_tokens [B + 1] on the host, or null: no list
@@ -21,7 +20,7 @@ static inline VmTiles vm_list_tiles(const int* host_cu_tokens, int B, int rows, 
     VmTiles t;
     t.n = 0;
     t.sms = vm_sm_count();
-    if (host_cu_tokens == nullptr || n_tiles > VM_TILES_LISTED || t.sms <= 0 || B > 65535 || rows > 64 || host_cu_tokens[B] >= 1 << 26) return t;
+    if (host_cu_tokens == nullptr || n_tiles > VM_TILES_LISTED || t.sms <= 0 || B > 256) return t;
     int place[VM_TILES_LISTED + 1] = {}, total = 0;      // tiles of each length, then where the next of that length goes
     for (int b = 0; b < B; ++b) {
         const int k = (host_cu_tokens[b + 1] - host_cu_tokens[b] + rows - 1) / rows;
@@ -31,28 +30,22 @@ static inline VmTiles vm_list_tiles(const int* host_cu_tokens, int B, int rows, 
     }
     if (total != n_tiles) return t;
     for (int i = VM_TILES_LISTED, before = 0; i >= 0; --i) { const int here = place[i]; place[i] = before; before += here; }
-    for (int b = 0; b < B; ++b) {
-        const int a = host_cu_tokens[b], end = host_cu_tokens[b + 1];
-        for (int i = 0; a + i * rows < end; ++i) {
-            const int k = place[i]++, left = end - a - i * rows;
-            t.at[k] = (unsigned)(a + i * rows) | (unsigned)((left < rows ? left : rows) - 1) << 26;
-            t.seq[k] = (unsigned short)b;
-        }
-    }
+    for (int b = 0; b < B; ++b)
+        for (int i = 0; host_cu_tokens[b] + i * rows < host_cu_tokens[b + 1]; ++i) t.where[place[i]++] = (unsigned short)(b << 8 | i);
     t.n = n_tiles;
     return t;
 }
 
-// The tile and the head of this CTA of a grid (tiles, heads); false: none.  cu_tokens [B + 1] on the device (read without a list only).
+// The tile and the head of this CTA of a grid (tiles, heads); false: none.  cu_tokens [B + 1] on the device.
 __device__ __forceinline__ bool vm_tile_of(const VmTiles& tiles, const int* __restrict__ cu_tokens, int B, int rows, int& seq, int& t0, int& n_rows, int& head) {
     if (tiles.n > 0) {
         const int items = gridDim.x * gridDim.y, turn = blockIdx.y * gridDim.x + blockIdx.x, wave = turn / tiles.sms, first = wave * tiles.sms;
         const int item = wave & 1 ? first + min(tiles.sms, items - first) - 1 - (turn - first) : turn;
         const int k = item / gridDim.y;
         head = item - k * gridDim.y;
-        seq = tiles.seq[k];
-        t0 = (int)(tiles.at[k] & 0x3ffffffu);
-        n_rows = (int)(tiles.at[k] >> 26) + 1;
+        seq = tiles.where[k] >> 8;
+        t0 = cu_tokens[seq] + (tiles.where[k] & 255) * rows;
+        n_rows = min(rows, cu_tokens[seq + 1] - t0);
         return true;
     }
     int tile = gridDim.x - 1 - blockIdx.x;               // (the last tiles of a sequence see the most keys: they are started first)
