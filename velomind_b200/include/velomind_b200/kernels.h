@@ -257,6 +257,11 @@ int vm_rope_kv_write(void* qkv, const int* positions, const int* seq_of_token, c
                      int n_pages, int act_dtype, int* err, cudaStream_t stream);
 
 // ---- attention
+// ---- products_f32.cu: out[T, N] = x[T, K] W[N, K]^T in float32 for many rows (x rows ldx apart)
+int vm_products_f32_pays(int T, int N);      // 1 where it is faster than the library's product
+int vm_products_f32_fits(const void* x, long long ldx, const void* w, const void* out, int T, int K);
+int vm_products_f32(const float* x, long long ldx, const float* w, float* out, int T, int N, int K, cudaStream_t stream);
+
 // ---- skinny_f32.cu: out[T, N] = x[T, K] W[N, K]^T in float32 for up to eight rows
 int vm_skinny_f32_fits(const void* x, long long ldx, const void* w, int T, int K);
 int vm_skinny_f32(const float* x, long long ldx, const float* w, float* out, int T, int N, int K, cudaStream_t stream);
