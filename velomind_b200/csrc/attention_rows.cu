@@ -21,6 +21,10 @@
 namespace {
 
 constexpr int MAX_ROWS = 8;
+// Prompts that take attention_tiles_f32.cu: eight tokens a sequence and more, enough rows to fill the GPU, no long cached prefix (whose keys the warps here share)
+bool tiles_pay(int n_tokens, int n_seqs, int H, int max_blocks) {
+    return n_seqs > 0 && n_tokens >= 8 * n_seqs && (long long)n_tokens * H >= 2000 && (max_blocks == 1 || 16ll * max_blocks * n_seqs <= n_tokens);
+}
 constexpr int KEYS = 32;                 // keys of a warp's turn
 constexpr int SLICE = 64;                // columns of the keys in shared memory at a time
 template <typename T> constexpr int pitch() { return SLICE + 16 / (int)sizeof(T); }      // of a key row there: a lane's row starts 16 bytes further round the banks
@@ -183,7 +187,7 @@ attn_rows_kernel(const T* __restrict__ q, int q_row_stride, const T* __restrict_
                 const float use = top == -INFINITY ? 0.f : top;      // nothing seen so far: no factor changes anything
                 const float p = valid ? expf(x - use) : 0.f;
                 const float alpha = expf(m[r] - use);
-                l[r] = l[r] * alpha + vm_warp_sum(p);
+                l[r] = fmaf(l[r], alpha, vm_warp_sum(p));
 #pragma unroll
                 for (int i = 0; i < VP; ++i) { acc[r][i][0] *= alpha; acc[r][i][1] *= alpha; }
                 m[r] = top;
@@ -352,6 +356,9 @@ VM_API int vm_attention_rows(const void* q, int q_row_stride, const void* kpages
                              int keep_first, int chunk, int n_pages, int act_dtype, int* err, int n_seqs, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (!vm_attention_rows_fits(kpages, vpages, H, Hkv, Dk, Dv, v_stride)) return VM_ERR_UNSUPPORTED;
+    if (act_dtype == VM_F32 && tiles_pay(n_tokens, n_seqs, H, max_blocks) && vm_attention_tiles_f32_fits(kpages, vpages, H, Dk, Dv, v_stride))
+        return vm_attention_tiles_f32(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, rel, bucket_of, far, sink, slopes,
+                                      v_stride, out, n_tokens, H, Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, err, 0, stream);
     if (act_dtype == VM_F32)
         return dispatch_rows<float>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, seq_of_token, rel, bucket_of, far, out, n_tokens, H,
                                     Hkv, Dk, Dv, scale, window, keep_first, chunk, n_pages, sink, slopes, v_stride, err, n_seqs, stream);

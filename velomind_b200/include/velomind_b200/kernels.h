@@ -275,6 +275,12 @@ int vm_attention_rows(const void* q, int q_row_stride, const void* kpages, const
                       const int* positions, const int* seq_of_token, const float* rel, const int* bucket_of, int far, const float* sink,
                       const float* slopes, int v_stride, void* out, int n_tokens, int H, int Hkv, int Dk, int Dv, float scale, int window,
                       int keep_first, int chunk, int n_pages, int act_dtype, int* err, int n_seqs, cudaStream_t stream);
+// ---- attention_tiles_f32.cu: the same in float32, the same bits, for prompts (rows_per_warp: 2, 4, 8, or 0: by the step's shape)
+int vm_attention_tiles_f32_fits(const void* kpages, const void* vpages, int H, int Dk, int Dv, int v_stride);
+int vm_attention_tiles_f32(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks,
+                           const int* positions, const int* seq_of_token, const float* rel, const int* bucket_of, int far, const float* sink,
+                           const float* slopes, int v_stride, void* out, int n_tokens, int H, int Hkv, int Dk, int Dv, float scale, int window,
+                           int keep_first, int chunk, int n_pages, int* err, int rows_per_warp, cudaStream_t stream);
 int vm_attention_generic(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
                          int max_blocks, const int* positions, const int* seq_of_token, void* out, int n_tokens, int H, int Hkv,
                          int D, float scale, int window, int n_pages, int act_dtype, int* err, cudaStream_t stream);
