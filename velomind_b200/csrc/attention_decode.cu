@@ -21,7 +21,7 @@ constexpr int DEC_WARPS_WIDE = 10;
 using namespace vmad;
 
 template <int D, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32)
+__global__ void __launch_bounds__(WARPS * 32) __maxnreg__((WARPS == 10 ? (D <= 64 ? 136 : 200) : 255))      // (136: the next kernel of the chain fits beside it)
 attn_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __nv_bfloat16* __restrict__ kpages,
                    const __nv_bfloat16* __restrict__ vpages, const int* __restrict__ block_table, int max_blocks,
                    const int* __restrict__ positions, __nv_bfloat16* __restrict__ out, float* __restrict__ partial,
@@ -68,8 +68,8 @@ VM_API int vm_attention_decode_bf16(const void* q, int q_row_stride, const void*
     const int G = H / Hkv;
     dim3 grid(n_splits, Hkv * ((G + DEC_ROWS - 1) / DEC_ROWS), B);
     const __nv_bfloat16 *qq = (const __nv_bfloat16*)q, *kk = (const __nv_bfloat16*)kpages, *vv = (const __nv_bfloat16*)vpages;
-    // one split and a CTA per SM at most: ten warps per CTA, if their pages fit into shared memory
-    const bool wide = n_splits == 1 && (long long)grid.y * grid.z <= vm_sm_count();
+    // one split and a CTA per SM at most: ten warps per CTA, if their pages fit into shared memory; a table of four pages and less has no work for more than four
+    const bool wide = n_splits == 1 && max_blocks > DEC_WARPS && (long long)grid.y * grid.z <= vm_sm_count();
 #define VM_DEC_CASE(DD)                                                                                                \
     case DD:                                                                                                           \
         if (wide && attn_decode_smem_bytes<DD, DEC_WARPS_WIDE>() <= 227 * 1024)                                        \

@@ -6,6 +6,9 @@ namespace vmad {
 
 constexpr int DEC_ROWS = 16;           // query heads per CTA (the M of the tensor-core tile); more heads per kv head take more CTAs
 constexpr int MAX_SPLITS = 16;         // the merge keeps one value per split in registers
+// Ten warps share the queries in shared memory, four fetch their own fragments: no barrier in front of the products (one row of 25 cached tokens, 9 heads, in a chain
+// of launches 3.35 -> 2.8 us; with ten warps the fragments' loads cost more than the barrier, eight rows of 520 tokens 3.9 -> 4.2)
+template <int WARPS> __host__ __device__ constexpr bool queries_shared() { return WARPS > 4; }
 
 // One warp works on one cache page (64 keys) at a time: K and V of the page go to the warp's own shared
 // memory with cp.async, S = Q K^T and O += P V run on mma.sync m16n8k16 with the G query heads of the kv
@@ -23,8 +26,9 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
     constexpr int CH = D / 8;              // 16-byte chunks per row
     constexpr int RW = D + 2;              // a result row: D sums, then the running max and the running sum
     constexpr int BN = VM_PAGE_TOKENS;
-    __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(smem_raw);                    // [16][DP]
-    __nv_bfloat16* sKV = sQ + DEC_ROWS * DP;                                            // [warps][K,V][64][DP]
+    constexpr bool SHARED_Q = queries_shared<DEC_WARPS>();
+    __nv_bfloat16* sQ = reinterpret_cast<__nv_bfloat16*>(smem_raw);                    // [16][DP], of many warps
+    __nv_bfloat16* sKV = sQ + (SHARED_Q ? DEC_ROWS * DP : 0);                           // [warps][K,V][64][DP]
     float* res = reinterpret_cast<float*>(sKV + DEC_WARPS * 2 * BN * DP);               // [warps][16][RW]
     if (PDL) vm_pdl_launch_dependents();
     // Before the wait this kernel reads what OLDER steps wrote: positions, the block table and the cache rows of earlier
@@ -49,10 +53,25 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
     __nv_bfloat16* vs = ks + BN * DP;
     const int new_row = pos - last_page * BN;              // the row of the last page that this step's token takes
 
-    // the calling warp fetches K and V of one page; skip >= 0: all rows but that one
-    auto load_page = [&](int blk, int skip) -> bool {
-        const int page = (blk < max_blocks) ? table[blk] : -1;
-        if (page < 0 || page >= n_pages) { if (lane == 0 && err) atomicExch(err, 3); return false; }
+    auto page_of = [&](int blk) { return blk < page_b && blk < max_blocks ? table[blk] : -1; };
+    // the calling warp fetches the keys (or the values) of one page
+    auto load_rows = [&](__nv_bfloat16* to, const __nv_bfloat16* pool, int page) {
+        const __nv_bfloat16* from = pool + (size_t)page * page_stride + (size_t)hk * BN * D;
+#pragma unroll 4
+        for (int c = lane; c < BN * CH; c += 32) {
+            const int r = c / CH, ch = c - r * CH;
+            vm_cp_async16(to + r * DP + ch * 8, from + r * D + ch * 8);
+        }
+    };
+    auto there = [&](int page) {
+        const bool ok = page >= 0 && page < n_pages;
+        if (!ok && lane == 0 && err) atomicExch(err, 3);
+        return ok;
+    };
+    int blk = page_a + warp, page = page_of(blk);
+    bool have = blk < page_b && there(page);
+    if (have) {
+        const int skip = PDL && blk == last_page ? new_row : -1;
         const __nv_bfloat16* kg = kpages + (size_t)page * page_stride + (size_t)hk * BN * D;
         const __nv_bfloat16* vg = vpages + (size_t)page * page_stride + (size_t)hk * BN * D;
 #pragma unroll 4
@@ -63,45 +82,56 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
                 vm_cp_async16(vs + r * DP + ch * 8, vg + r * D + ch * 8);
             }
         }
-        return true;
-    };
-    int blk = page_a + warp;
-    bool have = (blk < page_b) && load_page(blk, PDL && blk == last_page ? new_row : -1);
+    }
     vm_cp_async_commit();
     if (PDL) {
         vm_pdl_wait();
         if (have && blk == last_page && lane < 2 * CH) {   // the new token's key and value
-            const int page = table[blk];
             const size_t at = (size_t)page * page_stride + ((size_t)hk * BN + new_row) * D + (lane % CH) * 8;
             if (lane < CH) vm_cp_async16(ks + new_row * DP + lane * 8, kpages + at);
             else vm_cp_async16(vs + new_row * DP + (lane - CH) * 8, vpages + at);
         }
     }
-    // ---- the queries of this CTA's heads (rows past the last head are zero)
-    for (int c = tid; c < DEC_ROWS * CH; c += DEC_WARPS * 32) {
-        const int r = c / CH, ch = c - r * CH;
-        if (r < ng) vm_cp_async16(sQ + r * DP + ch * 8, q + (size_t)b * q_row_stride + (size_t)(h0 + r) * D + ch * 8);
-        else *reinterpret_cast<uint4*>(sQ + r * DP + ch * 8) = make_uint4(0u, 0u, 0u, 0u);
+    // ---- the queries of this CTA's heads (rows past the last head are zero): many warps share them, few fetch their fragments
+    const int g = lane >> 2, t4 = lane & 3;
+    unsigned qa[D / 16][4];
+    if (SHARED_Q) {
+        for (int c = tid; c < DEC_ROWS * CH; c += DEC_WARPS * 32) {
+            const int r = c / CH, ch = c - r * CH;
+            if (r < ng) vm_cp_async16(sQ + r * DP + ch * 8, q + (size_t)b * q_row_stride + (size_t)(h0 + r) * D + ch * 8);
+            else *reinterpret_cast<uint4*>(sQ + r * DP + ch * 8) = make_uint4(0u, 0u, 0u, 0u);
+        }
+    } else if (blk < page_b) {
+        const __nv_bfloat16* qg = q + (size_t)b * q_row_stride + (size_t)(h0 + g) * D + 2 * t4;
+        auto pair = [&](int row, int at) { return row < ng ? __ldcg(reinterpret_cast<const unsigned*>(qg + (row - g) * D + at)) : 0u; };
+#pragma unroll
+        for (int kk = 0; kk < D / 16; ++kk) {
+            qa[kk][0] = pair(g, kk * 16); qa[kk][1] = pair(g + 8, kk * 16);
+            qa[kk][2] = pair(g, kk * 16 + 8); qa[kk][3] = pair(g + 8, kk * 16 + 8);
+        }
     }
     vm_cp_async_commit();
     vm_cp_async_wait_all();
-    __syncthreads();                                       // the queries (fetched by all threads) are in place
-
-    const int g = lane >> 2, t4 = lane & 3;
-    unsigned qa[D / 16][4];
+    if (SHARED_Q) {
+        __syncthreads();                                   // the queries (fetched by all threads) are in place
 #pragma unroll
-    for (int kk = 0; kk < D / 16; ++kk)
-        vm_ldmatrix_x4(qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3],
-                       sQ + ((lane & 7) + 8 * ((lane >> 3) & 1)) * DP + kk * 16 + 8 * (lane >> 4));
+        for (int kk = 0; kk < D / 16; ++kk)
+            vm_ldmatrix_x4(qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3],
+                           sQ + ((lane & 7) + 8 * ((lane >> 3) & 1)) * DP + kk * 16 + 8 * (lane >> 4));
+    } else {
+        __syncwarp();
+    }
     float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.f, l_b = 0.f;     // rows g and g + 8 of the tile
     float o[D / 8][4];
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
 
+    // A further page's keys are fetched as soon as this one's are multiplied, its values as soon as these are: the loads of either run under the other's work.
     while (blk < page_b) {
+        const int next = blk + DEC_WARPS, next_page = page_of(next);
+        const bool have_next = next < page_b && there(next_page);
+        float s[BN / 8][4];
         if (have) {
-            const int key0 = blk * BN;
-            float s[BN / 8][4];
 #pragma unroll
             for (int nb = 0; nb < BN / 8; ++nb) { s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f; }
 #pragma unroll
@@ -114,6 +144,14 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
                     vm_mma_bf16_16816(s[nb + 1], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], b2, b3);
                 }
             }
+        }
+        if (next < page_b) {
+            __syncwarp();                                  // every lane is done with the keys before they are overwritten
+            if (have_next) load_rows(ks, kpages, next_page);
+            vm_cp_async_commit();
+        }
+        if (have) {
+            const int key0 = blk * BN;
             float mx_a = -INFINITY, mx_b = -INFINITY;
 #pragma unroll
             for (int nb = 0; nb < BN / 8; ++nb) {
@@ -146,6 +184,11 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
             m_a = mn_a; m_b = mn_b;
 #pragma unroll
             for (int i = 0; i < D / 8; ++i) { o[i][0] *= al_a; o[i][1] *= al_a; o[i][2] *= al_b; o[i][3] *= al_b; }
+            if (blk != page_a + warp) {                    // (the first page came whole; of a further one the values are the group before the last, or the last)
+                if (next < page_b) asm volatile("cp.async.wait_group 1;\n" ::);
+                else vm_cp_async_wait_all();
+                __syncwarp();
+            }
 #pragma unroll
             for (int kk = 0; kk < BN / 16; ++kk) {
 #pragma unroll
@@ -157,61 +200,79 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
                 }
             }
         }
-        blk += DEC_WARPS;
+        blk = next; have = have_next;
         if (blk < page_b) {
-            __syncwarp();                                  // every lane is done with the page before it is overwritten
-            have = load_page(blk, -1);
+            __syncwarp();                                  // every lane is done with the values
+            if (have) load_rows(vs, vpages, next_page);
             vm_cp_async_commit();
-            vm_cp_async_wait_all();
+            asm volatile("cp.async.wait_group 1;\n" ::);   // the keys
             __syncwarp();
         }
     }
-    // ---- this warp's result rows: join the quad's sums; res[warp][row] = (o[D], m, l)
+    vm_cp_async_wait_all();
+    // ---- this warp's result rows: join the quad's sums; res[warp][row] = (o[D], m, l), of the warps that had a page and the rows that are there
     l_a += __shfl_xor_sync(0xffffffffu, l_a, 1); l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
     l_b += __shfl_xor_sync(0xffffffffu, l_b, 1); l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
-    {
-        float* ra = res + ((size_t)warp * DEC_ROWS + g) * RW;
-        float* rb = res + ((size_t)warp * DEC_ROWS + g + 8) * RW;
+    const int used = min(DEC_WARPS, max(0, page_b - page_a));
+    if (n_splits == 1 && used == 1) {                      // one page: nothing to join
+        if (warp == 0) {
+            const float inv[2] = {l_a, l_b};
 #pragma unroll
-        for (int i = 0; i < D / 8; ++i) {
-            const int d = i * 8 + 2 * t4;
-            ra[d] = o[i][0]; ra[d + 1] = o[i][1]; rb[d] = o[i][2]; rb[d + 1] = o[i][3];
+            for (int half = 0; half < 2; ++half)
+                if (g + 8 * half < ng) {
+                    __nv_bfloat16* dst = out + ((size_t)b * H + (h0 + g + 8 * half)) * D + 2 * t4;
+#pragma unroll
+                    for (int i = 0; i < D / 8; ++i)
+                        *reinterpret_cast<unsigned*>(dst + 8 * i) = vm_pack_bf16(o[i][2 * half] / inv[half], o[i][2 * half + 1] / inv[half]);
+                }
         }
-        if (t4 == 0) { ra[D] = m_a; ra[D + 1] = l_a; rb[D] = m_b; rb[D + 1] = l_b; }
+        return;
+    }
+    if (warp < used) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+            if (g + 8 * half < ng) {
+                float* r = res + ((size_t)warp * DEC_ROWS + g + 8 * half) * RW;
+#pragma unroll
+                for (int i = 0; i < D / 8; ++i) *reinterpret_cast<float2*>(r + i * 8 + 2 * t4) = make_float2(o[i][2 * half], o[i][2 * half + 1]);
+                if (t4 == 0) { r[D] = half ? m_b : m_a; r[D + 1] = half ? l_b : l_a; }
+            }
     }
     __syncthreads();
+    // row r, column d over the warps that had a page (all loads first: no chain from warp to warp)
+    auto join = [&](int r, int d, float& M, float& acc, float& L) {
+        float ms[DEC_WARPS], os[DEC_WARPS], ls[DEC_WARPS];
+#pragma unroll
+        for (int w = 0; w < DEC_WARPS; ++w) {
+            const float* rr = res + ((size_t)w * DEC_ROWS + r) * RW;
+            ms[w] = w < used ? rr[D] : -INFINITY;
+            os[w] = w < used ? rr[d] : 0.f;
+            ls[w] = w < used ? rr[D + 1] : 0.f;
+        }
+        M = -INFINITY; acc = L = 0.f;
+#pragma unroll
+        for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, ms[w]);
+#pragma unroll
+        for (int w = 0; w < DEC_WARPS; ++w) {
+            const float f = (ms[w] == -INFINITY) ? 0.f : exp2f(ms[w] - M);
+            acc += f * os[w]; L += f * ls[w];
+        }
+    };
     if (n_splits == 1) {
         // one CTA holds all keys of the sequence: the warps' rows are joined straight into the output
         for (int i = tid; i < ng * D; i += DEC_WARPS * 32) {
             const int r = i / D, d = i - r * D;
-            float M = -INFINITY;
-#pragma unroll
-            for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, res[((size_t)w * DEC_ROWS + r) * RW + D]);
-            float acc = 0.f, L = 0.f;
-#pragma unroll
-            for (int w = 0; w < DEC_WARPS; ++w) {
-                const float* rr = res + ((size_t)w * DEC_ROWS + r) * RW;
-                const float f = (rr[D] == -INFINITY) ? 0.f : exp2f(rr[D] - M);
-                acc += f * rr[d]; L += f * rr[D + 1];
-            }
+            float M, acc, L;
+            join(r, d, M, acc, L);
             out[((size_t)b * H + (h0 + r)) * D + d] = __float2bfloat16_rn(acc / L);
         }
-        __syncthreads();                                   // shared memory may be reused for another item
         return;
     }
     // partial[b, h, split, :] = (o[D], m, l), merged over the warps (max and sums in base 2)
     for (int i = tid; i < ng * D; i += DEC_WARPS * 32) {
         const int r = i / D, d = i - r * D;
-        float M = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, res[((size_t)w * DEC_ROWS + r) * RW + D]);
-        float acc = 0.f, L = 0.f;
-#pragma unroll
-        for (int w = 0; w < DEC_WARPS; ++w) {
-            const float* rr = res + ((size_t)w * DEC_ROWS + r) * RW;
-            const float f = (rr[D] == -INFINITY) ? 0.f : exp2f(rr[D] - M);
-            acc += f * rr[d]; L += f * rr[D + 1];
-        }
+        float M, acc, L;
+        join(r, d, M, acc, L);
         float* dst = partial + (((size_t)b * H + (h0 + r)) * n_splits + split) * RW;
         dst[d] = acc;
         if (d == 0) { dst[D] = M; dst[D + 1] = L; }
@@ -254,12 +315,11 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
         out[((size_t)b * H + (h0 + r)) * D + d] = __float2bfloat16_rn(acc / L);
     }
     }
-    __syncthreads();                                       // shared memory may be reused for another item
 }
 
 template <int D, int WARPS>
 __host__ __device__ constexpr size_t attn_decode_smem_bytes() {
-    return (size_t)(DEC_ROWS + WARPS * 2 * VM_PAGE_TOKENS) * (D + 8) * sizeof(__nv_bfloat16)
+    return (size_t)((queries_shared<WARPS>() ? DEC_ROWS : 0) + WARPS * 2 * VM_PAGE_TOKENS) * (D + 8) * sizeof(__nv_bfloat16)
            + (size_t)WARPS * DEC_ROWS * (D + 2) * sizeof(float);
 }
 
