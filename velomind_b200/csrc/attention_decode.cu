@@ -6,7 +6,7 @@
 // online form of src/cpu/ops/fused_attention.cpp:84-135); the G = H / Hkv query heads that share a kv
 // head (src/cpu/ops/repeat_kv.cpp:51-61) are served by one CTA, so each key and value is read once.
 //
-// grid = (n_splits, Hkv * ceil(G / 16), B), 128 threads; or, with one split and no more CTAs than SMs, 320 threads
+// grid = (n_splits, Hkv * ceil(G / 16), B), 128 threads; or, with one split, no more CTAs than SMs and a block table wider than four pages, 320 threads
 // (ten warps, a cache page each: a sequence of up to 640 tokens is one round, and no partial result leaves the CTA).  A CTA's key range is a whole number of cache
 // pages, computed on the device from the sequence's length: the launch shape does not depend on the
 // lengths, so the launch can sit in a CUDA graph.  Head sizes 16, 32, ..., 128.  Scratch (global memory beyond inputs and outputs):
@@ -20,7 +20,7 @@ constexpr int DEC_WARPS = 4;
 constexpr int DEC_WARPS_WIDE = 10;
 using namespace vmad;
 
-template <int D, int WARPS>
+template <int D, int WARPS, bool AHEAD>
 __global__ void __launch_bounds__(WARPS * 32) __maxnreg__((WARPS == 10 ? (D <= 64 ? 136 : 200) : 255))      // (136: the next kernel of the chain fits beside it)
 attn_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __nv_bfloat16* __restrict__ kpages,
                    const __nv_bfloat16* __restrict__ vpages, const int* __restrict__ block_table, int max_blocks,
@@ -28,12 +28,12 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, const 
                    int* __restrict__ counters, int H, int Hkv, float scale_log2, int window, int n_pages,
                    int* __restrict__ err) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    attn_decode_body<D, WARPS, true>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, out, partial,
+    attn_decode_body<D, WARPS, true, AHEAD>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, out, partial,
                                          counters, H, Hkv, scale_log2, window, n_pages, err, blockIdx.x, gridDim.x, blockIdx.y,
                                          gridDim.y, blockIdx.z, smem_raw);
 }
 
-template <int D, int WARPS>
+template <int D, int WARPS, bool AHEAD>
 int launch_decode(dim3 grid, cudaStream_t stream, const __nv_bfloat16* q, int q_row_stride, const __nv_bfloat16* kpages,
                   const __nv_bfloat16* vpages, const int* block_table, int max_blocks, const int* positions,
                   __nv_bfloat16* out, float* partial, int* counters, int H, int Hkv, float scale, int window, int n_pages,
@@ -41,11 +41,11 @@ int launch_decode(dim3 grid, cudaStream_t stream, const __nv_bfloat16* q, int q_
     const size_t smem = attn_decode_smem_bytes<D, WARPS>();
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<D, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<D, WARPS, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    vm_launch_pdl(attn_decode_kernel<D, WARPS>, grid, dim3(WARPS * 32), smem, stream, q, q_row_stride, kpages, vpages, block_table,
+    vm_launch_pdl(attn_decode_kernel<D, WARPS, AHEAD>, grid, dim3(WARPS * 32), smem, stream, q, q_row_stride, kpages, vpages, block_table,
                   max_blocks, positions, out, partial, counters, H, Hkv, scale * 1.4426950408889634f, window, n_pages, err);
     return vm_launch_status();
 }
@@ -68,15 +68,21 @@ VM_API int vm_attention_decode_bf16(const void* q, int q_row_stride, const void*
     const int G = H / Hkv;
     dim3 grid(n_splits, Hkv * ((G + DEC_ROWS - 1) / DEC_ROWS), B);
     const __nv_bfloat16 *qq = (const __nv_bfloat16*)q, *kk = (const __nv_bfloat16*)kpages, *vv = (const __nv_bfloat16*)vpages;
-    // one split and a CTA per SM at most: ten warps per CTA, if their pages fit into shared memory; a table of four pages and less has no work for more than four
+    // one split and a CTA per SM at most: ten warps per CTA, if their pages fit into shared memory; a table of four pages and less has no work for more than four.
+    // Tables of more than two pages a warp have the next page fetched ahead (attn_decode_body.cuh).
     const bool wide = n_splits == 1 && max_blocks > DEC_WARPS && (long long)grid.y * grid.z <= vm_sm_count();
 #define VM_DEC_CASE(DD)                                                                                                \
     case DD:                                                                                                           \
-        if (wide && attn_decode_smem_bytes<DD, DEC_WARPS_WIDE>() <= 227 * 1024)                                        \
-            return launch_decode<DD, DEC_WARPS_WIDE>(grid, stream, qq, q_row_stride, kk, vv, block_table, max_blocks,  \
-                                                     positions, (__nv_bfloat16*)out, partial, counters, H, Hkv, scale, \
-                                                     window, n_pages, err);                                            \
-        return launch_decode<DD, DEC_WARPS>(grid, stream, qq, q_row_stride, kk, vv, block_table, max_blocks, positions, \
+        if (wide && attn_decode_smem_bytes<DD, DEC_WARPS_WIDE>() <= 227 * 1024) {                                      \
+            if (max_blocks > 2 * DEC_WARPS_WIDE)                                                                       \
+                return launch_decode<DD, DEC_WARPS_WIDE, true>(grid, stream, qq, q_row_stride, kk, vv, block_table,    \
+                                                               max_blocks, positions, (__nv_bfloat16*)out, partial,    \
+                                                               counters, H, Hkv, scale, window, n_pages, err);         \
+            return launch_decode<DD, DEC_WARPS_WIDE, false>(grid, stream, qq, q_row_stride, kk, vv, block_table,       \
+                                                            max_blocks, positions, (__nv_bfloat16*)out, partial,       \
+                                                            counters, H, Hkv, scale, window, n_pages, err);            \
+        }                                                                                                              \
+        return launch_decode<DD, DEC_WARPS, false>(grid, stream, qq, q_row_stride, kk, vv, block_table, max_blocks, positions, \
                                             (__nv_bfloat16*)out, partial, counters, H, Hkv, scale, window, n_pages, err);
     switch (D) {
         VM_DEC_CASE(16) VM_DEC_CASE(32) VM_DEC_CASE(48) VM_DEC_CASE(64)

@@ -7,14 +7,17 @@ namespace vmad {
 constexpr int DEC_ROWS = 16;           // query heads per CTA (the M of the tensor-core tile); more heads per kv head take more CTAs
 constexpr int MAX_SPLITS = 16;         // the merge keeps one value per split in registers
 // Ten warps share the queries in shared memory, four fetch their own fragments: no barrier in front of the products (one row of 25 cached tokens, 9 heads, in a chain
-// of launches 3.35 -> 2.8 us; with ten warps the fragments' loads cost more than the barrier, eight rows of 520 tokens 3.9 -> 4.2)
+// of launches 3.35 -> 2.5 us; with ten warps the fragments' loads cost more than the barrier, eight rows of 520 tokens 3.9 -> 4.2)
 template <int WARPS> __host__ __device__ constexpr bool queries_shared() { return WARPS > 4; }
 
 // One warp works on one cache page (64 keys) at a time: K and V of the page go to the warp's own shared
 // memory with cp.async, S = Q K^T and O += P V run on mma.sync m16n8k16 with the G query heads of the kv
 // head as the rows of the tile (padded to 16), the softmax state is float32 in base 2.
 // (split, group_y, b) of (n_splits, n_group_y, B) is what (blockIdx, gridDim) are for the stand-alone kernel.
-template <int D, int DEC_WARPS, bool PDL>
+// AHEAD: a further page's keys are fetched as soon as this one's are multiplied, its values as soon as these are, so that the loads of either run under the other's
+// work (four sequences of 1,000 to 3,000 tokens, 32 heads 16.9 -> 15.2 us); without it the page comes whole, which is the shorter code where most warps have one
+// page (in a chain of launches, eight rows of 520 tokens, 9 heads 3.7 us, with it 4.0; one row of 25 2.5 / 2.8).
+template <int D, int DEC_WARPS, bool PDL, bool AHEAD>
 __device__ __forceinline__ void
 attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __nv_bfloat16* __restrict__ kpages,
                  const __nv_bfloat16* __restrict__ vpages, const int* __restrict__ block_table, int max_blocks,
@@ -63,15 +66,8 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
             vm_cp_async16(to + r * DP + ch * 8, from + r * D + ch * 8);
         }
     };
-    auto there = [&](int page) {
-        const bool ok = page >= 0 && page < n_pages;
-        if (!ok && lane == 0 && err) atomicExch(err, 3);
-        return ok;
-    };
-    int blk = page_a + warp, page = page_of(blk);
-    bool have = blk < page_b && there(page);
-    if (have) {
-        const int skip = PDL && blk == last_page ? new_row : -1;
+    // both of one page; skip >= 0: all rows but that one
+    auto load_page = [&](int page, int skip) {
         const __nv_bfloat16* kg = kpages + (size_t)page * page_stride + (size_t)hk * BN * D;
         const __nv_bfloat16* vg = vpages + (size_t)page * page_stride + (size_t)hk * BN * D;
 #pragma unroll 4
@@ -82,7 +78,15 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
                 vm_cp_async16(vs + r * DP + ch * 8, vg + r * D + ch * 8);
             }
         }
-    }
+    };
+    auto there = [&](int page) {
+        const bool ok = page >= 0 && page < n_pages;
+        if (!ok && lane == 0 && err) atomicExch(err, 3);
+        return ok;
+    };
+    int blk = page_a + warp, page = page_of(blk);
+    bool have = blk < page_b && there(page);
+    if (have) load_page(page, PDL && blk == last_page ? new_row : -1);
     vm_cp_async_commit();
     if (PDL) {
         vm_pdl_wait();
@@ -126,10 +130,9 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
 
-    // A further page's keys are fetched as soon as this one's are multiplied, its values as soon as these are: the loads of either run under the other's work.
     while (blk < page_b) {
-        const int next = blk + DEC_WARPS, next_page = page_of(next);
-        const bool have_next = next < page_b && there(next_page);
+        const int next = blk + DEC_WARPS, next_page = AHEAD ? page_of(next) : -1;
+        const bool have_next = AHEAD && next < page_b && there(next_page);
         float s[BN / 8][4];
         if (have) {
 #pragma unroll
@@ -145,7 +148,7 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
                 }
             }
         }
-        if (next < page_b) {
+        if (AHEAD && next < page_b) {
             __syncwarp();                                  // every lane is done with the keys before they are overwritten
             if (have_next) load_rows(ks, kpages, next_page);
             vm_cp_async_commit();
@@ -184,7 +187,7 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
             m_a = mn_a; m_b = mn_b;
 #pragma unroll
             for (int i = 0; i < D / 8; ++i) { o[i][0] *= al_a; o[i][1] *= al_a; o[i][2] *= al_b; o[i][3] *= al_b; }
-            if (blk != page_a + warp) {                    // (the first page came whole; of a further one the values are the group before the last, or the last)
+            if (AHEAD && blk != page_a + warp) {           // (the first page came whole; of a further one the values are the group before the last, or the last)
                 if (next < page_b) asm volatile("cp.async.wait_group 1;\n" ::);
                 else vm_cp_async_wait_all();
                 __syncwarp();
@@ -200,16 +203,24 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
                 }
             }
         }
-        blk = next; have = have_next;
+        blk = next;
         if (blk < page_b) {
             __syncwarp();                                  // every lane is done with the values
-            if (have) load_rows(vs, vpages, next_page);
-            vm_cp_async_commit();
-            asm volatile("cp.async.wait_group 1;\n" ::);   // the keys
+            if (AHEAD) {
+                have = have_next;
+                if (have) load_rows(vs, vpages, next_page);
+                vm_cp_async_commit();
+                asm volatile("cp.async.wait_group 1;\n" ::);      // the keys
+            } else {
+                page = page_of(blk);
+                have = there(page);
+                if (have) load_page(page, -1);
+                vm_cp_async_commit();
+                vm_cp_async_wait_all();
+            }
             __syncwarp();
         }
     }
-    vm_cp_async_wait_all();
     // ---- this warp's result rows: join the quad's sums; res[warp][row] = (o[D], m, l), of the warps that had a page and the rows that are there
     l_a += __shfl_xor_sync(0xffffffffu, l_a, 1); l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
     l_b += __shfl_xor_sync(0xffffffffu, l_b, 1); l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
