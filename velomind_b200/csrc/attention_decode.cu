@@ -26,10 +26,10 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, const 
                    const __nv_bfloat16* __restrict__ vpages, const int* __restrict__ block_table, int max_blocks,
                    const int* __restrict__ positions, __nv_bfloat16* __restrict__ out, float* __restrict__ partial,
                    int* __restrict__ counters, int H, int Hkv, float scale_log2, int window, int n_pages,
-                   int* __restrict__ err) {
+                   int* __restrict__ err, int in_step) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     attn_decode_body<D, WARPS, true, AHEAD>(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, out, partial,
-                                         counters, H, Hkv, scale_log2, window, n_pages, err, blockIdx.x, gridDim.x, blockIdx.y,
+                                         counters, H, Hkv, scale_log2, window, n_pages, err, in_step, blockIdx.x, gridDim.x, blockIdx.y,
                                          gridDim.y, blockIdx.z, smem_raw);
 }
 
@@ -37,7 +37,7 @@ template <int D, int WARPS, bool AHEAD>
 int launch_decode(dim3 grid, cudaStream_t stream, const __nv_bfloat16* q, int q_row_stride, const __nv_bfloat16* kpages,
                   const __nv_bfloat16* vpages, const int* block_table, int max_blocks, const int* positions,
                   __nv_bfloat16* out, float* partial, int* counters, int H, int Hkv, float scale, int window, int n_pages,
-                  int* err) {
+                  int* err, int in_step) {
     const size_t smem = attn_decode_smem_bytes<D, WARPS>();
     static bool configured = false;
     if (!configured) {
@@ -46,7 +46,7 @@ int launch_decode(dim3 grid, cudaStream_t stream, const __nv_bfloat16* q, int q_
         configured = true;
     }
     vm_launch_pdl(attn_decode_kernel<D, WARPS, AHEAD>, grid, dim3(WARPS * 32), smem, stream, q, q_row_stride, kpages, vpages, block_table,
-                  max_blocks, positions, out, partial, counters, H, Hkv, scale * 1.4426950408889634f, window, n_pages, err);
+                  max_blocks, positions, out, partial, counters, H, Hkv, scale * 1.4426950408889634f, window, n_pages, err, in_step);
     return vm_launch_status();
 }
 
@@ -57,11 +57,9 @@ VM_API long long vm_attention_decode_scratch_floats(int B, int H, int D, int n_s
     return (long long)B * H * n_splits * (D + 2);
 }
 
-// q: [B, H, D] rows with stride q_row_stride; out: [B, H*D].  counters: at least B * Hkv * ceil(G/16) ints, zero.
-VM_API int vm_attention_decode_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages,
-                                    const int* block_table, int max_blocks, const int* positions, void* out,
-                                    float* partial, int* counters, int B, int H, int Hkv, int D, int n_splits,
-                                    float scale, int window, int n_pages, int* err, cudaStream_t stream) {
+static int attention_decode(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table, int max_blocks, const int* positions,
+                            void* out, float* partial, int* counters, int B, int H, int Hkv, int D, int n_splits, float scale, int window, int n_pages, int* err,
+                            int in_step, cudaStream_t stream) {
     if (B <= 0) return 0;
     if (H <= 0 || Hkv <= 0 || H % Hkv != 0 || n_splits < 1 || n_splits > MAX_SPLITS || (q_row_stride % 8) != 0)
         return VM_ERR_UNSUPPORTED;
@@ -77,19 +75,37 @@ VM_API int vm_attention_decode_bf16(const void* q, int q_row_stride, const void*
             if (max_blocks > 2 * DEC_WARPS_WIDE)                                                                       \
                 return launch_decode<DD, DEC_WARPS_WIDE, true>(grid, stream, qq, q_row_stride, kk, vv, block_table,    \
                                                                max_blocks, positions, (__nv_bfloat16*)out, partial,    \
-                                                               counters, H, Hkv, scale, window, n_pages, err);         \
+                                                               counters, H, Hkv, scale, window, n_pages, err, in_step); \
             return launch_decode<DD, DEC_WARPS_WIDE, false>(grid, stream, qq, q_row_stride, kk, vv, block_table,       \
                                                             max_blocks, positions, (__nv_bfloat16*)out, partial,       \
-                                                            counters, H, Hkv, scale, window, n_pages, err);            \
+                                                            counters, H, Hkv, scale, window, n_pages, err, in_step);   \
         }                                                                                                              \
         return launch_decode<DD, DEC_WARPS, false>(grid, stream, qq, q_row_stride, kk, vv, block_table, max_blocks, positions, \
-                                            (__nv_bfloat16*)out, partial, counters, H, Hkv, scale, window, n_pages, err);
+                                            (__nv_bfloat16*)out, partial, counters, H, Hkv, scale, window, n_pages, err, in_step);
     switch (D) {
         VM_DEC_CASE(16) VM_DEC_CASE(32) VM_DEC_CASE(48) VM_DEC_CASE(64)
         VM_DEC_CASE(80) VM_DEC_CASE(96) VM_DEC_CASE(112) VM_DEC_CASE(128)
         default: return VM_ERR_UNSUPPORTED;
     }
 #undef VM_DEC_CASE
+}
+
+// q: [B, H, D] rows with stride q_row_stride; out: [B, H*D].  counters: at least B * Hkv * ceil(G/16) ints, zero.
+VM_API int vm_attention_decode_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages,
+                                    const int* block_table, int max_blocks, const int* positions, void* out,
+                                    float* partial, int* counters, int B, int H, int Hkv, int D, int n_splits,
+                                    float scale, int window, int n_pages, int* err, cudaStream_t stream) {
+    return attention_decode(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, out, partial, counters, B, H, Hkv, D, n_splits, scale, window,
+                            n_pages, err, 0, stream);
+}
+
+// The same inside a step whose first kernel waits before it lets its dependents start (kernels.h): fetches what older steps wrote in front of its own wait.
+VM_API int vm_attention_decode_in_step_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages,
+                                            const int* block_table, int max_blocks, const int* positions, void* out,
+                                            float* partial, int* counters, int B, int H, int Hkv, int D, int n_splits,
+                                            float scale, int window, int n_pages, int* err, cudaStream_t stream) {
+    return attention_decode(q, q_row_stride, kpages, vpages, block_table, max_blocks, positions, out, partial, counters, B, H, Hkv, D, n_splits, scale, window,
+                            n_pages, err, 1, stream);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -23,7 +23,7 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
                  const __nv_bfloat16* __restrict__ vpages, const int* __restrict__ block_table, int max_blocks,
                  const int* __restrict__ positions, __nv_bfloat16* __restrict__ out, float* __restrict__ partial,
                  int* __restrict__ counters, int H, int Hkv, float scale_log2, int window, int n_pages,
-                 int* __restrict__ err, const int split, const int n_splits, const int group_y, const int n_group_y,
+                 int* __restrict__ err, const int in_step, const int split, const int n_splits, const int group_y, const int n_group_y,
                  const int b, unsigned char* smem_raw) {
     constexpr int DP = D + 8;              // padded row: an odd number of 16-byte units -> conflict-free ldmatrix
     constexpr int CH = D / 8;              // 16-byte chunks per row
@@ -34,10 +34,11 @@ attn_decode_body(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __
     __nv_bfloat16* sKV = sQ + (SHARED_Q ? DEC_ROWS * DP : 0);                           // [warps][K,V][64][DP]
     float* res = reinterpret_cast<float*>(sKV + DEC_WARPS * 2 * BN * DP);               // [warps][16][RW]
     if (PDL) vm_pdl_launch_dependents();
-    // Before the wait this kernel reads what OLDER steps wrote: positions, the block table and the cache rows of earlier
-    // tokens.  That is sound because a step's first kernel lets its dependents start only after its own wait, when
+    // Inside a step (in_step) this kernel reads, before the wait below, what OLDER steps wrote: positions, the block table and the cache rows of
+    // earlier tokens.  That is sound because a step's first kernel lets its dependents start only after its own wait, when
     // everything older than the step is complete (common.cuh).  The new row and the queries, which the step itself
-    // writes, are fetched after the wait.
+    // writes, are fetched after that wait.  Elsewhere nothing orders the writers of older rows in front of a kernel that has not waited: it waits here.
+    if (PDL && !in_step) vm_pdl_wait();
     const int G = H / Hkv;
     const int groups_per_kv = (G + DEC_ROWS - 1) / DEC_ROWS;
     const int hk = group_y / groups_per_kv, gg = group_y - hk * groups_per_kv;

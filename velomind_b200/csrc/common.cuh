@@ -53,11 +53,11 @@ __device__ __forceinline__ int vm_first_seen(int pos, int window, int chunk) {
 // vm_pdl_wait() before it reads anything an earlier kernel wrote and before its first global write.
 // vm_pdl_launch_dependents() lets the successor start its own preamble.  Without the launch attribute both
 // are no-ops.
-// One kernel reads more than constants in its preamble: the decode attention fetches positions, the block table
-// and the cache rows of EARLIER tokens there, all of them written before this step began.  The rule that makes this
+// One kernel reads more than constants in its preamble, where the engine asks for it (vm_attention_decode_in_step_bf16): the decode attention fetches
+// positions, the block table and the cache rows of EARLIER tokens there, all of them written before this step began.  The rule that makes this
 // sound: a step's FIRST kernel (the embedding) calls vm_pdl_launch_dependents() only AFTER its own vm_pdl_wait(), so no
 // later kernel of the step starts before everything older than the step is complete and visible; what the step itself
-// writes (the new rows, the queries) is read after the attention's wait.
+// writes (the new rows, the queries) is read after the attention's wait.  Outside of a step (vm_attention_decode_bf16) it waits first.
 // Kernels launched without the attribute (and library kernels) never release their successor early.
 __device__ __forceinline__ void vm_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void vm_pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -37,7 +37,7 @@ skinny_direct_kernel(const SkinnyParams p) {
     __shared__ float red[WARPS][TP * 16][RS];
     __shared__ float scale[8 * NT];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-    vm_pdl_launch_dependents();                          // (of the form that writes the cache too: its reader asks for the new row after its own wait)
+    vm_pdl_launch_dependents();                          // (of the form that writes the cache too: its reader asks for the new row after its own wait, common.cuh)
     const bool two = EPI == DIRECT_UNIT || EPI == DIRECT_ROPE || p.tiles == 2;
     const int pairs = p.N / (two ? 16 : 8);
     int nA[TP], nB[TP], head[TP];

@@ -492,7 +492,7 @@ void attention(StepContext& ctx, const void* q, int q_row_stride, const KVView& 
         float* partial = static_cast<float*>(ctx.take(static_cast<long long>(ctx.B_cap) * H * MAX_DECODE_SPLITS * (D + 2), DType::F32));   // sized by shape
         {
             Timed t("attention_decode_bf16", s);
-            check(vm_attention_decode_bf16(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, out, partial,
+            check(vm_attention_decode_in_step_bf16(q, q_row_stride, kv.k_pages, kv.v_pages, kv.block_table, kv.table_width, ctx.positions, out, partial,
                                            decode_counters(), ctx.B, H, Hkv, D, n_splits, scale, window, kv.n_pages, ctx.err, s),
                   "attention_decode_bf16", s);
         }

@@ -306,6 +306,13 @@ long long vm_attention_decode_scratch_floats(int B, int H, int D, int n_splits);
 int vm_attention_decode_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
                              int max_blocks, const int* positions, void* out, float* partial, int* counters, int B, int H,
                              int Hkv, int D, int n_splits, float scale, int window, int n_pages, int* err, cudaStream_t stream);
+// The same for a chain of launches (a step) in which each sequence gets ONE new token: with programmatic launch on it may fetch positions, block table and
+// the cache rows of EARLIER tokens while the launches in front of it still run.  Those must be complete before the chain's first kernel lets its
+// dependents start: the embeddings of this library wait first, kernels launched without the attribute never let them start early.  Two tokens of a
+// sequence in one such chain are two chains; vm_attention_decode_bf16 asks for none of this.
+int vm_attention_decode_in_step_bf16(const void* q, int q_row_stride, const void* kpages, const void* vpages, const int* block_table,
+                                     int max_blocks, const int* positions, void* out, float* partial, int* counters, int B, int H,
+                                     int Hkv, int D, int n_splits, float scale, int window, int n_pages, int* err, cudaStream_t stream);
 
 // ---- routed_experts_grouped.cu: the same feed-forward for many tokens (bfloat16), pairs grouped by expert on the device
 long long vm_experts_grouped_rows(int T, int top, int E);

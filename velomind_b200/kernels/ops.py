@@ -242,17 +242,17 @@ def decode_splits(B: int, Hkv: int, G: int, D: int, table_width: int, device=Non
 def attention_decode_bf16(q: torch.Tensor, q_row_stride: int, k_pages: torch.Tensor, v_pages: torch.Tensor,
                           block_table: torch.Tensor, positions: torch.Tensor, out: torch.Tensor, partial: torch.Tensor,
                           counters: torch.Tensor, H: int, Hkv: int, D: int, n_splits: int, scale: float, window: int = 0,
-                          err: Optional[torch.Tensor] = None) -> None:
+                          err: Optional[torch.Tensor] = None, in_step: bool = False) -> None:
     """One new token per sequence: split-KV attention over the cache (bfloat16, D <= 128, D % 8 == 0).
-    partial: float32 scratch of B*H*n_splits*(D+2); counters: zeroed int32, left zero."""
+    partial: float32 scratch of B*H*n_splits*(D+2); counters: zeroed int32, left zero.  in_step: as one launch of a step, whose older
+    cache rows may be fetched while the launches in front still run (the condition is beside the declaration in kernels.h)."""
     B = out.shape[0]
     if partial.numel() < B * H * n_splits * (D + 2) or counters.numel() < B * H:
         raise KernelError("attention_decode_bf16: scratch too small")
-    _check(library().vm_attention_decode_bf16(_ptr(q), _c_int(q_row_stride), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
-                                              _c_int(block_table.shape[1]), _ptr(positions), _ptr(out), _ptr(partial),
-                                              _ptr(counters), _c_int(B), _c_int(H), _c_int(Hkv), _c_int(D), _c_int(n_splits),
-                                              _c_f(scale), _c_int(window), _c_int(k_pages.shape[0]), _ptr(err), _stream()),
-           "attention_decode_bf16")
+    launch = library().vm_attention_decode_in_step_bf16 if in_step else library().vm_attention_decode_bf16
+    _check(launch(_ptr(q), _c_int(q_row_stride), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), _c_int(block_table.shape[1]), _ptr(positions), _ptr(out),
+                  _ptr(partial), _ptr(counters), _c_int(B), _c_int(H), _c_int(Hkv), _c_int(D), _c_int(n_splits), _c_f(scale), _c_int(window),
+                  _c_int(k_pages.shape[0]), _ptr(err), _stream()), "attention_decode_bf16")
 
 
 _sm_counts = {}
