@@ -125,3 +125,13 @@ def test_more_rows_than_the_kernel_takes():
     h, nw, squares = torch.zeros(40, 64, device=DEV), torch.ones(64, device=DEV), torch.zeros(40, 8, device=DEV)
     assert _lib().vm_skinny_residual_ready(_p(x), _p(w), _i(40), _i(64), _i(96), _p(h), _p(nw), _p(out), _p(squares), _stream()) == -1
     assert _lib().vm_skinny_linear(_p(x), _i(2), _p(squares), _f(1e-5), _p(w), _i(40), _i(64), _i(96), _p(out), _i(64), _i(1), _p(None), _p(None), _stream()) == -1
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 64, 96), (8, 576, 576), (32, 144, 1536)])
+def test_ready_rows_into_a_residual_sum_are_refused(M, N, K):
+    g = torch.Generator().manual_seed(6)
+    x, w, h = _bf(torch.randn(M, K, generator=g)), _bf(torch.randn(N, K, generator=g)), torch.randn(M, N, generator=g).to(DEV)
+    squares, before = torch.ones(M, _lib().vm_skinny_ready_parts(_i(K)), device=DEV), h.clone()
+    assert _lib().vm_skinny_linear(_p(x), _i(2), _p(squares), _f(1e-5), _p(w), _i(M), _i(N), _i(K), _p(None), _i(N), _i(0), _p(h), _p(None), _stream()) == -1
+    torch.cuda.synchronize()
+    assert torch.equal(h, before)

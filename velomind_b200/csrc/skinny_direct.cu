@@ -275,7 +275,8 @@ template <int EPI> int launch_direct(const SkinnyParams& p, int items, cudaStrea
 
 int vm_skinny_direct(const vmsk::SkinnyParams& p, int items, cudaStream_t stream) {
     if (p.M <= 0 || items <= 0) return 0;
-    if (p.M > 32 || p.K <= 0 || p.K % 32 != 0 || (p.squares && p.parts % 4)) return VM_ERR_UNSUPPORTED;
+    // (a residual product has no warp that joins squares, and no scale in its epilogue: its rows are plain)
+    if (p.M > 32 || p.K <= 0 || p.K % 32 != 0 || (p.squares && (p.parts % 4 || p.epi == EPI_RESIDUAL))) return VM_ERR_UNSUPPORTED;
     switch (p.epi) {
         case EPI_STORE_BF16: case EPI_STORE_F32: return launch_direct<DIRECT_STORE>(p, items, stream);
         case EPI_RESIDUAL: return launch_direct<DIRECT_RESIDUAL>(p, items, stream);

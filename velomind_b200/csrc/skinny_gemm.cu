@@ -183,10 +183,10 @@ VM_API int vm_skinny_residual_ready(const void* A, const void* W, int M, int N, 
     return skinny_dispatch(p, N / (8 * p.tiles), stream);
 }
 
-// out = A W^T (pro 0, 2) or rmsnorm(h) W^T (pro 1); out bf16 (out_f32 0) or float32 (1); or h += ... (residual 1).
+// out = A W^T (pro 0, 2) or rmsnorm(h) W^T (pro 1); out bf16 (out_f32 0) or float32 (1); or h += ... (residual_h; of pro 0 and 1).
 VM_API int vm_skinny_linear(const void* A, int pro, const float* norm_w, float eps, const void* W, int M, int N, int K,
                             void* out, int out_stride, int out_f32, float* residual_h, int* err, cudaStream_t stream) {
-    if (N % 8 != 0) return VM_ERR_UNSUPPORTED;
+    if (N % 8 != 0 || (pro == 2 && residual_h)) return VM_ERR_UNSUPPORTED;
     SkinnyParams p{};
     p.err = err;
     p.W = (const __nv_bfloat16*)W; p.M = M; p.N = N; p.K = K;

@@ -348,7 +348,7 @@ int vm_skinny_gated(const void* A, int pro, const float* norm_w, float eps, cons
 int vm_skinny_clamped(const void* A, int pro, const float* norm_w, float eps, const void* W, int M, int I, int K, float limit, float alpha, void* out, int* err,
                       cudaStream_t stream);
 // pro above: 0, A bf16 [M, K]; 1, A the float32 residual, normed with norm_w and eps; 2, A the `ready` rows of vm_skinny_residual_ready (at most 32) and
-// norm_w their `squares`.  h += A W^T for at most 32 rows, which leaves ready = h next_w in bf16 and the parts of the rows' sums of squares:
+// norm_w their `squares` (refused together with residual_h).  h += A W^T for at most 32 rows, which leaves ready = h next_w in bf16 and the parts of the rows' sums of squares:
 // [M, vm_skinny_ready_parts(N)] float32, whose sum over a row is that row's sum of squares.
 int vm_skinny_ready_parts(int N);
 int vm_skinny_residual_ready(const void* A, const void* W, int M, int N, int K, float* h, const float* next_w, void* ready, float* squares,
