@@ -11,20 +11,24 @@
 // values of the next two steps on their way into registers; they are asked for behind the proxy fence of a step, which waits for loads in flight.  Warp 12
 // issues the products (tcgen05.mma, M = 128, K = 16), warps 8..11 empty the accumulator of the large products, which lies twice in tensor memory.
 //
-// Measured against the library's float32 product: 446 rows, 3,072 x 576 31 / 43.7 us, 960 x 576 14.7 / 17.6, 1,024 x 2,816 56 / 72, 5,632 x 1,024 72 / 118; 130 rows,
-// 4,128 x 1,024 27.7 / 46.8; 1,000 rows, 5,632 x 1,024 123 / 247; 33 rows, 5,632 x 1,024 23 / 31.5.  Below some 350,000 cells it is no faster: 446 rows, 576 x 576
+// Measured against the library's float32 product: 446 rows, 3,072 x 576 32 / 43.7 us, 960 x 576 15.2 / 17.6, 1,024 x 2,816 57 / 72, 5,632 x 1,024 74 / 118; 130 rows,
+// 4,128 x 1,024 27.4 / 46.8; 1,000 rows, 5,632 x 1,024 127 / 247; 33 rows, 5,632 x 1,024 24.3 / 31.5.  Below some 350,000 cells it is no faster: 446 rows, 576 x 576
 // 14.6 / 13.3, 576 x 1,536 32.3 / 30.2; 130 rows, 960 x 576 14.3 / 12.7.  2-norm of the error against 64 bits, of the result's: 0.9 to 1.5 x 10^-7 / 4 to 9 x 10^-7.
 //
-// Values that bfloat16 cannot hold (infinities, NaN, above its largest finite value) have no such parts: a CTA that meets one computes its cells again with
-// fused multiply-adds straight from memory, as it does after a wait that ran out.
+// What the parts cannot express is computed again, cell by cell, with fused multiply-adds straight from memory, as all cells are after a wait that ran out: the
+// cells of a row or column with a value that bfloat16 cannot hold (infinities, NaN, above its largest finite value); cells whose sum is not finite (of operands whose product passes float32's
+// range the large sum holds an infinity and a small one, whose parts have signs of their own, may hold the other); and cells so small beside their row and
+// column that low parts below the smallest normal number, which the tensor cores may take for zero, could show in the last place (pf_smallest).  Looking costs 0.2 to 0.5 us a CTA; one infinity in 446 rows, 3,072 x 576
+// 32 -> 56 us.
 //
-// Sizes: K % 4 == 0, 16-byte rows.  A row's result does not depend on the other rows.
+// Sizes: K % 4 == 0, 16-byte rows.  A row's result does not depend on the other rows: which way a cell goes depends on its row, its column and its sum alone.
 #include "tc05.cuh"
 
 namespace {
 
 constexpr int PF_ROWS = 128, PF_K = 64, PF_SPLITTERS = 8, PF_DRAINERS = 4, PF_STAGES = 2;
 constexpr int PF_THREADS = (PF_SPLITTERS + PF_DRAINERS + 1) * 32;
+
 constexpr float PF_LARGEST = 3.38e38f;                   // below what rounds to infinity in bfloat16 (3.3953e38)
 
 __device__ __forceinline__ float pf_max_nan(float a, float b) {      // NaN if either is
@@ -32,6 +36,10 @@ __device__ __forceinline__ float pf_max_nan(float a, float b) {      // NaN if e
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
     return y;
 }
+
+// Below this a sum may have lost something that matters.  Parts, products and sums below 2^-126 may be taken for zero: at most three parts of a value times the other
+// operand (at most `most_x` and `most_w`), and six products, at each of K places; that is 2^-24 of the sum and less from here on.
+__device__ __forceinline__ float pf_smallest(int K, float most_x, float most_w) { return (float)K * 1.9721523e-31f * (6.f + 3.f * (most_x + most_w)); }      // (2^-102)
 
 __device__ __forceinline__ void pf_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -60,13 +68,14 @@ products_f32_kernel(const float* __restrict__ x, long long ldx, const float* __r
     extern __shared__ __align__(1024) unsigned char tiles[];
     __shared__ __align__(8) unsigned long long bars[9];  // full[2], empty[2], large full[2], large free[2], done
     __shared__ uint32_t tmem_slot;
-    __shared__ int gave_up, odd_values;
+    __shared__ int gave_up;
+    __shared__ float most[PF_ROWS + BN];                 // the largest magnitude of each row of x, of each row of W
+    __shared__ uint32_t again[PF_ROWS][BN / 32];         // cells to be computed again
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.y * PF_ROWS, n0 = blockIdx.x * BN, steps = (K + PF_K - 1) / PF_K;
     const uint32_t full0 = ta_u32(&bars[0]), empty0 = ta_u32(&bars[2]), large0 = ta_u32(&bars[4]), free0 = ta_u32(&bars[6]), done = ta_u32(&bars[8]);
     if (tid == 0) {
         gave_up = (ta_u32(tiles) & 1023u) ? 1 : 0;       // (misaligned tiles would give wrong sums)
-        odd_values = 0;
         for (int s = 0; s < 2; ++s) {
             ta_bar_init(full0 + 8 * s, PF_SPLITTERS); ta_bar_init(empty0 + 8 * s, 1);
             ta_bar_init(large0 + 8 * s, 1); ta_bar_init(free0 + 8 * s, PF_DRAINERS);
@@ -96,7 +105,9 @@ products_f32_kernel(const float* __restrict__ x, long long ldx, const float* __r
         const float* wb = W + (size_t)(n0 + r0) * K + eighth * 8;
         // (rows past the last are neither split nor cleared: what their tiles hold enters cells that are not stored)
         auto there = [&](int j) { return j < AJ ? m0 + r0 + 32 * j < T : n0 + r0 + 32 * (j - AJ) < N; };
-        float largest = 0.f;
+        float largest[PIECES];
+#pragma unroll
+        for (int j = 0; j < PIECES; ++j) largest[j] = 0.f;
         auto fetch = [&](float4 (&v)[PIECES][2], int step) {
             const int k = step * PF_K + eighth * 8;
 #pragma unroll
@@ -118,8 +129,8 @@ products_f32_kernel(const float* __restrict__ x, long long ldx, const float* __r
                 uint4 h, m, l;
                 pf_split(v[j][0].x, v[j][0].y, h.x, m.x, l.x); pf_split(v[j][0].z, v[j][0].w, h.y, m.y, l.y);
                 pf_split(v[j][1].x, v[j][1].y, h.z, m.z, l.z); pf_split(v[j][1].z, v[j][1].w, h.w, m.w, l.w);
-                largest = pf_max_nan(pf_max_nan(pf_max_nan(fabsf(v[j][0].x), fabsf(v[j][0].y)), pf_max_nan(fabsf(v[j][0].z), fabsf(v[j][0].w))), largest);
-                largest = pf_max_nan(pf_max_nan(pf_max_nan(fabsf(v[j][1].x), fabsf(v[j][1].y)), pf_max_nan(fabsf(v[j][1].z), fabsf(v[j][1].w))), largest);
+                largest[j] = pf_max_nan(pf_max_nan(pf_max_nan(fabsf(v[j][0].x), fabsf(v[j][0].y)), pf_max_nan(fabsf(v[j][0].z), fabsf(v[j][0].w))), largest[j]);
+                largest[j] = pf_max_nan(pf_max_nan(pf_max_nan(fabsf(v[j][1].x), fabsf(v[j][1].y)), pf_max_nan(fabsf(v[j][1].z), fabsf(v[j][1].w))), largest[j]);
                 unsigned char* at = tiles + s * STAGE + (j < AJ ? 0u : 3 * A_PART) + row * 128 + ((eighth ^ (row & 7)) << 4);
                 *reinterpret_cast<uint4*>(at) = h;
                 *reinterpret_cast<uint4*>(at + part) = m;
@@ -139,7 +150,12 @@ products_f32_kernel(const float* __restrict__ x, long long ldx, const float* __r
             if (i + 1 >= steps || !put(odd, i + 1)) break;
             fetch(odd, i + 3);
         }
-        if (!(largest < PF_LARGEST)) odd_values = 1;
+#pragma unroll
+        for (int j = 0; j < PIECES; ++j) {               // (eight neighbouring lanes have a row)
+#pragma unroll
+            for (int o = 1; o < 8; o *= 2) largest[j] = pf_max_nan(largest[j], __shfl_xor_sync(0xffffffffu, largest[j], o));
+            if (eighth == 0) most[j < AJ ? r0 + 32 * j : PF_ROWS + r0 + 32 * (j - AJ)] = largest[j];
+        }
     } else if (warp == PF_SPLITTERS + PF_DRAINERS) {
         if (lane == 0) {
             for (int i = 0; i < steps; ++i) {
@@ -197,34 +213,74 @@ products_f32_kernel(const float* __restrict__ x, long long ldx, const float* __r
         ta_fence_before();
     }
     __syncthreads();
+    int any = 0;
     if (warp == PF_SPLITTERS + PF_DRAINERS) {
         ta_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS));
-        return;
-    }
-    if (warp < PF_SPLITTERS) return;
-    const int row = m0 + quarter * 32 + lane;
-    if (row >= T) return;
-    if (odd_values || gave_up) {
-        const float* xr = x + (size_t)row * ldx;
+    } else if (warp >= PF_SPLITTERS) {
+        const int mine = quarter * 32 + lane, row = m0 + mine;
+        if (row < T) {                                   // (what is computed again is stored again behind the barrier below)
+            float* o = out + (size_t)row * N + n0;
+            if (n0 + BN <= N && N % 4 == 0) {
 #pragma unroll
-        for (int j = 0; j < BN; ++j) {
-            if (n0 + j >= N) break;
-            const float* wr = W + (size_t)(n0 + j) * K;
-            float s = 0.f;
-#pragma unroll 1
-            for (int k = 0; k < K; ++k) s = fmaf(xr[k], wr[k], s);
-            sums[j] = s;
+                for (int j = 0; j < BN; j += 4) *reinterpret_cast<float4*>(o + j) = make_float4(sums[j], sums[j + 1], sums[j + 2], sums[j + 3]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < BN; ++j)
+                    if (n0 + j < N) o[j] = sums[j];
+            }
+        }
+        const float most_x = most[mine];
+        uint32_t odd[BN / 32];
+#pragma unroll
+        for (int p = 0; p < BN / 32; ++p) odd[p] = 0u;
+        // first all of a row's cells at once, against the largest value of any column: nearly always that is all
+        float most_w = most[PF_ROWS + lane], least[4], top[4];
+        if (BN > 32) most_w = pf_max_nan(most_w, most[PF_ROWS + BN - 32 + lane]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) most_w = pf_max_nan(most_w, __shfl_xor_sync(0xffffffffu, most_w, o));
+        if (n0 + BN > N) {                               // (cells of no column: some value that is in order)
+#pragma unroll
+            for (int j = 0; j < BN; ++j) sums[j] = n0 + j < N ? sums[j] : 1.f;
+        }
+#pragma unroll
+        for (int j = 0; j < BN; ++j) {                   // (four chains)
+            least[j % 4] = j < 4 ? fabsf(sums[j]) : fminf(least[j % 4], fabsf(sums[j]));
+            top[j % 4] = j < 4 ? fabsf(sums[j]) : pf_max_nan(top[j % 4], fabsf(sums[j]));
+        }
+        const bool fine = (most_x < PF_LARGEST) & (most_w < PF_LARGEST) & !gave_up & (pf_max_nan(pf_max_nan(top[0], top[1]), pf_max_nan(top[2], top[3])) < INFINITY) &
+                          (fminf(fminf(least[0], least[1]), fminf(least[2], least[3])) >= pf_smallest(K, most_x, most_w));
+        if (!fine && row < T) {
+#pragma unroll
+            for (int j = 0; j < BN; ++j) {
+                const float w = most[PF_ROWS + j], size = fabsf(sums[j]);
+                const bool zeros = (most_x == 0.f) | (w == 0.f), whole = (size >= pf_smallest(K, most_x, w)) & (size < INFINITY);
+                if (!((most_x < PF_LARGEST) & (w < PF_LARGEST) & (zeros | whole)) | (gave_up != 0)) odd[j / 32] |= 1u << (j % 32);
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < BN / 32; ++p) {
+            const int n = min(32, N - n0 - 32 * p);
+            odd[p] = row < T && n > 0 ? odd[p] & (0xffffffffu >> (32 - n)) : 0u;
+            again[mine][p] = odd[p];
+            any |= odd[p] != 0u;
         }
     }
-    float* o = out + (size_t)row * N + n0;
-    if (n0 + BN <= N && N % 4 == 0) {
-#pragma unroll
-        for (int j = 0; j < BN; j += 4) *reinterpret_cast<float4*>(o + j) = make_float4(sums[j], sums[j + 1], sums[j + 2], sums[j + 3]);
-    } else {
-#pragma unroll
-        for (int j = 0; j < BN; ++j)
-            if (n0 + j < N) o[j] = sums[j];
+    if (!__syncthreads_or(any)) return;
+    for (int r = warp; r < PF_ROWS; r += PF_THREADS / 32) {      // the cells that are computed again, a warp each
+#pragma unroll 1
+        for (int p = 0; p < BN / 32; ++p)
+            for (uint32_t left = again[r][p]; left != 0u; left &= left - 1u) {
+                const int n = n0 + 32 * p + __ffs(left) - 1;
+                const float4 *xr = reinterpret_cast<const float4*>(x + (size_t)(m0 + r) * ldx), *wr = reinterpret_cast<const float4*>(W + (size_t)n * K);
+                float s = 0.f;
+                for (int k = lane; k < K / 4; k += 32) {
+                    const float4 a = __ldg(xr + k), b = __ldg(wr + k);
+                    s = fmaf(a.x, b.x, s); s = fmaf(a.y, b.y, s); s = fmaf(a.z, b.z, s); s = fmaf(a.w, b.w, s);
+                }
+                s = vm_warp_sum(s);
+                if (lane == 0) out[(size_t)(m0 + r) * N + n] = s;
+            }
     }
 }
 
