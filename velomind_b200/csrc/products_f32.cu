@@ -13,13 +13,15 @@
 //
 // Measured against the library's float32 product: 446 rows, 3,072 x 576 32 / 43.7 us, 960 x 576 15.2 / 17.6, 1,024 x 2,816 57 / 72, 5,632 x 1,024 74 / 118; 130 rows,
 // 4,128 x 1,024 27.4 / 46.8; 1,000 rows, 5,632 x 1,024 127 / 247; 33 rows, 5,632 x 1,024 24.3 / 31.5.  Below some 350,000 cells it is no faster: 446 rows, 576 x 576
-// 14.6 / 13.3, 576 x 1,536 32.3 / 30.2; 130 rows, 960 x 576 14.3 / 12.7.  2-norm of the error against 64 bits, of the result's: 0.9 to 1.5 x 10^-7 / 4 to 9 x 10^-7.
+// 14.6 / 13.3, 576 x 1,536 32.3 / 30.2; 130 rows, 960 x 576 14.3 / 12.7.  Nor is it up to 32 rows, for which the library has kernels of its own, however many the
+// columns: 9 rows, 49,152 x 576 79 / 50, 49,152 x 2,048 236 / 158; 32 rows 83 / 51, 244 / 163, 12,288 x 2,048 112 / 68; but 33 rows 86 / 83, 252 / 311, 85 / 86;
+// 64 rows 90 / 97, 259 / 321, 88 / 86, 32,000 x 1,024 95 / 87; 96 rows and more are faster at every size.  2-norm of the error against 64 bits, of the result's: 0.9 to 1.5 x 10^-7 / 4 to 9 x 10^-7.
 //
 // What the parts cannot express is computed again, cell by cell, with fused multiply-adds straight from memory, as all cells are after a wait that ran out: the
-// cells of a row or column with a value that bfloat16 cannot hold (infinities, NaN, above its largest finite value); cells whose sum is not finite (of operands whose product passes float32's
-// range the large sum holds an infinity and a small one, whose parts have signs of their own, may hold the other); and cells so small beside their row and
-// column that low parts below the smallest normal number, which the tensor cores may take for zero, could show in the last place (pf_smallest).  Looking costs 0.2 to 0.5 us a CTA; one infinity in 446 rows, 3,072 x 576
-// 32 -> 56 us.
+// cells of a row or column with a value that bfloat16 cannot hold (infinities, NaN, above its largest finite value); cells whose sum is not finite (of operands
+// whose product passes float32's range the large sum holds an infinity and a small one, whose parts have signs of their own, may hold the other); and cells so
+// small beside their row and column that low parts below the smallest normal number, which the tensor cores may take for zero, could show in the last place
+// (pf_smallest).  Looking costs 0.2 to 0.5 us a CTA; one infinity in 446 rows, 3,072 x 576 32 -> 56 us.
 //
 // Sizes: K % 4 == 0, 16-byte rows.  A row's result does not depend on the other rows: which way a cell goes depends on its row, its column and its sum alone.
 #include "tc05.cuh"
@@ -28,7 +30,6 @@ namespace {
 
 constexpr int PF_ROWS = 128, PF_K = 64, PF_SPLITTERS = 8, PF_DRAINERS = 4, PF_STAGES = 2;
 constexpr int PF_THREADS = (PF_SPLITTERS + PF_DRAINERS + 1) * 32;
-
 constexpr float PF_LARGEST = 3.38e38f;                   // below what rounds to infinity in bfloat16 (3.3953e38)
 
 __device__ __forceinline__ float pf_max_nan(float a, float b) {      // NaN if either is
@@ -308,8 +309,8 @@ int choose_columns(int T, int N) {
 
 }  // namespace
 
-// 1 where vm_products_f32 is the faster one (see above); it takes fewer cells too
-VM_API int vm_products_f32_pays(int T, int N) { return (long long)T * N >= 350000 ? 1 : 0; }
+// 1 where vm_products_f32 is the faster one (see above); it takes fewer rows and cells too
+VM_API int vm_products_f32_pays(int T, int N) { return T > 32 && (long long)T * N >= 350000 ? 1 : 0; }
 
 // 1 if vm_products_f32 takes these rows (whole 16-byte pieces)
 VM_API int vm_products_f32_fits(const void* x, long long ldx, const void* w, const void* out, int T, int K) {

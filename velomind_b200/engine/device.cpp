@@ -379,7 +379,7 @@ void linear(const void* x, DType x_dtype, long long ldx, const DeviceTensor& W, 
               "linear", s);
         return;
     }
-    // many cells in float32: split products on the tensor cores (both sides measured in csrc/products_f32.cu)
+    // many rows and cells in float32: split products on the tensor cores (both sides measured in csrc/products_f32.cu)
     if (x_dtype == DType::F32 && vm_products_f32_pays(T, static_cast<int>(W.rows())) && vm_products_f32_fits(x, ldx, W.ptr, out, T, static_cast<int>(W.cols()))) {
         check(vm_products_f32(static_cast<const float*>(x), ldx, static_cast<const float*>(W.ptr), static_cast<float*>(out), T, static_cast<int>(W.rows()),
                               static_cast<int>(W.cols()), s),
