@@ -60,6 +60,45 @@ def test_products_of_plain_rows(M, N, K):
     assert bool(((unit.double() - silu * up).abs() <= loose + (silu * up).abs() * (2.0 ** -8 + 2.0 ** -20) + 1e-30).all())
 
 
+# either side of the rule: 8 rows and 9 of 18 MB and more, 17 of 10 MB and more, column tiles of eight, two pairs of tiles a block, blocks for one SM and a half
+@pytest.mark.parametrize("form,M,N,K,ring", [("gated", 9, 6144, 2048, True), ("gated", 8, 6144, 2048, False), ("sum", 16, 6144, 1536, True), ("sum", 17, 5632, 960, True), ("sum", 17, 5120, 960, False),
+                                             ("gated", 32, 16384, 1024, True), ("gated", 17, 12288, 960, False), ("store", 17, 4088, 1280, True), ("store", 5, 4088, 4096, True), ("store", 9, 4088, 2048, True),
+                                             ("store", 16, 3200, 4096, False), ("sum", 32, 3072, 2048, False)])
+def test_plain_rows_of_many_weights(form, M, N, K, ring):
+    """Where memory sets the time, plain rows take the kernel that stages them once a CTA: its bits; and either kernel's sums are right, bounds as above."""
+    g = torch.Generator().manual_seed(M + N + K)
+    x, w = _bf(torch.randn(M, K, generator=g)), _bf(torch.randn(N, K, generator=g) * 0.1)
+    h0, err = torch.randn(M, N, generator=g).to(DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(variant):
+        out, h = torch.full((M, N), float("nan"), device=DEV), h0.clone()
+        unit = torch.full((M, N // 2), float("nan"), dtype=torch.bfloat16, device=DEV)
+        _lib().vm_skinny_variant(_i(variant))
+        try:
+            if form == "gated":
+                rc = _lib().vm_skinny_gated(_p(x), _i(0), _p(None), _f(0), _p(w), _i(M), _i(N // 2), _i(K), _i(0), _p(unit), _p(err), _stream())
+            else:
+                rc = _lib().vm_skinny_linear(_p(x), _i(0), _p(None), _f(0), _p(w), _i(M), _i(N), _i(K), _p(out), _i(N), _i(1), _p(h if form == "sum" else None), _p(err), _stream())
+        finally:
+            _lib().vm_skinny_variant(_i(0))
+        assert rc == 0
+        return {"gated": unit, "sum": h, "store": out}[form]
+
+    got = run(0)
+    if ring:
+        assert torch.equal(got, run(2))
+    want = x.double() @ w.double().T
+    bound = (x.double().abs() @ w.double().abs().T + (h0.double().abs() if form == "sum" else 0)) * (K + 1) * 2.0 ** -24
+    if form == "gated":
+        gate, up = want[:, :N // 2], want[:, N // 2:]
+        bg, bu = bound[:, :N // 2], bound[:, N // 2:]
+        silu = gate / (1 + torch.exp(-gate))
+        want, bound = silu * up, 1.1 * bg * up.abs() + (silu.abs() + bg) * bu + (silu * up).abs() * (2.0 ** -8 + 2.0 ** -20) + 1e-30
+    elif form == "sum":
+        want = want + h0.double()
+    assert bool(((got.double() - want).abs() <= bound).all()) and int(err.item()) == 0
+
+
 @pytest.mark.parametrize("M,N,K", SIZES)
 def test_rows_left_ready(M, N, K):
     """The residual sum, the rows for the next product and their sums of squares."""

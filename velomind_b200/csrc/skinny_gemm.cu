@@ -21,10 +21,10 @@
 // it waits for its predecessor; the rope_kv form lets ITS successor, the decode attention, start only after that wait
 // (common.cuh says why).
 //
-// Rows that lie ready in bfloat16 (at most 32 of them) take skinny_direct_kernel (skinny_direct.cu) whatever the size; the kernels here are for the norm
-// as a prologue, for the vocabulary head and for more rows.
+// Rows that lie ready in bfloat16 (at most 32 of them) take skinny_direct_kernel (skinny_direct.cu) but for 9 and more plain rows of many megabytes of
+// weights (ring_pays); the kernels here are for those, for the norm as a prologue, for the vocabulary head and for more rows.
 //
-// Products with the norm that read many megabytes of weights for at most 32 rows take skinny_stream_kernel (skinny_stream.cuh): the same
+// Products with the norm, and those, that read many megabytes of weights for at most 32 rows take skinny_stream_kernel (skinny_stream.cuh): the same
 // work items and epilogues, the weights streamed through shared memory by a warp of their own.
 //
 // Sizes: K % 32 == 0, N % 8 == 0 (16 for the two-tile forms), head size % 16 == 0, I % 8 == 0; M <= 64.
@@ -142,9 +142,23 @@ int skinny_variant = 0;
 constexpr long long STREAM_MIN_WEIGHT_BYTES = 9ll << 20;
 constexpr long long STREAM_MIN_WEIGHT_BYTES_TWO_ROWS = 9ll << 19;      // 4.5 MB: with one or two rows there is next to no prologue
 
+// Plain rows whose weights are so many that memory sets the time, not a chain of latencies: the ring kernel, which stages the rows once a CTA, where every block of
+// the direct kernel fetches them anew.  Measured, direct / ring: up to 8 rows 0.4 to 1.05 times as long nearly everywhere (24,576 x 960 with the sum 11.5 / 11.0 us, 16,384 x 2,048
+// gated 13.6 / 13.6; K of 4,096 and more 0.7 to 1.1) but for column tiles of eight alone (4,088 x 4,096 12.9 / 11.6; 9 rows 13.5 / 11.7, 4,088 x 2,048 8.4 / 7.8).  9 rows: 6,144 x 2,048 gated 8.8 / 8.1, 16,384 x 2,048 16.9 / 14.1, 16,384 x 576 with the sum
+// 8.6 / 7.7, but with two pairs of tiles a block 16,384 x 1,024 gated 8.9 / 9.2, and rows that fill shared memory 8,192 x 4,096 gated 15.8 / 16.4.  17 rows, where the
+// direct kernel has four tiles of rows a block: 6,144 x 2,048 gated 14.1 / 11.1, 16,384 x 2,048 32.5 / 21.8, 5,632 x 960 with the sum 8.3 / 7.5, 12,288 x 960 15.9 / 12.0; with
+// two pairs 12,288 x 960 gated 11.9 / 12.7, 16,384 x 1,024 16.3 / 15.6; blocks for one and a half SMs and less 3,072 x 8,192 30 / 34.5, 2,048 x 8,192 with the sum 14.6 / 31.5.
+bool ring_pays(const SkinnyParams& p, int items) {
+    const long long bytes = (long long)p.N * p.K * 2, sms = vm_sm_count();
+    const bool two_pairs = (p.epi == EPI_SWIGLU || p.epi == EPI_STORE_BF16 || p.epi == EPI_STORE_F32) && items > sms && p.K <= 1024;
+    if (p.M <= 8) return p.tiles == 1 && bytes >= 32000000;
+    if (p.M <= 16) return (p.tiles == 1 && bytes >= 16000000) || (!two_pairs && items > 2 * sms && p.K <= 2048 && bytes >= 18000000);
+    return two_pairs ? bytes >= 32000000 : 2 * items > 3 * sms && bytes >= 10000000;
+}
+
 int skinny_dispatch(SkinnyParams p, int items, cudaStream_t stream) {
     if (p.squares || p.next_w) return vm_skinny_direct(p, items, stream);
-    if (skinny_variant == 0 && p.pro == PRO_NONE && p.M <= 32) return vm_skinny_direct(p, items, stream);
+    if (skinny_variant == 0 && p.pro == PRO_NONE && p.M <= 32 && !ring_pays(p, items)) return vm_skinny_direct(p, items, stream);
     const long long weight_bytes = (long long)p.N * p.K * 2;
     if (skinny_variant >= 2 || (skinny_variant == 0 && p.M <= 32 && weight_bytes >= (p.M <= 2 ? STREAM_MIN_WEIGHT_BYTES_TWO_ROWS : STREAM_MIN_WEIGHT_BYTES))) {
         const int rc = skinny_stream_launch(p, items, stream, skinny_variant == 3 ? 2 : (skinny_variant == 4 ? 1 : 0));
