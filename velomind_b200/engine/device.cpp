@@ -518,10 +518,15 @@ void attention(StepContext& ctx, const void* q, int q_row_stride, const KVView& 
         // kernel below, which deals them out by their length, unless the sequences are long on average.  Measured, mma.sync / warp-specialised / tcgen05: 9 heads, one
         // prompt of 1,536 tokens 23.6 / 26.2 / 23.8 us, of 2,048 30.2 / 31.6 / 37.7, of 3,000 52.6 / 50.3 / 57.5; 15 heads, 2,048 40.5 / 38.9 / 46, sixteen of 64 to 1,024
         // 53 / 71 / 86; 16 heads, 1,400 + 2,000 52.8 / 53.4 / 67.  Behind a cached prefix every tile is long, and where there are fewer tiles than that a tile's keys
-        // are dealt out to several CTAs: by the table's width, as far as the two kernels below go.
+        // are dealt out to several CTAs: by the table's width, as far as the two kernels below go.  (More tiles than the list holds are not dealt out: the
+        // mma.sync kernel is 8 to 15 % slower then, and the line between the two lies where it did: 9 / 16 / 32 heads, twenty prompts of 1,024 115 / 90, 190 / 171,
+        // 362 / 295 us, forty of 512 74 / 72, 123 / 129, 234 / 261.)
         const bool dealt = D == 64 && kv.table_width < 2 * newest && 5 * items > 7 * sms;
-        // (many tiles of middling length keep the warp-specialised kernel's CTAs busy: 15 heads, four prompts of 1,024 tokens 43 us; 32 heads, three of 1,024 61 / 55 for
-        //  the mma.sync kernel, four of 1,000 to 3,000 222 / 271.  Short prompts beside long ones do not, each pays for a CTA's set-up)
+        // (many tiles of middling length keep the warp-specialised kernel's CTAs busy, short prompts beside long ones do not, each pays for a CTA's set-up.  Measured, mma.sync /
+        //  warp-specialised: 15 heads, three prompts of 1,500 59 / 54, eight of 2,048 233 / 188; 16 heads, four of 1,024 41 / 34, three of 1,500 62 / 44; 32 heads, two of 3,000
+        //  259 / 172, four of 1,000 to 3,000 244 / 200.  The lines are by mean length alone and take the slower kernel where the other's last wave of clusters is nearly
+        //  empty: 9 heads, eight of 800 33 / 42, two of 3,000 82 / 89; 15 heads, four of 1,024 39 / 43; 16 heads, eight of 800 51 / 62, one of 2,048 44 / 53; 32 heads, three of
+        //  1,024 57 / 61, eight of 800 97 / 108)
         const bool many = most_blocks >= WS_ATTENTION_MANY_BLOCKS && tiles128 * H >= 3 * sms &&
                           blocks128 >= (dealt ? WS_ATTENTION_MEAN_BLOCKS_DEALT : WS_ATTENTION_MEAN_BLOCKS) * tiles128;
         const bool long_ones = dealt ? blocks128 >= WS_ATTENTION_MIN_BLOCKS * tiles128 : most_blocks >= WS_ATTENTION_MIN_BLOCKS;
