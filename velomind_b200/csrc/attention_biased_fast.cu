@@ -271,12 +271,9 @@ int launch_biased_prefill(const void* q, int q_row_stride, const void* kpages, c
     const size_t smem = (size_t)(BM + 2 * BN) * (DK + 8) * sizeof(__nv_bfloat16) + (VK ? 0 : (size_t)2 * BN * (DV + 8) * sizeof(__nv_bfloat16)) +
                         (size_t)table * sizeof(float);
     if (smem > 200 * 1024) return VM_ERR_UNSUPPORTED;
-    static size_t raised = 48 * 1024;                       // per instantiation
-    if (smem > raised) {
-        cudaError_t e = cudaFuncSetAttribute(attn_biased_prefill_kernel<DK, DV, VK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        raised = smem;
-    }
+    static VmOncePerDevice once;
+    const cudaError_t e = smem > 48 * 1024 ? vm_allow_smem(once, attn_biased_prefill_kernel<DK, DV, VK>, 200 * 1024) : cudaSuccess;
+    if (e != cudaSuccess) return (int)e;
     // (not as a programmatic dependent: CTAs that start while the kernel in front still holds some SMs are not dealt out in turn)
     attn_biased_prefill_kernel<DK, DV, VK><<<dim3(n_tiles, H), 128, smem, stream>>>(
         (const __nv_bfloat16*)q, q_row_stride, (const __nv_bfloat16*)kpages, (const __nv_bfloat16*)vpages, block_table, max_blocks, positions,

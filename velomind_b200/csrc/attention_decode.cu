@@ -39,12 +39,9 @@ int launch_decode(dim3 grid, cudaStream_t stream, const __nv_bfloat16* q, int q_
                   __nv_bfloat16* out, float* partial, int* counters, int H, int Hkv, float scale, int window, int n_pages,
                   int* err, int in_step) {
     const size_t smem = attn_decode_smem_bytes<D, WARPS>();
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<D, WARPS, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static VmOncePerDevice once;
+    const cudaError_t e = vm_allow_smem(once, attn_decode_kernel<D, WARPS, AHEAD>, smem);
+    if (e != cudaSuccess) return (int)e;
     vm_launch_pdl(attn_decode_kernel<D, WARPS, AHEAD>, grid, dim3(WARPS * 32), smem, stream, q, q_row_stride, kpages, vpages, block_table,
                   max_blocks, positions, out, partial, counters, H, Hkv, scale * 1.4426950408889634f, window, n_pages, err, in_step);
     return vm_launch_status();

@@ -281,12 +281,9 @@ int launch_prefill_ng(const void* q, int q_row_stride, const void* kpages, const
     size_t smem = (size_t)(BM + 4 * NG * BN) * DP * sizeof(__nv_bfloat16);
     const size_t merge = (size_t)(NG - 1) * BM * (D + 2) * sizeof(float) + (size_t)BM * DP * sizeof(__nv_bfloat16);
     if (merge > smem) smem = merge;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_mma_kernel<D, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static VmOncePerDevice once;
+    const cudaError_t e = vm_allow_smem(once, attn_prefill_mma_kernel<D, NG>, smem);
+    if (e != cudaSuccess) return (int)e;
     dim3 grid(n_tiles, H);
     // (not as a programmatic dependent: CTAs that start while the kernel in front still holds some SMs are not dealt out in turn)
     attn_prefill_mma_kernel<D, NG><<<grid, 128 * NG, smem, stream>>>(

@@ -327,12 +327,9 @@ template <int NC>
 int ta_launch(int n_tiles, int H, cudaStream_t stream, const __nv_bfloat16* q, int q_row_stride, const __nv_bfloat16* kpages,
               const __nv_bfloat16* vpages, const int* block_table, int max_blocks, const int* positions, const int* cu_tokens,
               int B, __nv_bfloat16* out, int Hkv, float scale_log2, int window, int n_pages, int* err) {
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, TA_SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static VmOncePerDevice once;
+    const cudaError_t allowed = vm_allow_smem(once, attn_prefill_tc_kernel<NC>, TA_SMEM);
+    if (allowed != cudaSuccess) return (int)allowed;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_tiles * NC, H); cfg.blockDim = dim3(TA_THREADS); cfg.dynamicSmemBytes = TA_SMEM; cfg.stream = stream;
     cudaLaunchAttribute attr[1];

@@ -645,12 +645,9 @@ int ws_active_clusters(int nc) {
 template <int NT>
 int ws_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const WsParams& p, long long units, int grid_y, int est_blocks, int groups,
               cudaStream_t stream) {
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_ws_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws_smem_bytes<NT>());
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static VmOncePerDevice once;
+    const cudaError_t allowed = vm_allow_smem(once, attn_prefill_ws_kernel<NT>, ws_smem_bytes<NT>());
+    if (allowed != cudaSuccess) return (int)allowed;
     int nc = groups;
     if (nc <= 0) {
         // As many CTAs per cluster as make the step shortest, in key blocks of one CTA (about 1.75 us each, measured): waves of

@@ -112,13 +112,8 @@ int launch_scan(const float* proj, int ld, const float* bias_i, const float* bia
     if (threads > 1024) return VM_ERR_UNSUPPORTED;
     const size_t smem = ((size_t)D * V + 4 * D + 8 + 4 * (threads / 32)) * sizeof(float);
     if (smem > 200 * 1024) return VM_ERR_UNSUPPORTED;
-    if (smem > 48 * 1024) {
-        static size_t raised = 0;       // per instantiation
-        if (smem > raised) {
-            if (cudaFuncSetAttribute(mlstm_scan_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return vm_launch_status();
-            raised = smem;
-        }
-    }
+    static VmOncePerDevice once;
+    if (smem > 48 * 1024 && vm_allow_smem(once, mlstm_scan_kernel<T>, 200 * 1024) != cudaSuccess) return vm_launch_status();
     vm_launch_pdl(mlstm_scan_kernel<T>, dim3(H, B), dim3(threads), smem, stream, proj, ld, bias_i, bias_f, norm_w, state, cu_tokens, slots, (T*)out, H, D,
                   V, cap, eps);
     return vm_launch_status();
@@ -690,13 +685,10 @@ VM_API int vm_mlstm_chunks(const float* proj, int ld, const float* bias_i, const
     if (act_dtype != VM_F32 && act_dtype != VM_BF16) return VM_ERR_UNSUPPORTED;
     const ChunkSizes c = chunk_sizes(D, V);
     if (c.smem > 200 * 1024) return VM_ERR_UNSUPPORTED;
-    static size_t raised = 0;
-    if (c.smem > 48 * 1024 && c.smem > raised) {
-        if (cudaFuncSetAttribute(mlstm_chunk_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem) != cudaSuccess ||
-            cudaFuncSetAttribute(mlstm_chunk_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem) != cudaSuccess)
-            return vm_launch_status();
-        raised = c.smem;
-    }
+    static VmOncePerDevice once[2];
+    if (c.smem > 48 * 1024 && (vm_allow_smem(once[0], mlstm_chunk_local_kernel, 200 * 1024) != cudaSuccess ||
+                               vm_allow_smem(once[1], mlstm_chunk_finish_kernel, 200 * 1024) != cudaSuccess))
+        return vm_launch_status();
     const long long chunks = (long long)T / c.L + B + 1;          // at least sum over sequences of ceil(n / L)
     if (chunks > 65535) return VM_ERR_UNSUPPORTED;
     float* o_raw = scratch;

@@ -216,15 +216,9 @@ int launch_experts(const void* x, const float* norm_w, float eps, const void* w_
     const int warps = 8;
     const size_t up_smem = (size_t)hidden * sizeof(float), down_smem = (size_t)act_cols * sizeof(float);
     if (up_smem > 200 * 1024 || down_smem > 200 * 1024) return VM_ERR_UNSUPPORTED;
-    static size_t up_raised = 48 * 1024, down_raised = 48 * 1024;       // per instantiation
-    if (up_smem > up_raised) {
-        if (cudaFuncSetAttribute(experts_up_kernel<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)up_smem) != cudaSuccess) return vm_launch_status();
-        up_raised = up_smem;
-    }
-    if (down_smem > down_raised) {
-        if (cudaFuncSetAttribute(experts_down_kernel<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)down_smem) != cudaSuccess) return vm_launch_status();
-        down_raised = down_smem;
-    }
+    static VmOncePerDevice once[2];       // per instantiation
+    if (up_smem > 48 * 1024 && vm_allow_smem(once[0], experts_up_kernel<T, W>, 200 * 1024) != cudaSuccess) return vm_launch_status();
+    if (down_smem > 48 * 1024 && vm_allow_smem(once[1], experts_down_kernel<T, W>, 200 * 1024) != cudaSuccess) return vm_launch_status();
     const int per_block = warps * ROWS_PER_WARP;
     vm_launch_pdl(experts_up_kernel<T, W>, dim3((rows + per_block - 1) / per_block, T_), dim3(warps * 32), (size_t)hidden * sizeof(float), stream, x, norm_w, eps,
                   (const W*)w_up, (const W*)w_up_shared, chosen, hidden, ff, ff_shared, top, act_kind, act_kind_shared, E_real, glu, limit, alpha, act_cols,

@@ -617,24 +617,18 @@ VM_API int vm_sample(const float* logits, long long row_stride, int R, int V, co
         const int slice = ((V + SC_CTAS - 1) / SC_CTAS + 3) / 4 * 4;
         const size_t smem = (size_t)slice * sizeof(float);
         if (smem <= SAMPLE_CACHE_LIMIT) {
-            static bool configured_c = false;
-            if (!configured_c) {
-                cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_CACHE_LIMIT);
-                if (e != cudaSuccess) return (int)e;
-                configured_c = true;
-            }
+            static VmOncePerDevice once;
+            const cudaError_t e = vm_allow_smem(once, sample_cluster_kernel, SAMPLE_CACHE_LIMIT);
+            if (e != cudaSuccess) return (int)e;
             sample_cluster_kernel<<<R * SC_CTAS, SC_THREADS, smem, stream>>>(logits, row_stride, V, slice, temperature, top_p, seed,
                                                                            stream_id, step, step_add, out);
             return vm_launch_status();
         }
     }
     if (cache <= SAMPLE_CACHE_LIMIT) {
-        static bool configured = false;
-        if (!configured) {
-            cudaError_t e = cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_CACHE_LIMIT);
-            if (e != cudaSuccess) return (int)e;
-            configured = true;
-        }
+        static VmOncePerDevice once;
+        const cudaError_t e = vm_allow_smem(once, sample_kernel<true>, SAMPLE_CACHE_LIMIT);
+        if (e != cudaSuccess) return (int)e;
         sample_kernel<true><<<R, SAMPLE_THREADS, cache, stream>>>(logits, row_stride, V, temperature, top_p, seed, stream_id, step, step_add, out);
     } else {
         sample_kernel<false><<<R, SAMPLE_THREADS, 0, stream>>>(logits, row_stride, V, temperature, top_p, seed, stream_id, step, step_add, out);

@@ -384,12 +384,9 @@ int launch_scan_mode(const ScanParams& p, int n_pieces, cudaStream_t stream) {
 #define VM_SEL(NPT)                                                                             \
     if (p.N <= 4 * NPT) {                                                                       \
         constexpr int smem = SS_STAGES * ss_stage_bytes<T, NPT>();                              \
-        static bool raised = false;                                                             \
-        if (smem > 32 * 1024 && !raised) {                                                      \
-            cudaError_t e = cudaFuncSetAttribute(selective_scan_kernel<T, NPT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
-            if (e != cudaSuccess) return (int)e;                                                \
-            raised = true;                                                                      \
-        }                                                                                       \
+        static VmOncePerDevice once;                                                            \
+        const cudaError_t e = smem > 32 * 1024 ? vm_allow_smem(once, selective_scan_kernel<T, NPT, MODE>, smem) : cudaSuccess; \
+        if (e != cudaSuccess) return (int)e;                                                    \
         selective_scan_kernel<T, NPT, MODE><<<grid, SS_THREADS, smem, stream>>>(p);             \
         return vm_launch_status();                                                              \
     }

@@ -67,12 +67,9 @@ int skinny_wide_launch(SkinnyParams p, cudaStream_t stream) {
     const int grid = (p.N / 8 + SK_WARPS - 1) / SK_WARPS;
 #define VM_SKW_CASE(X)                                                                                                \
     case X: {                                                                                                         \
-        static size_t configured = 0;                                                                                 \
-        if (smem > 48 * 1024 && smem > configured) {                                                                  \
-            cudaError_t e = cudaFuncSetAttribute(skinny_wide_kernel<X>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
-            if (e != cudaSuccess) return (int)e;                                                                      \
-            configured = 200 * 1024;                                                                                  \
-        }                                                                                                             \
+        static VmOncePerDevice once;                                                                                  \
+        const cudaError_t e = smem > 48 * 1024 ? vm_allow_smem(once, skinny_wide_kernel<X>, 200 * 1024) : cudaSuccess; \
+        if (e != cudaSuccess) return (int)e;                                                                          \
         vm_launch_pdl(skinny_wide_kernel<X>, dim3(grid), dim3(SK_THREADS), smem, stream, p);                          \
     } break;
     switch (MT) { VM_SKW_CASE(1) VM_SKW_CASE(2) VM_SKW_CASE(4) }
@@ -112,12 +109,9 @@ int skinny_launch(SkinnyParams p, int grid, cudaStream_t stream) {
     const bool few = kc <= SK_WARPS * 32 * 4;
 #define VM_SK_CASE(X, P, L)                                                                                           \
     {                                                                                                                 \
-        static size_t configured = 0;                                                                                 \
-        if (smem > 48 * 1024 && smem > configured) {                                                                  \
-            cudaError_t e = cudaFuncSetAttribute(skinny_gemm_kernel<X, P, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); \
-            if (e != cudaSuccess) return (int)e;                                                                      \
-            configured = 160 * 1024;                                                                                  \
-        }                                                                                                             \
+        static VmOncePerDevice once;                                                                                  \
+        const cudaError_t e = smem > 48 * 1024 ? vm_allow_smem(once, skinny_gemm_kernel<X, P, L>, 160 * 1024) : cudaSuccess; \
+        if (e != cudaSuccess) return (int)e;                                                                          \
         vm_launch_pdl(skinny_gemm_kernel<X, P, L>, dim3(grid), dim3(SK_THREADS), smem, stream, p);                    \
     }
 #define VM_SK_ROWS(X)                                                                                                 \

@@ -374,12 +374,9 @@ inline int skinny_stream_launch(SkinnyParams p, int items, cudaStream_t stream, 
     const size_t smem = (size_t)stream_layout(p.M, p.K, rows, stage_rows, S, groups).total;
 #define VM_SS_CASE(X, G, P)                                                                                           \
     {                                                                                                                 \
-        static bool configured = false;                                                                               \
-        if (!configured) {                                                                                            \
-            cudaError_t e = cudaFuncSetAttribute(skinny_stream_kernel<X, G, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_BYTES - CTA_RESERVED); \
-            if (e != cudaSuccess) return (int)e;                                                                      \
-            configured = true;                                                                                        \
-        }                                                                                                             \
+        static VmOncePerDevice once;                                                                                  \
+        const cudaError_t e = vm_allow_smem(once, skinny_stream_kernel<X, G, P>, SM_BYTES - CTA_RESERVED);            \
+        if (e != cudaSuccess) return (int)e;                                                                          \
         vm_launch_pdl(skinny_stream_kernel<X, G, P>, dim3(grid), dim3(G * (SS_CW + P) * 32), smem, stream, p);        \
     }
     if (MT == 2) VM_SS_CASE(2, 1, 4) else if (groups == 2) VM_SS_CASE(1, 2, 2) else VM_SS_CASE(1, 1, 2)

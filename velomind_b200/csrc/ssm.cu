@@ -588,13 +588,10 @@ int launch_chunks_mma(const __nv_bfloat16* xbc, int C, const __nv_bfloat16* proj
     float* dS = scratch;
     float* decay = dS + (size_t)n_chunks * H * N * P;
     const size_t smem1 = ((size_t)3 * CL * XP + (size_t)CL * (N + 8)) * 2, smem3 = ((size_t)CL * XP + (size_t)3 * NT * XP + (size_t)2 * CL * (N + 8)) * 2;
-    static bool raised = false;           // per instantiation, for the largest sizes it takes
-    if (!raised) {
-        const int most1 = (3 * CL * XP + CL * 264) * 2, most3 = (CL * XP + 3 * NT * XP + 2 * CL * 264) * 2;
-        if (cudaFuncSetAttribute(ssm_mma_adds_kernel<PB>, cudaFuncAttributeMaxDynamicSharedMemorySize, most1) != cudaSuccess) return vm_launch_status();
-        if (cudaFuncSetAttribute(ssm_mma_out_kernel<PB>, cudaFuncAttributeMaxDynamicSharedMemorySize, most3) != cudaSuccess) return vm_launch_status();
-        raised = true;
-    }
+    static VmOncePerDevice once[2];       // per instantiation, for the largest sizes it takes
+    const int most1 = (3 * CL * XP + CL * 264) * 2, most3 = (CL * XP + 3 * NT * XP + 2 * CL * 264) * 2;
+    if (vm_allow_smem(once[0], ssm_mma_adds_kernel<PB>, most1) != cudaSuccess || vm_allow_smem(once[1], ssm_mma_out_kernel<PB>, most3) != cudaSuccess)
+        return vm_launch_status();
     ssm_mma_adds_kernel<PB><<<dim3(n_chunks, H), MMA_THREADS, smem1, stream>>>(xbc, C, proj, ld, dt_col, dt_bias, A_log, cu_tokens, B, dS, decay, H, P, N, G);
     int st = vm_launch_status();
     if (st) return st;
@@ -615,12 +612,9 @@ int launch_chunks_pc(const void* xbc, int C, const void* proj, int ld, int dt_co
     float* decay = cum + (size_t)T_ * H;
     const size_t smem1 = ((size_t)3 * CL * LDT + (size_t)2 * CL * XP + 2 * CL) * sizeof(float);
     const size_t smem3 = ((size_t)CL * LDT + (size_t)NT * XP) * sizeof(float);
-    static bool raised = false;           // per instantiation
-    if (!raised) {
-        if (cudaFuncSetAttribute(ssm_chunk_local_kernel<T, PC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess) return vm_launch_status();
-        if (cudaFuncSetAttribute(ssm_chunk_finish_kernel<T, PC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3) != cudaSuccess) return vm_launch_status();
-        raised = true;
-    }
+    static VmOncePerDevice once[2];       // per instantiation
+    if (vm_allow_smem(once[0], ssm_chunk_local_kernel<T, PC>, smem1) != cudaSuccess || vm_allow_smem(once[1], ssm_chunk_finish_kernel<T, PC>, smem3) != cudaSuccess)
+        return vm_launch_status();
     ssm_chunk_local_kernel<T, PC><<<dim3(n_chunks, H), 256, smem1, stream>>>((const T*)xbc, C, (const T*)proj, ld, dt_col, dt_bias, A_log, cu_tokens, B, y,
                                                                             dS, cum, decay, H, P, N, G);
     int st = vm_launch_status();

@@ -22,6 +22,7 @@
 // Every wait on an mbarrier is bounded; when a wait gives up, the CTA raises an error word, waits (bounded)
 // for its own copies in flight, frees its tensor memory and returns.
 #include <cuda.h>
+#include <algorithm>
 #include "mma.cuh"
 
 namespace {
@@ -459,21 +460,16 @@ int tc_launch(const void* A, long long lda, const void* W, TcParams p, int tiles
     }
     constexpr int STAGES = 3;
     const size_t smem = (size_t)STAGES * TC_KPS * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + 4 * 4096 + 128;   // stages, epilogue staging, barriers
-    static bool configured = false;
-    static int num_sms = 0;
-    static int per_sm = 1;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(tc_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+    static VmOncePerDevice once;
+    const cudaError_t allowed = vm_allow_smem(once, tc_gemm_kernel<BN>, smem);
+    if (allowed != cudaSuccess) return (int)allowed;
+    const int num_sms = vm_sm_count() > 0 ? vm_sm_count() : 1;
+    static int per_sm = 0;                                 // (of the kernel: the same on every device of this kind)
+    if (per_sm == 0) {
         int occ = 1;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, tc_gemm_kernel<BN>, TC_THREADS, smem) != cudaSuccess || occ < 1) occ = 1;
         const int by_tmem = 512 / (2 * BN);                // tensor memory: 2 x BN columns per CTA of 512 per SM
-        per_sm = occ < by_tmem ? occ : by_tmem;
-        if (per_sm > 2) per_sm = 2;
-        configured = true;
+        per_sm = std::min(std::min(occ, by_tmem), 2);
     }
     p.tiles_n = tiles_n;
     p.tiles_m = (p.M + TC_BM - 1) / TC_BM;
