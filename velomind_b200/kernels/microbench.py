@@ -100,6 +100,8 @@ def main(argv=None) -> int:
     ap.add_argument("--temp", type=float, default=0.0, help="sample: temperature (0: greedy)")
     ap.add_argument("--top-p", type=float, default=0.9, help="sample: nucleus mass, with --temp")
     ap.add_argument("--variant", type=int, default=0, help="weight-streaming products: 0 the launcher's choice, 1 the register-fed kernel, 2 the one with a ring in shared memory (3 / 4: its form with two pipelines in one CTA / two CTAs per SM)")
+    ap.add_argument("--norm", action="store_true", help="qkv_rope, gate_up_swiglu: rows of the float32 stream with the norm in front of the product (a step's first layer) "
+                    "instead of rows that the product in front left ready; out_residual, down_residual: leave no rows ready")
     ap.add_argument("--repeat", type=int, default=50)
     ap.add_argument("--no-graph", action="store_true")
     a = ap.parse_args(argv)
@@ -128,28 +130,31 @@ def main(argv=None) -> int:
     n_pages = M * width
     inv = torch.ones(D // 2, device=dev)
     bytes_read = 0
+    norm = a.norm or M > 32 or a.variant > 0                        # (33 rows and more are normed by a kernel of their own; a forced kernel takes no ready rows)
+    ready, squares = h.to(bf), torch.full((M, ops.ready_parts(hid)), float(hid) / ops.ready_parts(hid), device=dev)
+    rows = (h, (nw, 1e-5)) if norm else (ready, ops.ReadyRows(squares, 1e-5))
     if a.kernel in ("qkv_rope", "attn_decode", "attn_prefill", "attn_prefill_tc", "attn_prefill_ws"):
         kp = torch.randn(n_pages, Hkv, 64, D, device=dev).to(bf)
         vp = torch.randn_like(kp)
     if a.kernel == "qkv_rope":
         ws = [torch.randn((H + 2 * Hkv) * D, hid, device=dev).to(bf) for _ in range(copies)]
         q = torch.empty(M, H * D, device=dev, dtype=bf)
-        fn = lambda: ops.skinny_qkv_rope(h, (nw, 1e-5), nxt(ws), q, pos, seq, table, inv, D, kp, vp, H, Hkv, D)
+        fn = lambda: ops.skinny_qkv_rope(*rows, nxt(ws), q, pos, seq, table, inv, D, kp, vp, H, Hkv, D)
         bytes_read = ws[0].numel() * 2
     elif a.kernel == "out_residual":
         ws = [torch.randn(hid, H * D, device=dev).to(bf) for _ in range(copies)]
         att = torch.randn(M, H * D, device=dev).to(bf)
-        fn = lambda: ops.skinny_linear(att, None, nxt(ws), None, residual=h)
+        fn = (lambda: ops.skinny_linear(att, None, nxt(ws), None, residual=h)) if norm else (lambda: ops.skinny_residual_ready(att, nxt(ws), h, nw, ready, squares))
         bytes_read = ws[0].numel() * 2
     elif a.kernel == "gate_up_swiglu":
         ws = [torch.randn(2 * I, hid, device=dev).to(bf) for _ in range(copies)]
         act = torch.empty(M, I, device=dev, dtype=bf)
-        fn = lambda: ops.skinny_swiglu(h, (nw, 1e-5), nxt(ws), act)
+        fn = lambda: ops.skinny_swiglu(*rows, nxt(ws), act)
         bytes_read = ws[0].numel() * 2
     elif a.kernel == "down_residual":
         ws = [torch.randn(hid, I, device=dev).to(bf) for _ in range(copies)]
         act = torch.randn(M, I, device=dev).to(bf)
-        fn = lambda: ops.skinny_linear(act, None, nxt(ws), None, residual=h)
+        fn = (lambda: ops.skinny_linear(act, None, nxt(ws), None, residual=h)) if norm else (lambda: ops.skinny_residual_ready(act, nxt(ws), h, nw, ready, squares))
         bytes_read = ws[0].numel() * 2
     elif a.kernel == "head":
         ws = [torch.randn(V, hid, device=dev).to(bf) for _ in range(4)]
@@ -162,7 +167,7 @@ def main(argv=None) -> int:
         partial = torch.empty(M * H * ops.MAX_DECODE_SPLITS * (D + 2), device=dev)
         out = torch.empty(M, H * D, device=dev, dtype=bf)
         fn = lambda: ops.attention_decode_bf16(q, H * D, kp, vp, table, pos, out, partial, ops.decode_counters(dev), H, Hkv, D,
-                                               splits, 1.0 / math.sqrt(D))
+                                               splits, 1.0 / math.sqrt(D), in_step=True)
         bytes_read = M * (a.ctx + 1) * 2 * Hkv * D * 2
     elif a.kernel in ("attn_prefill", "attn_prefill_tc", "attn_prefill_ws"):
         T = a.tokens

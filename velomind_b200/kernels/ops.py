@@ -9,7 +9,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from typing import Optional
+from typing import NamedTuple, Optional
 
 import torch
 
@@ -282,9 +282,22 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> None:
         torch.mm(x, weight.t(), out_dtype=out.dtype, out=out)
 
 
+class ReadyRows(NamedTuple):
+    """As the `norm` of a product: its rows carry the norm's weight already, as skinny_residual_ready leaves them (at most 32)."""
+    squares: torch.Tensor        # float32 [M, ready_parts(K)], the parts of the rows' sums of squares
+    eps: float
+
+
+def ready_parts(columns: int) -> int:
+    """Parts of a row's sum of squares that skinny_residual_ready leaves."""
+    return library().vm_skinny_ready_parts(_c_int(columns))
+
+
 def _norm_args(norm):
     if norm is None:
         return 0, None, 0.0
+    if isinstance(norm, ReadyRows):
+        return 2, norm.squares, float(norm.eps)
     weight, eps = norm
     return 1, weight, float(eps)
 
@@ -299,7 +312,8 @@ def skinny_variant(variant: int) -> None:
 def skinny_linear(x: torch.Tensor, norm, weight: torch.Tensor, out: Optional[torch.Tensor],
                   residual: Optional[torch.Tensor] = None, err: Optional[torch.Tensor] = None) -> None:
     """out = x' W^T (bf16 or float32 out), or residual += x' W^T (float32), for M <= 64 rows.
-    x' = x (bf16 [M, K]) when `norm` is None, else rmsnorm(x) * norm[0] with eps norm[1] from x float32 [M, K]."""
+    x' = x (bf16 [M, K]) when `norm` is None, the normed rows that x (bf16) stands for when it is ReadyRows, else rmsnorm(x) * norm[0] with eps norm[1]
+    from x float32 [M, K]."""
     M, K = x.shape
     N = weight.shape[0]
     pro, nw, eps = _norm_args(norm)
@@ -307,6 +321,14 @@ def skinny_linear(x: torch.Tensor, norm, weight: torch.Tensor, out: Optional[tor
                                       _c_int(K), _ptr(out), _c_int(out.stride(0) if out is not None else N),
                                       _c_int(1 if (out is not None and out.dtype == torch.float32) else 0), _ptr(residual),
                                       _ptr(err), _stream()), "skinny_linear")
+
+
+def skinny_residual_ready(x: torch.Tensor, weight: torch.Tensor, residual: torch.Tensor, next_norm: torch.Tensor, ready: torch.Tensor,
+                          squares: torch.Tensor) -> None:
+    """residual += x W^T for M <= 32 rows of bfloat16; leaves ready = residual * next_norm in bfloat16 and `squares` for the product behind that norm."""
+    M, K = x.shape
+    _check(library().vm_skinny_residual_ready(_ptr(_contig(x, "x")), _ptr(weight), _c_int(M), _c_int(weight.shape[0]), _c_int(K), _ptr(residual),
+                                              _ptr(next_norm), _ptr(_contig(ready, "ready")), _ptr(_contig(squares, "squares")), _stream()), "skinny_linear")
 
 
 def skinny_swiglu(x: torch.Tensor, norm, weight: torch.Tensor, out: torch.Tensor, err: Optional[torch.Tensor] = None) -> None:
