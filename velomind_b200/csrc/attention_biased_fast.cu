@@ -91,9 +91,10 @@ attn_biased_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride
         cp_async16_zfill(sQ + r * KP + ch * 8, q + (size_t)(t0 + (r < n_rows ? r : 0)) * q_row_stride + (size_t)h * DK + ch * 8, r < n_rows);
     }
     auto block_of = [&](int step) { return step < kept_blocks ? step : blk_lo + (step - kept_blocks); };
-    // a page is asked for a step ahead of its copies (not by the widest heads, whose registers are taken: keys and values of 128, one prompt of 512 tokens, 16
-    // heads 18.5 us with it, 16.8 without)
-    constexpr bool AHEAD = DK + DV <= 160;
+    // a page is asked for a step ahead of its copies (not where keys or values are 128 wide, whose registers are taken: keys and values of 128, one prompt of 512 tokens,
+    // 16 heads 18.5 us with it, 16.8 without; keys of 128 and values of 32, 300 tokens 10.2 / 9.8, of 16, 2,048 tokens 62.7 / 58.7, of 32 and 128 69.2 / 66.7; but keys of 96
+    // and values of 64, 2,048 tokens 62.9 / 65.7)
+    constexpr bool AHEAD = DK <= 96 && DV <= 96;
     auto page_of = [&](int step) {
         const int blk = block_of(step);
         return step < n_steps && blk < max_blocks ? table[blk] : -1;

@@ -57,8 +57,13 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
     return *reinterpret_cast<unsigned*>(&v);
 }
 
+// CTAs an SM that the registers leave: four of heads up to 64 (128 registers), three of 80 and 96 in one group, as their shared memory does (unbounded they take 177 and
+// 195 registers and are two: 300 prompts of 60 tokens, 9 heads of 80 123 us against 95, of 96 127 / 105; eight of 512, 32 heads of 80 66 / 59; 1,400 + 2,000 tokens,
+// 9 heads of 80 47 / 52)
+template <int D, int NG> constexpr int prefill_ctas() { return D <= 64 && NG <= 2 ? 4 / NG : NG == 1 && D <= 96 ? 3 : 1; }
+
 template <int D, int NG>
-__global__ void __launch_bounds__(128 * NG, D <= 64 && NG <= 2 ? 4 / NG : 1)      // (128 registers: as many CTAs an SM as its shared memory leaves)
+__global__ void __launch_bounds__(128 * NG, prefill_ctas<D, NG>())
 attn_prefill_mma_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, const __nv_bfloat16* __restrict__ kpages,
                         const __nv_bfloat16* __restrict__ vpages, const int* __restrict__ block_table, int max_blocks,
                         const int* __restrict__ positions, const int* __restrict__ cu_tokens, int B, const __grid_constant__ VmTiles tiles,

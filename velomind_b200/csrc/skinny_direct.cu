@@ -16,6 +16,9 @@
 // 3.15 -> 1.9, 3.3 -> 2.0 us; 576 x 576 with the residual sum 2.3 -> 1.5, 2.45 -> 1.65; 2 x 1,536 x 576 with norm and unit 3.2 -> 2.0, 3.45 -> 2.3;
 // 576 x 1,536 with the sum 3.2 -> 1.7, 3.3 -> 1.9.  Larger matrices, against the kernel of skinny_stream.cuh, 8 rows: 960 x 2,560 5.4 -> 2.7,
 // 2 x 2,560 x 960 5.9 -> 3.4, 2,048 x 8,192 11.8 -> 8.2 (33.6 MB: 4.1 TB/s), 6,144 x 2,048 7.9 -> 5.9, 2 x 8,192 x 2,048 14.7 -> 13.8 (4.9 TB/s).
+// 17 and 32 plain rows: 960 x 576 3.4 -> 2.0, 3.8 -> 2.2; 2 x 1,536 x 576 4.35 -> 3.6, 5.0 -> 3.8; 576 x 1,536 with the sum 3.3 -> 3.0, 3.6 -> 3.3; 2 x 2,560 x 960
+// 7.9 -> 7.5, 9.9 -> 8.1; 960 x 2,560 with the sum 6.0 -> 5.5, 7.1 -> 5.9; 2,048 x 2,048 with the sum 10.4 -> 4.7, 11.9 -> 5.2.  Where it loses, plain rows do not
+// take it (ring_pays in skinny_gemm.cu).
 #include "skinny_body.cuh"
 
 namespace {

@@ -18,8 +18,7 @@
 // 16-byte loads possible.  A (at most 64 rows) sits in shared memory; when a product has more column tiles than the
 // GPU holds CTAs and all of K fits the tile, a CTA takes several tiles one after another with A staged once.
 // Under programmatic dependent launch the kernel requests its first weight blocks (and the rotary frequencies) before
-// it waits for its predecessor; the rope_kv form lets ITS successor, the decode attention, start only after that wait
-// (common.cuh says why).
+// it waits for its predecessor; the rope_kv form lets its successor, the decode attention, start only after that wait.
 //
 // Rows that lie ready in bfloat16 (at most 32 of them) take skinny_direct_kernel (skinny_direct.cu) but for 9 and more plain rows of many megabytes of
 // weights (ring_pays); the kernels here are for those, for the norm as a prologue, for the vocabulary head and for more rows.

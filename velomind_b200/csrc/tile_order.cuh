@@ -4,7 +4,8 @@
 // (2,048 tokens, 9 heads in tiles of 64 rows: 288 CTAs, all resident, 12 to 52 key blocks an SM, 33 on average).  So the host lists a step's tiles by their number
 // of blocks, the longest first (shape only: new tokens per sequence), and the CTAs, which the GPU deals out to its SMs in turn, take them forwards and
 // backwards from wave to wave.  The list rides along as a kernel argument, two bytes a tile, so that no CTA walks over the sequences' offsets (a chain of loads)
-// either.  Steps of more tiles than it holds keep that walk and take a prompt's last tiles first: they are many waves long.
+// either.  Steps of more tiles than it holds keep that walk and take a prompt's last tiles first: they are many waves long.  A step of one tile gains nothing and pays
+// 0.1 to 0.3 us (a prompt of 33 to 64 tokens, 9 heads of 64 3.6 -> 3.9; without the list 3.8, so most of it is the kernel's other code).
 #pragma once
 #include "common.cuh"
 
