@@ -616,6 +616,8 @@ public:
 
 class Embedding : public Part {
 public:
+    // The first work of a step.  Later kernels of the step read, before their own turn, what earlier steps wrote (kernels.h, the decode attention inside a
+    // step), so the first kernel enqueued here must not let its dependents start before it has waited itself; a launch without attributes never does.
     virtual void forward(StepContext& ctx, const int* tokens, float* h) = 0;
     // float32 words the embedding keeps per sequence (the token before the step's first one); while it runs, `ctx.state()` is that
     // area, which lies behind the schedule's own: a state area numbered schedule.size()
